@@ -1,0 +1,32 @@
+"""Kernels at the sizes where they can go wrong -- edges of tiles and groups, remainders, the
+smallest and largest of a range -- against the CPU oracle. Sets of edges: every comparison is exact."""
+import numpy as np
+import pytest
+
+import grg_gen as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nv", [1, 31, 32, 33, 193, 1000, 40_000])
+def test_counts_and_hash_by_row_groups(grg_mod, oracle_mod, nv):
+    """Counts, degrees and the hash are summed over groups of 1 to 32 rows a warp (fewer in small
+    graphs); ranges that start and end inside a group add up to the whole."""
+    w = G.alias(seed=nv, num_vars=nv, num_base_edges=3 * nv, block=min(nv, 300)) if nv > 1 else None
+    if w is None:                                   # one vertex with a loop of each label
+        src, dst, lab = np.zeros(3, np.uint32), np.zeros(3, np.uint32), np.arange(1, 4, dtype=np.uint8)
+        rules, nl = np.array([[1, 1, 1], [2, 3, 1]], np.int32), 3
+    else:
+        src, dst, lab, rules, nl = w.src, w.dst, w.lab, w.rule_ids(), w.num_labels
+    r = oracle_mod.closure(nv, rules, nl, 0, src, dst, lab)
+    ctx, st = grg_mod.run_closure(nv, rules, nl, 0, src, dst, lab)
+    counts = r.label_counts().tolist()
+    assert ctx.label_counts().tolist() == counts and ctx.set_hash() == r.set_hash
+    deg = ctx.degree()
+    e, el = r.degree()
+    assert np.array_equal(deg[0], e) and np.array_equal(deg[3], el)
+    cuts = [0, nv // 3, nv // 3 + 1, nv - nv // 5, nv]
+    parts = [ctx.range_counts(a, b) for a, b in zip(cuts, cuts[1:])]
+    assert np.sum([p[0] for p in parts], axis=0).tolist() == counts
+    assert sum(p[1] for p in parts) % (1 << 64) == r.set_hash
+    ctx.close()
