@@ -73,7 +73,11 @@ enum : int {
     C_JQ = C_LABEL0 + MAX_SLOTS + 20,    // work queue of a join or push launch: next 32-record batch (zeroed before each launch)
     C_NOSLOT = C_LABEL0 + MAX_SLOTS + 21, // of C_WOUT: items of a run of records left without a window slot
     C_CANDS = C_LABEL0 + MAX_SLOTS + 22,  // candidates k_apply inserted over the closure
-    NCTR = C_LABEL0 + MAX_SLOTS + 23
+    C_TN = C_LABEL0 + MAX_SLOTS + 23,     // tiles of the round (k_tile_starts); zeroed with the next two
+    C_TQ = C_LABEL0 + MAX_SLOTS + 24,     // work queue of k_tile: next tile
+    C_LN = C_LABEL0 + MAX_SLOTS + 25,     // records k_tile left to k_join
+    C_TS = C_LABEL0 + MAX_SLOTS + 26,     // log2 of the rows of a tile in a device-driven round (0 = not tiled)
+    NCTR = C_LABEL0 + MAX_SLOTS + 27
 };
 // error bits of C_ERR; ERR_IN_* (in C_BADIN) flag input edges that were refused
 // (label outside 1..L, vertex id outside the graph) and never touched a table

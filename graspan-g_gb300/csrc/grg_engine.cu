@@ -1,6 +1,8 @@
 // grg_engine.cu -- CUDA kernels and the C ABI of the closure engine (sm_103a).
 //
 // Hot path (reference: src/kernel.cu):
+//   k_tile    the same joins for grammars with a derivable right-hand label, over tiles of
+//             neighbouring rows (dense rows, read once a tile); leaves the rest to k_join.
 //   k_join    binary joins A ::= B C for a round's delta records, delta-left
 //             (D_B o O_C) and old-left (O_B o D_C, pulled through this round's
 //             delta index: virtual records from k_oldleft),
@@ -267,18 +269,27 @@ struct MinCap { uint32_t cap[MAX_LABELS + 1]; };
 // the edge histogram (held in cnt), bump-allocate. rowmark (nullable, 1 bit per
 // row): the minimum capacities apply only to marked rows -- an element image
 // holds a few partitions' rows, and rows it does not hold never gain edges.
-__global__ void k_load_alloc(Dev d, uint32_t first, uint32_t nv, uint32_t L, MinCap mc,
-                             const uint32_t *__restrict__ rowmark)
+// A block allocates its ALLOC_ROWS consecutive rows of one label with one atomic, in
+// row order: gathered delta records come in slot order, so the records of 1,024
+// neighbouring rows lie together and k_tile finds whole tiles (with one atomic a
+// warp, groups of 32 rows came in any order and a 256-row tile in 8 pieces).
+constexpr int ALLOC_ROWS = 1024;
+__global__ void __launch_bounds__(ALLOC_ROWS) k_load_alloc(Dev d, uint32_t first, uint32_t nv, uint32_t L, MinCap mc,
+                                                           const uint32_t *__restrict__ rowmark)
 {
-    const uint64_t ntables = (uint64_t)L * nv;
-    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < ((ntables + 31) & ~31ull);
-         u += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t lab = u < ntables ? (uint32_t)(u / nv) + 1 : 1;
-        const uint64_t t = (uint64_t)(lab - 1) * d.V + first + (u < ntables ? u % nv : 0);
-        uint32_t h = u < ntables ? d.cnt[t] : 0;
-        uint32_t cap = u < ntables ? mc.cap[lab] : 0;
+    __shared__ uint32_t warp_sum[ALLOC_ROWS / 32];
+    __shared__ unsigned long long base_s;
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+    const uint64_t groups = ((uint64_t)nv + ALLOC_ROWS - 1) / ALLOC_ROWS;
+    for (uint64_t g = blockIdx.x; g < groups * L; g += gridDim.x) {
+        const uint32_t lab = (uint32_t)(g / groups) + 1;
+        const uint64_t r = g % groups * ALLOC_ROWS + threadIdx.x;
+        const bool have = r < nv;
+        const uint64_t t = (uint64_t)(lab - 1) * d.V + first + (have ? r : 0);
+        const uint32_t h = have ? d.cnt[t] : 0;
+        uint32_t cap = have ? mc.cap[lab] : 0;
         if (rowmark && cap) {
-            const uint32_t row = first + (uint32_t)(u % nv);
+            const uint32_t row = first + (uint32_t)r;
             if (!((rowmark[row >> 5] >> (row & 31)) & 1u)) cap = 0;
         }
         if (h) {
@@ -286,18 +297,26 @@ __global__ void k_load_alloc(Dev d, uint32_t first, uint32_t nv, uint32_t L, Min
             if (cap < 4) cap = 4;
             while (cap < need) cap <<= 1;
         }
-        // warp-aggregated bump allocation
         uint32_t incl = cap;
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane_id() >= (uint32_t)o) incl += y;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
         }
-        uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        unsigned long long base = 0;
-        if (lane_id() == 31 && total) base = atomicAdd(&d.ctr[C_POOL_TOP], (unsigned long long)total);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        if (u < ntables) {
-            uint64_t off = base + incl - cap;
+        if (lane == 31) warp_sum[wid] = incl;
+        __syncthreads();
+        if (wid == 0) {
+            const uint32_t s = warp_sum[lane];
+            uint32_t si = s;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, si, o);
+                if (lane >= (uint32_t)o) si += y;
+            }
+            warp_sum[lane] = si - s;
+            if (lane == 31) base_s = si ? atomicAdd(&d.ctr[C_POOL_TOP], (unsigned long long)si) : 0ull;
+        }
+        __syncthreads();
+        if (have) {
+            const uint64_t off = base_s + warp_sum[wid] + incl - cap;
             if (cap && off + cap > d.pool_cap) {
                 atomicOr(&d.ctr[C_ERR], (unsigned long long)ERR_POOL);
                 cap = 0;
@@ -305,7 +324,15 @@ __global__ void k_load_alloc(Dev d, uint32_t first, uint32_t nv, uint32_t L, Min
             d.desc[t] = cap ? ((uint64_t)cap << 32) | (uint32_t)off : 0ull;
             d.cnt[t] = 0;
         }
+        __syncthreads();
     }
+}
+
+// Blocks of k_load_alloc for L labels over nv rows.
+static int alloc_grid(int sms, uint32_t L, uint32_t nv)
+{
+    const uint64_t g = (uint64_t)L * (((uint64_t)nv + ALLOC_ROWS - 1) / ALLOC_ROWS);
+    return (int)std::max<uint64_t>(std::min<uint64_t>(g, (uint64_t)sms * 2), 1);
 }
 
 __global__ void k_load_insert(Dev d, const uint32_t *src, const uint32_t *dst, const uint8_t *lab, uint64_t n,
@@ -547,18 +574,26 @@ __global__ void k_dindex_clear(Dev d, const uint4 *__restrict__ recs, int n_ctr)
 // masked to the vertices k whose row C[k] has deltas this round, becomes a
 // virtual delta record (label slot OL_SLOT0 + q). The 192 ids of an element are
 // exactly 6 words of the dirty-vertex bitmap. Records past cap are counted only.
-__global__ void k_oldleft(Dev d, uint32_t q, uint4 *out, uint64_t cap, const uint32_t *__restrict__ row_job,
-                          const uint32_t *__restrict__ job_cnt)
+// A block takes OL_ROWS consecutive rows and writes their records together, in
+// row order (the joins merge a row's records and share right-hand rows between
+// neighbouring rows): it counts them, reserves room once, and writes them, the
+// slots of a warp's 32 rows dealt over its lanes both times.
+constexpr int OL_ROWS = 256;
+__global__ void __launch_bounds__(OL_ROWS) k_oldleft(Dev d, uint32_t q, uint4 *out, uint64_t cap,
+                                                     const uint32_t *__restrict__ row_job,
+                                                     const uint32_t *__restrict__ job_cnt)
 {
     if (d.ctr[C_HALT]) return;
-    const uint32_t B = d.rt.ol_B[q], C = d.rt.ol_C[q];
+    __shared__ uint32_t warp_n[OL_ROWS / 32];
+    __shared__ unsigned long long base_s;
+    __shared__ uint8_t own_s[OL_ROWS / 32][32];
+    const uint32_t B = d.rt.ol_B[q], C = d.rt.ol_C[q], lane = lane_id(), wid = threadIdx.x >> 5;
     const uint32_t *dv = d.dvm + (size_t)(C - 1) * d.vwords;
     const uint32_t vkey = (OL_SLOT0 + q) << KEY_SHIFT;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t b0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); b0 < d.V; b0 += stride) {
-        const uint64_t v = b0 + lane_id();
+    uint8_t *own = own_s[wid];
+    for (uint64_t b0 = blockIdx.x * (uint64_t)OL_ROWS; b0 < d.V; b0 += (uint64_t)gridDim.x * OL_ROWS) {
+        const uint64_t v = b0 + threadIdx.x;
         const uint64_t de = v < d.V ? d.desc[(size_t)(B - 1) * d.V + v] : 0ull;
-        const uint32_t off = (uint32_t)de;
         uint32_t cap_v = (uint32_t)(de >> 32);
         if (v < d.V && prefix_table(d, B, cap_v)) cap_v = min(cap_v, d.cnt[(size_t)(B - 1) * d.V + v]);
         // batched jobs: a job without delta records this round adds no virtual records
@@ -566,38 +601,67 @@ __global__ void k_oldleft(Dev d, uint32_t q, uint4 *out, uint64_t cap, const uin
             const uint32_t job = row_job[v];
             if (job == EMPTY || job_cnt[job] == 0) cap_v = 0;
         }
-        const uint32_t maxc = __reduce_max_sync(0xffffffffu, cap_v);
-        for (uint32_t j = 0; j < maxc; j++) {
-            Bits m;
-            uint32_t any = 0, base = 0;
-            if (j < cap_v) {
-                const uint4 *e = reinterpret_cast<const uint4 *>(d.elems + (size_t)(off + j) * 8);
-                const uint4 e0 = e[0], e1 = e[1];
-                if (e1.z != EMPTY) {
-                    base = e1.z & BASE_MASK;
-                    const uint64_t w0 = (uint64_t)base * EW;
-                    const uint32_t ew[EW] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y};
+        uint32_t incl = cap_v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31), start = incl - cap_v;
+        const uint32_t adj = (uint32_t)de - start;
+        const unsigned full = __ballot_sync(0xffffffffu, cap_v != 0);
+        if (cap_v) own[__popc(full & ((1u << lane) - 1u))] = (uint8_t)lane;
+        __syncwarp();
+        unsigned long long pos = 0;
+        for (int write = 0; write < 2; write++) {
+            uint32_t before = 0, n = 0;
+            for (uint32_t f0 = 0; f0 < total; f0 += 32) {
+                const unsigned marks = __reduce_or_sync(0xffffffffu, cap_v && start - f0 < 32u ? 1u << (start - f0) : 0u);
+                const uint32_t o = own[before + __popc(marks & (0xFFFFFFFFu >> (31 - lane))) - 1];
+                before += __popc(marks);
+                const uint32_t s = __shfl_sync(0xffffffffu, adj, o) + f0 + lane;
+                Bits m;
+                uint32_t any = 0, base = 0;
+                if (f0 + lane < total) {
+                    uint4 e0, e1;
+                    ld32(d.elems + (size_t)s * 8, e0, e1);
+                    if (e1.z != EMPTY) {
+                        base = e1.z & BASE_MASK;
+                        const uint64_t w0 = (uint64_t)base * EW;
+                        const uint32_t ew[EW] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y};
 #pragma unroll
-                    for (int x = 0; x < EW; x++) {
-                        m.w[x] = (w0 + x < d.vwords) ? ew[x] & __ldg(dv + w0 + x) : 0u;
-                        any |= m.w[x];
+                        for (int x = 0; x < EW; x++) {
+                            m.w[x] = (w0 + x < d.vwords) ? ew[x] & __ldg(dv + w0 + x) : 0u;
+                            any |= m.w[x];
+                        }
                     }
                 }
-            }
-            const unsigned em = __ballot_sync(0xffffffffu, any != 0);
-            if (!em) continue;
-            unsigned long long p0 = 0;
-            const int leader = __ffs(em) - 1;
-            if ((int)lane_id() == leader) p0 = atomicAdd(&d.ctr[C_VN], (unsigned long long)__popc(em));
-            p0 = __shfl_sync(0xffffffffu, p0, leader);
-            if (any) {
-                const uint64_t p = p0 + __popc(em & ((1u << lane_id()) - 1u));
-                if (p < cap) {
-                    out[2 * p] = make_uint4(m.w[0], m.w[1], m.w[2], m.w[3]);
-                    out[2 * p + 1] = make_uint4(m.w[4], m.w[5], vkey | base, (uint32_t)v);
+                const unsigned em = __ballot_sync(0xffffffffu, any != 0);
+                if (write && any) {
+                    const uint64_t p = pos + n + __popc(em & ((1u << lane) - 1u));
+                    if (p < cap) {
+                        out[2 * p] = make_uint4(m.w[0], m.w[1], m.w[2], m.w[3]);
+                        out[2 * p + 1] = make_uint4(m.w[4], m.w[5], vkey | base, (uint32_t)(b0 + wid * 32 + o));
+                    }
                 }
+                n += __popc(em);
             }
+            if (write) break;
+            if (lane == 0) warp_n[wid] = n;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                uint32_t sum = 0;
+                for (int w = 0; w < OL_ROWS / 32; w++) {
+                    const uint32_t c = warp_n[w];
+                    warp_n[w] = sum;
+                    sum += c;
+                }
+                base_s = sum ? atomicAdd(&d.ctr[C_VN], (unsigned long long)sum) : 0ull;
+            }
+            __syncthreads();
+            pos = base_s + warp_n[wid];
+            if (!n) break;
         }
+        __syncthreads();
     }
 }
 
@@ -1161,6 +1225,552 @@ __global__ void __launch_bounds__(PUSH_WARPS * 32, 4) k_push_flat(Dev d, const u
     }
 }
 
+// ---------------------------------------------------------------- tile joins
+//
+// Grammars with a derivable right-hand label (alias, points-to) join dense rows: in a block of
+// 1,000 vertices that reach each other nearly every row i meets nearly every k, and all rows C[k]
+// hold nearly the same ids. A record at a time (k_join) then reads C's elements once per (i, k):
+// 2.3e10 elements for the 6.3e7 new ones of the 1M-vertex alias closure. k_tile takes the records
+// of up to TILE_ROWS neighbouring rows together:
+//  - the rows C[k] of one 192-id block kb of intermediates are read once for all of the tile's
+//    rows, as dense rows of TILE_W elements in shared memory, and the unions of all subsets of each
+//    4 of them are laid out beside them: a record then takes 48 lookups, one per 4 bits, instead of
+//    up to 192 rows (the method of Arlazarov, Dinic, Kronrod and Faradzev);
+//  - the tile's output rows A[i] are held as dense accumulators over the same TILE_W elements,
+//    loaded with what A[i] already has;
+//  - a record whose panel's union adds nothing to A[i] is done at once: late rounds (0.9M (i, k)
+//    pairs a block and round in the old-left joins, against a few thousand new edges) cost a
+//    compare a record instead of a pass over C's rows.
+// 1M-vertex alias closure: right-hand elements read 2.3e10 -> 5.4e8, closure 189 -> 82.5 ms;
+// 37k vertices 13.4 -> 7.5 ms. A block holds one tile a SM (214 KB), bound by the lookups' shared
+// memory reads (21 of 16 bytes a lane and record in the mean) and by the waits between its phases.
+// Only accumulator words that changed are inserted. Right-hand elements outside the window of
+// TILE_W elements are joined in further windows (up to TILE_WINDOWS, each from the lowest base
+// not yet covered); blocks of intermediates with few records, and records that even the last
+// window leaves something of, go to a list that k_join takes.
+constexpr int TILE_THREADS = 1024;
+constexpr int TILE_WARPS = TILE_THREADS / 32;
+constexpr int TILE_ROWS_LG = 8, TILE_ROWS = 1 << TILE_ROWS_LG;
+constexpr int TILE_ROWS_MIN_LG = 4;
+constexpr int TILE_W = 8;                      // elements of a window: 48 words, 12 lanes of 16 bytes
+constexpr int TILE_Q = TILE_W * EW / 4;
+constexpr int TILE_G = EIDS / 4;               // groups of 4 intermediates
+constexpr int TILE_RECS = 2048;                // records a tile holds at once (more are taken in turns)
+constexpr int TILE_KB = 32;                    // distinct blocks of intermediates at once
+constexpr int TILE_WINDOWS = 8;
+#ifndef GRG_TILE_BITS
+#define GRG_TILE_BITS 128
+#endif
+constexpr uint32_t TILE_MIN_BITS = GRG_TILE_BITS;  // (record, k) pairs that pay for reading a panel
+constexpr uint32_t TILE_MIN_RECS = 4;
+
+// Rows of a tile for a round of n records (some 6 a row): as many as leave every SM two tiles or more.
+__host__ __device__ inline uint32_t tile_rows_lg(uint64_t n)
+{
+    uint32_t lg = TILE_ROWS_MIN_LG;
+    while (lg < (uint32_t)TILE_ROWS_LG && (n / 1800) >> (lg + 1)) lg++;
+    return lg;
+}
+
+struct TileSmem {
+    uint4 tab[TILE_G][16][TILE_Q];             // per 4 rows C[k]: the unions of their 16 subsets
+    uint4 acc[TILE_ROWS][TILE_Q];              // rows A[i]
+    uint32_t rmeta[TILE_RECS];                 // local row, kb entry << 8 (TILE_KB: none), TM_ flags
+    uint32_t U[TILE_W * EW];                   // the panel's union
+    uint32_t kb[TILE_KB], kbits[TILE_KB], kcnt[TILE_KB], kpos[TILE_KB];
+    uint32_t kmore;                            // blocks whose panels have elements outside every window so far
+    uint32_t outk[EW];                         // the panel's rows with such elements
+    uint32_t rowoff[TILE_ROWS];                // first pool slot of A[i]
+    uint32_t rowhas[TILE_ROWS / 32], rowfail[TILE_ROWS / 32];
+    uint32_t rowchg[TILE_ROWS];                // accumulator quads that changed
+    uint32_t wins[TILE_WINDOWS];
+    uint32_t next_w, end, tile, kmin;
+    uint32_t heavy;                            // entries of kb with enough pairs
+    uint16_t ord[TILE_RECS];
+    __align__(8) uint16_t look[TILE_WARPS][TILE_G + 8];   // a record's lookups: subset entries of tab
+    uint8_t slot[TILE_ROWS][TILE_W];           // slot of A[i]'s element within its table (0xFF: none seen)
+};
+static_assert(sizeof(TileSmem) <= 227 * 1024, "a tile fits an SM's shared memory");
+constexpr uint32_t TM_LEFT = 1u << 16;         // the record goes to k_join
+
+// Tiles of the round's records: a tile starts where the label or the row block (row >> C_TS)
+// differs from the record before it. Starts are listed in any order (bit 31: virtual records).
+// sh: log2 of the rows of a tile; 0 = take it from the counters (device-driven rounds), where 0
+// means a round that is joined as sub-records.
+__global__ void k_tile_starts(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint32_t *list,
+                              uint64_t list_cap, uint32_t sh)
+{
+    if (d.ctr[C_HALT]) return;
+    if (!sh) sh = (uint32_t)d.ctr[C_TS];
+    if (!sh) return;
+    const uint64_t nd = d.ctr[C_DIRTY_N], n = nd + d.ctr[C_VN];
+    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
+         i0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = i0 + lane_id();
+        bool start = false;
+        uint32_t at = 0;
+        if (i < n) {
+            const bool virt = i >= nd;
+            at = (uint32_t)(virt ? i - nd : i);
+            const uint2 *r = reinterpret_cast<const uint2 *>(virt ? vrecs : grecs);
+            const uint2 k = r[4 * (uint64_t)at + 3];
+            start = at == 0;
+            if (!start) {
+                const uint2 p = r[4 * (uint64_t)at - 1];
+                start = (p.x >> KEY_SHIFT) != (k.x >> KEY_SHIFT) || (p.y >> sh) != (k.y >> sh);
+            }
+            if (virt) at |= 1u << 31;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, start);
+        if (!m) continue;
+        unsigned long long p = 0;
+        if (lane_id() == (uint32_t)(__ffs(m) - 1)) p = atomicAdd(&d.ctr[C_TN], (unsigned long long)__popc(m));
+        p = __shfl_sync(0xffffffffu, p, __ffs(m) - 1) + __popc(m & ((1u << lane_id()) - 1u));
+        if (start && p < list_cap) list[p] = at;
+    }
+}
+
+// Appends a record to a list with a device counter; records past cap are counted only.
+__device__ __forceinline__ void list_push(unsigned long long *n, uint64_t cap, uint4 *out, const uint4 a, const uint4 b)
+{
+    const unsigned long long p = atomicAdd(n, 1ull);
+    if (p < cap) st32(out + 2 * p, a, b);
+}
+
+__device__ __forceinline__ uint4 or4(const uint4 a, const uint4 b)
+{
+    return make_uint4(a.x | b.x, a.y | b.y, a.z | b.z, a.w | b.w);
+}
+__device__ __forceinline__ uint4 tab_at(const unsigned char *tb, uint32_t i)
+{
+    return *reinterpret_cast<const uint4 *>(tb + i * (TILE_Q * 16));
+}
+// b has no bit that a lacks
+__device__ __forceinline__ bool covers4(const uint4 a, const uint4 b)
+{
+    return ((b.x & ~a.x) | (b.y & ~a.y) | (b.z & ~a.z) | (b.w & ~a.w)) == 0;
+}
+
+__global__ void __launch_bounds__(TILE_THREADS, 1)
+    k_tile(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, const uint32_t *__restrict__ list,
+           uint64_t list_cap, uint4 *left_out, uint64_t left_cap, uint4 *retry_out, uint32_t sh)
+{
+    extern __shared__ __align__(16) unsigned char tile_smem_raw[];
+    TileSmem &w = *reinterpret_cast<TileSmem *>(tile_smem_raw);
+    if (d.ctr[C_HALT]) return;
+    if (!sh) sh = (uint32_t)d.ctr[C_TS];
+    if (!sh) return;
+    const uint64_t ntiles = min((uint64_t)d.ctr[C_TN], list_cap);
+    const uint64_t nd = d.ctr[C_DIRTY_N], nv = d.ctr[C_VN];
+    const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, rows = 1u << sh;
+    // in the joins, lanes 0-11 and 16-27 hold a row's 12 quads of 16 bytes (12-15 and 28-31 repeat the last)
+    const uint32_t half = lane >> 4, q = min(lane & 15, (uint32_t)TILE_Q - 1);
+    uint32_t n_left = 0, n_right = 0, inserts = 0;
+    for (uint32_t i = tid; i < TILE_G * TILE_Q; i += TILE_THREADS)      // the empty subsets
+        w.tab[i / TILE_Q][0][i % TILE_Q] = make_uint4(0, 0, 0, 0);
+
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) w.tile = (uint32_t)min((unsigned long long)ntiles, atomicAdd(&d.ctr[C_TQ], 1ull));
+        __syncthreads();
+        if (w.tile >= ntiles) break;
+        const uint32_t at = list[w.tile];
+        const bool virt = at >> 31;
+        const uint4 *recs = virt ? vrecs : grecs;
+        const uint64_t nrec = virt ? nv : nd;
+        uint64_t pos = at & 0x7FFFFFFFu;
+        const uint2 head = reinterpret_cast<const uint2 *>(recs)[4 * pos + 3];
+        const uint32_t lab = head.x >> KEY_SHIFT, row0 = (head.y >> sh) << sh;
+        const bool real = !virt && lab >= 1 && lab <= (uint32_t)d.rt.L;
+        const uint32_t qv = lab - OL_SLOT0;
+        const uint32_t nrules = virt ? (qv < (uint32_t)d.rt.nol ? 1u : 0u)
+                                     : real ? (uint32_t)(d.rt.bin_start[lab + 1] - d.rt.bin_start[lab]) : 0u;
+        for (bool more = true; more;) {
+            // ---- the next records of the tile: bits, local rows, their blocks of intermediates
+            if (tid < TILE_KB) {
+                w.kb[tid] = EMPTY;
+                w.kbits[tid] = w.kcnt[tid] = 0;
+            }
+            if (tid < TILE_ROWS / 32) w.rowhas[tid] = w.rowfail[tid] = 0;
+            if (tid == 0) {
+                w.end = TILE_RECS;
+                w.kmin = EMPTY;
+            }
+            __syncthreads();
+            uint32_t nbits[TILE_RECS / TILE_THREADS];
+#pragma unroll
+            for (int u = 0; u < TILE_RECS / TILE_THREADS; u++) {
+                const uint32_t i = tid + u * TILE_THREADS;
+                bool mine = false;
+                nbits[u] = 0;
+                if (pos + i < nrec) {
+                    uint4 a, b;
+                    ld32(recs + 2 * (pos + i), a, b);
+                    if ((b.z >> KEY_SHIFT) == lab && (b.w >> sh) == (row0 >> sh)) {
+                        mine = true;
+                        nbits[u] = popc6(Bits{{a.x, a.y, a.z, a.w, b.x, b.y}});
+                        w.rmeta[i] = b.z & BASE_MASK;
+                        w.ord[i] = (uint16_t)(b.w - row0);
+                    }
+                }
+                if (!mine) atomicMin(&w.end, i);
+            }
+            __syncthreads();
+            const uint32_t nr = w.end;             // records at and past it are not this tile's
+            more = nr == TILE_RECS;
+#pragma unroll
+            for (int u = 0; u < TILE_RECS / TILE_THREADS; u++) {
+                // the lanes of one block look it up once
+                const uint32_t i = tid + u * TILE_THREADS;
+                const uint32_t kb = i < nr ? w.rmeta[i] : EMPTY;
+                const unsigned same = __match_any_sync(0xffffffffu, kb);
+                const uint32_t leader = __ffs(same) - 1;
+                uint32_t e = TILE_KB;
+                if (lane == leader && kb != EMPTY) {
+                    uint32_t h = (kb * 0x9E3779B1u) >> 27;
+                    for (int p = 0; p < TILE_KB; p++, h = (h + 1) & (TILE_KB - 1)) {
+                        const uint32_t prev = atomicCAS(&w.kb[h], EMPTY, kb);
+                        if (prev != EMPTY && prev != kb) continue;
+                        atomicAdd(&w.kcnt[h], (uint32_t)__popc(same));
+                        e = h;
+                        break;
+                    }
+                }
+                e = __shfl_sync(0xffffffffu, e, leader);
+                if (i < nr) {
+                    if (e < (uint32_t)TILE_KB) atomicAdd(&w.kbits[e], nbits[u]);
+                    w.rmeta[i] = w.ord[i] | (e << 8);
+                }
+            }
+            __syncthreads();
+            // ---- order by block; blocks with few pairs are left to k_join
+            if (wid == 0) {
+                const bool heavy = w.kb[lane] != EMPTY && w.kbits[lane] >= TILE_MIN_BITS && w.kcnt[lane] >= TILE_MIN_RECS;
+                const uint32_t c = heavy ? w.kcnt[lane] : 0;
+                uint32_t incl = c;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= (uint32_t)o) incl += y;
+                }
+                w.kpos[lane] = incl - c;           // becomes the end of the block's list below
+                w.kcnt[lane] = c;
+                const unsigned hm = __ballot_sync(0xffffffffu, heavy);
+                const uint32_t lo = __reduce_min_sync(0xffffffffu, heavy ? w.kb[lane] : EMPTY);
+                if (lane == 0) {
+                    w.kmin = lo;
+                    w.heavy = hm;
+                }
+            }
+            __syncthreads();
+            const bool any_heavy = w.kmin != EMPTY;
+            for (uint32_t i0 = tid & ~31u; i0 < nr; i0 += TILE_THREADS) {
+                const uint32_t i = i0 + lane;
+                const uint32_t m = i < nr ? w.rmeta[i] : (uint32_t)TILE_KB << 8, row = m & 0xFFu, e = (m >> 8) & 0xFFu;
+                const bool take = nrules && e < (uint32_t)TILE_KB && w.kcnt[e];
+                const unsigned same = __match_any_sync(0xffffffffu, take ? e : (uint32_t)TILE_KB);
+                const uint32_t leader = __ffs(same) - 1;
+                uint32_t p = 0;
+                if (take && lane == leader) p = atomicAdd(&w.kpos[e], (uint32_t)__popc(same));
+                p = __shfl_sync(0xffffffffu, p, leader) + __popc(same & ((1u << lane) - 1u));
+                if (i >= nr) continue;
+                if (take) {
+                    w.ord[p] = (uint16_t)i;
+                    atomicOr(&w.rowhas[row >> 5], 1u << (row & 31));
+                } else if (nrules) {
+                    w.rmeta[i] = m | TM_LEFT;
+                }
+                // unary rules A ::= B (records left to k_join take theirs there)
+                if (real && (take || !nrules) && d.rt.un_start[lab + 1] > d.rt.un_start[lab]) {
+                    uint4 r0, r1;
+                    ld32(recs + 2 * (pos + i), r0, r1);
+                    const uint32_t kb = r1.z & BASE_MASK;
+                    bool ok = true;
+                    const Bits b = {{r0.x, r0.y, r0.z, r0.w, r1.x, r1.y}};
+                    for (int u = d.rt.un_start[lab]; u < d.rt.un_start[lab + 1]; u++) {
+                        const uint32_t A = d.rt.un_A[u];
+                        ok &= g_insert(d, A, row0 + row, kb, b, d.rt.track[A]);
+                        inserts++;
+                    }
+                    if (!ok) atomicOr(&w.rowfail[row >> 5], 1u << (row & 31));
+                }
+            }
+            __syncthreads();
+
+            for (uint32_t rho = 0; any_heavy && rho < nrules; rho++) {
+                const uint32_t rq = virt ? qv : d.rt.bin_start[lab] + rho;
+                const uint32_t A = virt ? d.rt.ol_A[rq] : d.rt.bin_A[rq], C = virt ? d.rt.ol_C[rq] : d.rt.bin_C[rq];
+                const bool prefA = (d.prefix_mask >> (A - 1)) & 1ull, prefC = (d.prefix_mask >> (C - 1)) & 1ull;
+                uint32_t win = w.kmin, todo = w.heavy;       // the window, the blocks to join in it
+                for (int nw = 0; nw < TILE_WINDOWS; nw++) {
+                    const bool last = nw == TILE_WINDOWS - 1;
+                    if (tid == 0) {
+                        w.wins[nw] = win;
+                        w.next_w = EMPTY;
+                        w.kmore = 0;
+                    }
+                    // ---- the rows A[i]: 8 lanes a row, the loads of a thread's rows in flight together
+                    {
+                        constexpr int NR = TILE_ROWS / (TILE_THREADS / 8);
+                        const uint32_t sub = tid & 7;
+                        uint32_t off[NR], cap[NR], most = 0;
+#pragma unroll
+                        for (int u = 0; u < NR; u++) {
+                            const uint32_t r = (tid >> 3) + u * (TILE_THREADS / 8);
+                            off[u] = cap[u] = 0;
+                            if (r >= rows || !((w.rowhas[r >> 5] >> (r & 31)) & 1u)) continue;   // uniform in the 8 lanes
+                            uint2 *p = reinterpret_cast<uint2 *>(&w.acc[r][0]) + sub * (EW / 2);
+                            p[0] = p[1] = p[2] = make_uint2(0, 0);
+                            w.slot[r][sub] = 0xFF;
+                            const size_t ti = (size_t)(A - 1) * d.V + row0 + r;
+                            const uint64_t de = d.desc[ti];
+                            off[u] = (uint32_t)de;
+                            cap[u] = (uint32_t)(de >> 32);
+                            if (prefA && cap[u] <= PREFIX_CAP) cap[u] = min(cap[u], d.cnt[ti]);
+                            if (sub == 0) {
+                                w.rowchg[r] = 0;
+                                w.rowoff[r] = off[u];
+                            }
+                            most = max(most, cap[u]);
+                        }
+                        __syncwarp();
+                        for (uint32_t t = sub; t < most; t += 8) {
+                            uint4 e0[NR], e1[NR];
+#pragma unroll
+                            for (int u = 0; u < NR; u++) {
+                                e1[u].z = EMPTY;
+                                if (t < cap[u]) ld32(d.elems + ((size_t)off[u] + t) * 8, e0[u], e1[u]);
+                            }
+#pragma unroll
+                            for (int u = 0; u < NR; u++) {
+                                const uint32_t dd = (e1[u].z & BASE_MASK) - win;
+                                if (e1[u].z == EMPTY || dd >= (uint32_t)TILE_W) continue;
+                                const uint32_t r = (tid >> 3) + u * (TILE_THREADS / 8);
+                                uint2 *p = reinterpret_cast<uint2 *>(&w.acc[r][0]) + dd * (EW / 2);
+                                p[0] = make_uint2(e0[u].x, e0[u].y);
+                                p[1] = make_uint2(e0[u].z, e0[u].w);
+                                p[2] = make_uint2(e1[u].x, e1[u].y);
+                                if (t < 0xFFu) w.slot[r][dd] = (uint8_t)t;
+                            }
+                        }
+                    }
+                    for (; todo; todo &= todo - 1) {
+                        const uint32_t e = __ffs(todo) - 1;
+                        __syncthreads();
+                        const uint32_t cnt = w.kcnt[e];
+                        // the warp's first records of the block (4 at once, 8 lanes each), in flight
+                        // while the panel is read
+                        const uint32_t first = w.kpos[e] - cnt;
+                        auto fetch = [&](uint32_t m) {
+                            const uint32_t j = wid + TILE_WARPS * (m + (lane >> 3));
+                            return j < cnt ? __ldg(reinterpret_cast<const uint32_t *>(recs) +
+                                                   8 * (pos + w.ord[first + j]) + (lane & 7))
+                                           : 0u;
+                        };
+                        uint32_t v = fetch(0);
+                        // ---- the panel: rows C[k], k of block kb; 8 lanes a row
+                        const uint64_t k0 = (uint64_t)w.kb[e] * EIDS;
+                        if (tid < TILE_W * EW) w.U[tid] = 0;
+                        if (tid < EW) w.outk[tid] = 0;
+                        __syncthreads();
+                        {
+                            constexpr int NR = (EIDS + TILE_THREADS / 8 - 1) / (TILE_THREADS / 8);
+                            const uint32_t sub = tid & 7;
+                            uint32_t beg[NR], n[NR], most = 0;
+#pragma unroll
+                            for (int u = 0; u < NR; u++) {
+                                const uint32_t r = (tid >> 3) + u * (TILE_THREADS / 8);
+                                beg[u] = n[u] = 0;
+                                if (r < EIDS) {
+                                    uint2 *p = reinterpret_cast<uint2 *>(&w.tab[r >> 2][1 << (r & 3)][0]) + sub * (EW / 2);
+                                    p[0] = p[1] = p[2] = make_uint2(0, 0);
+                                }
+                                if (r < EIDS && k0 + r < d.V) {
+                                    const size_t ti = (size_t)(C - 1) * d.V + k0 + r;
+                                    if (virt) {
+                                        beg[u] = __ldg(d.drs + ti);
+                                        n[u] = beg[u] == EMPTY ? 0u : __ldg(d.drc + ti);
+                                    } else {
+                                        const uint64_t de = d.desc[ti];
+                                        beg[u] = (uint32_t)de;
+                                        n[u] = (uint32_t)(de >> 32);
+                                        if (prefC && n[u] <= PREFIX_CAP) n[u] = min(n[u], d.cnt[ti]);
+                                    }
+                                }
+                                most = max(most, n[u]);
+                            }
+                            __syncwarp();
+                            for (uint32_t t = sub; t < most; t += 8) {
+                                uint4 e0[NR], e1[NR];
+#pragma unroll
+                                for (int u = 0; u < NR; u++) {
+                                    e1[u].z = EMPTY;
+                                    if (t < n[u])
+                                        ld32(virt ? (const void *)(d.drec + 2 * ((size_t)beg[u] + t))
+                                                  : (const void *)(d.elems + ((size_t)beg[u] + t) * 8), e0[u], e1[u]);
+                                }
+#pragma unroll
+                                for (int u = 0; u < NR; u++) {
+                                    if (e1[u].z == EMPTY) continue;
+                                    const uint32_t r = (tid >> 3) + u * (TILE_THREADS / 8);
+                                    const uint32_t b = e1[u].z & BASE_MASK, dd = b - win;
+                                    n_right++;
+                                    if (dd < (uint32_t)TILE_W) {
+                                        uint2 *p = reinterpret_cast<uint2 *>(&w.tab[r >> 2][1 << (r & 3)][0]) + dd * (EW / 2);
+                                        p[0] = make_uint2(e0[u].x, e0[u].y);
+                                        p[1] = make_uint2(e0[u].z, e0[u].w);
+                                        p[2] = make_uint2(e1[u].x, e1[u].y);
+                                        continue;
+                                    }
+                                    bool done = false;                 // an earlier window held it
+                                    for (int x = 0; x < nw; x++) done |= b - w.wins[x] < (uint32_t)TILE_W;
+                                    if (done) continue;
+                                    atomicOr(&w.kmore, 1u << e);
+                                    atomicMin(&w.next_w, b);
+                                    if (last) atomicOr(&w.outk[r >> 5], 1u << (r & 31));
+                                }
+                            }
+                        }
+                        __syncthreads();
+                        // ---- the subsets of each 4 rows, and the panel's union
+                        if (tid < TILE_G * TILE_Q) {
+                            uint4(*g)[TILE_Q] = w.tab[tid / TILE_Q];
+                            const uint32_t c = tid % TILE_Q;
+                            const uint4 r0 = g[1][c], r1 = g[2][c], r2 = g[4][c], r3 = g[8][c];
+                            const uint4 a = or4(r0, r1), b = or4(r2, r3), all = or4(a, b);
+                            g[3][c] = a;
+                            g[5][c] = or4(r0, r2);
+                            g[6][c] = or4(r1, r2);
+                            g[7][c] = or4(a, r2);
+                            g[9][c] = or4(r0, r3);
+                            g[10][c] = or4(r1, r3);
+                            g[11][c] = or4(a, r3);
+                            g[12][c] = b;
+                            g[13][c] = or4(r0, b);
+                            g[14][c] = or4(r1, b);
+                            g[15][c] = all;
+                            if (all.x) atomicOr(&w.U[4 * c], all.x);
+                            if (all.y) atomicOr(&w.U[4 * c + 1], all.y);
+                            if (all.z) atomicOr(&w.U[4 * c + 2], all.z);
+                            if (all.w) atomicOr(&w.U[4 * c + 3], all.w);
+                        }
+                        __syncthreads();
+                        // ---- the block's records, one a warp at a time: its groups of 4 bits are listed, and
+                        // each half warp ORs the subsets that every other four of them name. Lanes whose
+                        // quad has nothing left to gain read nothing.
+                        const uint4 un = reinterpret_cast<const uint4 *>(w.U)[q];
+                        const unsigned char *tb = reinterpret_cast<const unsigned char *>(&w.tab[0][0][q]);
+                        uint16_t *look = w.look[wid];
+                        for (uint32_t m0 = 0; wid + TILE_WARPS * m0 < cnt; m0 += 4) {
+                            const uint32_t vn = fetch(m0 + 4);
+#pragma unroll 1
+                            for (uint32_t m = 0; m < 4 && wid + TILE_WARPS * (m0 + m) < cnt; m++) {
+                                const uint32_t row = __shfl_sync(0xffffffffu, v, m * 8 + 7) - row0;
+                                const uint4 a0 = w.acc[row][q];
+                                n_left += lane == 0 && nw == 0;
+                                if (last) {
+                                    const unsigned o = __ballot_sync(0xffffffffu, lane >> 3 == m && (lane & 7) < EW &&
+                                                                                      (v & w.outk[min(lane & 7, EW - 1u)]));
+                                    if (o && lane == 0) w.rmeta[w.ord[first + wid + TILE_WARPS * (m0 + m)]] |= TM_LEFT;
+                                }
+                                const bool need = !covers4(a0, un);
+                                if (!__any_sync(0xffffffffu, need)) continue;
+                                // the groups of 4 bits that are not empty (21 of 48 in the mean)
+                                const uint32_t g0 = (__shfl_sync(0xffffffffu, v, m * 8 + (lane >> 3)) >> (4 * (lane & 7))) & 15u;
+                                uint32_t g1 = (__shfl_sync(0xffffffffu, v, m * 8 + 4 + (lane >> 3 & 1)) >>
+                                               (4 * (lane & 7))) & 15u;
+                                if (half) g1 = 0;
+                                const unsigned b0 = __ballot_sync(0xffffffffu, g0 != 0), b1 = __ballot_sync(0xffffffffu, g1 != 0);
+                                const unsigned lt = (1u << lane) - 1u;
+                                const uint32_t n0 = __popc(b0), n = n0 + __popc(b1);
+                                if (g0) look[__popc(b0 & lt)] = (uint16_t)(lane * 16 + g0);
+                                if (g1) look[n0 + __popc(b1 & lt)] = (uint16_t)((32 + lane) * 16 + g1);
+                                if (lane < 8) look[n + lane] = 0;      // padding: the empty subset
+                                __syncwarp();
+                                uint4 a = a0;
+                                if (need) {
+                                    for (uint32_t t = half * 4; t < n; t += 8) {
+                                        const uint2 k = *reinterpret_cast<const uint2 *>(look + t);
+                                        const uint4 p0 = tab_at(tb, k.x & 0xFFFFu), p1 = tab_at(tb, k.x >> 16);
+                                        const uint4 p2 = tab_at(tb, k.y & 0xFFFFu), p3 = tab_at(tb, k.y >> 16);
+                                        a = or4(or4(a, or4(p0, p1)), or4(p2, p3));
+                                    }
+                                }
+                                __syncwarp();
+                                a.x |= __shfl_xor_sync(0xffffffffu, a.x, 16);
+                                a.y |= __shfl_xor_sync(0xffffffffu, a.y, 16);
+                                a.z |= __shfl_xor_sync(0xffffffffu, a.z, 16);
+                                a.w |= __shfl_xor_sync(0xffffffffu, a.w, 16);
+                                const unsigned cm = __ballot_sync(0xffffffffu, !covers4(a0, a)) & 0xFFFu;
+                                if (cm) {
+                                    if (lane < TILE_Q) w.acc[row][lane] = a;
+                                    if (lane == 0) w.rowchg[row] |= cm;
+                                }
+                            }
+                            v = vn;
+                        }
+                    }
+                    __syncthreads();
+                    // ---- changed elements go to the tables (or, as candidates, to k_apply)
+                    for (uint32_t f0 = tid & ~31u; f0 < rows * TILE_W; f0 += TILE_THREADS) {
+                        const uint32_t row = (f0 + lane) / TILE_W, e = (f0 + lane) % TILE_W;
+                        const bool has = f0 + lane < rows * TILE_W && ((w.rowhas[row >> 5] >> (row & 31)) & 1u) &&
+                                         ((w.rowchg[row] >> ((3 * e) >> 1)) & 3u);
+                        Bits b;
+                        uint32_t any = 0;
+                        if (has) {
+                            const uint2 *p = reinterpret_cast<const uint2 *>(&w.acc[row][0]) + e * (EW / 2);
+                            const uint2 p0 = p[0], p1 = p[1], p2 = p[2];
+                            b.w[0] = p0.x; b.w[1] = p0.y; b.w[2] = p1.x; b.w[3] = p1.y; b.w[4] = p2.x; b.w[5] = p2.y;
+                            any = p0.x | p0.y | p1.x | p1.y | p2.x | p2.y;
+                        }
+                        const uint64_t ci = cand_reserve(d, any != 0);
+                        if (any) {
+                            if (ci != ~0ull) {
+                                cand_write(d, ci, b, (A << KEY_SHIFT) | (win + e), row0 + row);
+                            } else {
+                                // an element seen when the row was read is ORed where it is
+                                const uint32_t s = w.slot[row][e];
+                                inserts++;
+                                if (s != 0xFFu)
+                                    g_or_into(d, w.rowoff[row] + s, b, d.rt.track[A]);
+                                else if (!g_insert(d, A, row0 + row, win + e, b, d.rt.track[A]))
+                                    atomicOr(&w.rowfail[row >> 5], 1u << (row & 31));
+                            }
+                        }
+                    }
+                    __syncthreads();
+                    win = w.next_w;
+                    todo = w.kmore;
+                    __syncthreads();
+                    if (win == EMPTY) break;
+                }
+            }
+            // ---- records left to k_join, and those of rows whose inserts failed
+            for (uint32_t i = tid; i < nr; i += TILE_THREADS) {
+                const uint32_t m = w.rmeta[i], row = m & 0xFFu;
+                const bool left = m & TM_LEFT, failed = (w.rowfail[row >> 5] >> (row & 31)) & 1u;
+                if (!left && !failed) continue;
+                uint4 r0, r1;
+                ld32(recs + 2 * (pos + i), r0, r1);
+                if (left) list_push(&d.ctr[C_LN], left_cap, left_out, r0, r1);
+                else list_push(&d.ctr[C_RETRY_N], d.retry_cap, retry_out, r0, r1);
+            }
+            pos += nr;
+            __syncthreads();
+        }
+    }
+    for (int o = 16; o; o >>= 1) {
+        n_left += __shfl_xor_sync(0xffffffffu, n_left, o);
+        n_right += __shfl_xor_sync(0xffffffffu, n_right, o);
+        inserts += __shfl_xor_sync(0xffffffffu, inserts, o);
+    }
+    if (lane == 0) {
+        if (n_left) atomicAdd(&d.ctr[C_LEFT], (unsigned long long)n_left);
+        if (n_right) atomicAdd(&d.ctr[C_RIGHT], (unsigned long long)n_right);
+        if (inserts) atomicAdd(&d.ctr[C_INSERTS], (unsigned long long)inserts);
+    }
+}
+
 // Small rounds: a warp joins 32 records, so a round of few, dense records (alias
 // rows reach a whole block) leaves most SMs idle. Below SPLIT_MAX records the
 // round's gathered and virtual records are cut into sub-records of at most
@@ -1172,14 +1782,16 @@ constexpr uint32_t SPLIT_MAX = 32768;
 constexpr uint32_t SPLIT_BITS = 8;
 constexpr uint32_t SPLIT_PARTS = (EIDS + SPLIT_BITS - 1) / SPLIT_BITS;
 
-__global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out)
+// tile: the rounds that are not split go through k_tile (C_TS: its rows), not k_join.
+__global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out, int tile)
 {
     if (d.ctr[C_HALT]) return;
     const uint64_t nd = d.ctr[C_DIRTY_N], nv = d.ctr[C_VN];
     const bool split = nd + nv < SPLIT_MAX;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        d.ctr[C_JN1] = split ? 0 : nd;
-        d.ctr[C_JN2] = split ? 0 : nv;
+        d.ctr[C_JN1] = split || tile ? 0 : nd;
+        d.ctr[C_JN2] = split || tile ? 0 : nv;
+        d.ctr[C_TS] = split || !tile ? 0 : tile_rows_lg(nd + nv);
     }
     if (!split) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nd + nv;
@@ -2139,6 +2751,9 @@ struct grg_ctx {
     uint4 *vbuf = nullptr;                     // virtual records of old-left joins
     uint64_t vbuf_cap = 0;
     uint4 *sbuf = nullptr;                     // sub-records of small rounds (k_split)
+    uint4 *lbuf = nullptr;                     // records that tiles leave to k_join
+    uint32_t *tlist = nullptr;                 // tiles of the round (lbuf_cap entries)
+    uint64_t lbuf_cap = 0;
     uint32_t *drs = nullptr, *drc = nullptr, *dvm = nullptr;   // delta index (per label x row / vertex bitmap)
     uint4 *cand[2] = {nullptr, nullptr};       // join candidates for k_apply / failed candidates
     uint64_t cand_cap = 0;
@@ -2591,6 +3206,8 @@ void grg_destroy(grg_ctx *c)
     cudaFree(c->gslot);
     cudaFree(c->vbuf);
     cudaFree(c->sbuf);
+    cudaFree(c->lbuf);
+    cudaFree(c->tlist);
     cudaFree(c->xbuf);
     cudaFree(c->xst);
     cudaFree(c->rowmark);
@@ -2793,7 +3410,7 @@ int alloc_tables(grg_ctx *c, const MinCap &mc, Hist hist, uint64_t *top, const u
     for (int attempt = 0;; attempt++) {
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_POOL_TOP, 0, 8, s));
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_ERR, 0, 8, s));
-        k_load_alloc<<<grid_for(c, c->ntables, 256), 256, 0, s>>>(make_dev(c), 0, c->V, (uint32_t)c->L, mc, rowmark);
+        k_load_alloc<<<alloc_grid(c->sms, (uint32_t)c->L, c->V), ALLOC_ROWS, 0, s>>>(make_dev(c), 0, c->V, (uint32_t)c->L, mc, rowmark);
         c->launches++;
         int st = read_ctr(c);
         if (st) return st;
@@ -3027,6 +3644,21 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
         k_join<WIN2, WIN2_LO><<<grid, JOIN_WARPS * 32, 0, s>>>(*dp, recs, n, n_ctr, retry_out);
     else
         k_join<WIN, WIN_LO><<<grid, JOIN_WARPS * 32, 0, s>>>(*dp, recs, n, n_ctr, retry_out);
+}
+
+// Rounds go through k_tile where a rule's second symbol is derivable (old-left joins): their right
+// rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 82.5 ms).
+// With static second symbols a right row is 1-2 elements and k_join's windows stay.
+static bool use_tiles(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
+
+// The tiles of a round's gathered and virtual records (counts on the device): list, then join.
+static void launch_tiles(int sms, cudaStream_t s, const Dev &d, const uint4 *grecs, const uint4 *vrecs, uint32_t *list,
+                         uint4 *left, uint64_t cap, uint4 *retry_out, uint32_t sh)
+{
+    cudaMemsetAsync(d.ctr + C_TN, 0, 24, s);                    // tiles, tile queue, records left to k_join
+    cudaFuncSetAttribute(k_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
+    k_tile_starts<<<sms * 8, 256, 0, s>>>(d, grecs, vrecs, list, cap, sh);
+    k_tile<<<sms, TILE_THREADS, sizeof(TileSmem), s>>>(d, grecs, vrecs, list, cap, left, cap, retry_out, sh);
 }
 
 static bool any_csr(const grg_ctx *c)
@@ -3387,6 +4019,13 @@ static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv,
                     C_SPLIT_N, c->rbuf[0], joins);
         return;
     }
+    if (use_tiles(c)) {
+        launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], tile_rows_lg(nd + nv));
+        launch_join(c, grid_for(c, (nd + nv + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_LN, c->rbuf[0]);
+        c->launches += 3;
+        joins += 2;
+        return;
+    }
     launch_pass(c, grid_for(c, (nd + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
     if (nv) {
         // virtual old-left records: joined by source rows only
@@ -3460,7 +4099,6 @@ static int round_retries(grg_ctx *c, uint64_t nr, uint64_t nf, grg_stats &S, dou
     }
 }
 
-// First join pass of a round over its nd gathered and nv virtual records, then retries.
 static int ensure_sbuf(grg_ctx *c)
 {
     if (c->sbuf) return GRG_OK;
@@ -3468,6 +4106,23 @@ static int ensure_sbuf(grg_ctx *c)
     return GRG_OK;
 }
 
+// Buffers of k_tile: a tile starts at one record, and a record is left to k_join once at most.
+static int ensure_tiles(grg_ctx *c)
+{
+    const uint64_t n = c->gbuf_cap + c->vbuf_cap;
+    if (!use_tiles(c) || n <= c->lbuf_cap) return GRG_OK;
+    cudaFree(c->lbuf);
+    cudaFree(c->tlist);
+    c->lbuf = nullptr;
+    c->tlist = nullptr;
+    c->lbuf_cap = 0;
+    GRG_CUDA(c, cudaMalloc(&c->lbuf, n * 32));
+    GRG_CUDA(c, cudaMalloc(&c->tlist, n * 4));
+    c->lbuf_cap = n;
+    return GRG_OK;
+}
+
+// First join pass of a round over its nd gathered and nv virtual records, then retries.
 static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, double &join_ms, uint64_t &joins)
 {
     cudaStream_t s = c->stream;
@@ -3475,12 +4130,13 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
     int st = ensure_rbuf(c, retry_room(c, nd + nv));
     if (st) return st;
     if (split && (st = ensure_sbuf(c))) return st;
+    if ((st = ensure_tiles(c))) return st;
     Dev d = make_dev(c);
     if (c->timing) GRG_CUDA(c, cudaEventRecord(c->ev_c, s));
     if (split) {
         // few records: their parts spread the join over more warps
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_SPLIT_N, 0, 8, s));
-        k_split<<<grid_for(c, nd + nv, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf);
+        k_split<<<grid_for(c, nd + nv, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, 0);
         c->launches++;
     }
     if (c->tune_pending && c->need_join && !split && nd >= TUNE_MIN_RECORDS) {
@@ -3590,7 +4246,7 @@ static std::vector<uint64_t> round_graph_key(const grg_ctx *c, uint32_t rs, uint
                                (uint64_t)c->elem_loaded, (uint64_t)c->rt.nol, (uint64_t)c->row_job,
                                (uint64_t)c->job_cnt, c->max_jobs, (uint64_t)c->join_wide, (uint64_t)c->sbuf,
                                (uint64_t)c->need_join, (uint64_t)c->need_push, (uint64_t)c->push_flat,
-                               (uint64_t)c->join_elems};
+                               (uint64_t)c->join_elems, (uint64_t)c->lbuf, (uint64_t)c->tlist, c->lbuf_cap};
     for (int l = 1; l <= c->L; l++) k.push_back(c->rt.dindex[l]);
     // the rule table is a parameter of every recorded launch
     uint64_t w[(sizeof(RuleTable) + 7) / 8] = {0};
@@ -3670,17 +4326,24 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
     }
     const int jgrid = grid_for(c, ~0u, JOIN_WARPS, 16);
     cudaMemsetAsync(ctr + C_SPLIT_N, 0, 8, s);
-    k_split<<<grid_for(c, SPLIT_MAX, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf);
+    const bool tiles = use_tiles(c);
+    k_split<<<grid_for(c, SPLIT_MAX, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles);
     nk++;
     {
         const uint64_t launches0 = c->launches;
         uint64_t unused = 0;
-        launch_pass(c, jgrid, s, d, c->gbuf, 0, C_JN1, c->rbuf[0], unused);
+        if (tiles) {
+            launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], 0);
+            launch_join(c, jgrid, s, d, c->lbuf, 0, C_LN, c->rbuf[0]);
+            nk += 3;
+        } else {
+            launch_pass(c, jgrid, s, d, c->gbuf, 0, C_JN1, c->rbuf[0], unused);
+        }
         launch_pass(c, jgrid, s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0], unused);
         nk += (int)(c->launches - launches0);
         c->launches = launches0;
     }
-    if (c->rt.nol) {
+    if (c->rt.nol && !tiles) {
         launch_join(c, jgrid, s, d, c->vbuf, 0, C_JN2, c->rbuf[0]);
         nk++;
     }
@@ -3748,6 +4411,7 @@ static int run_rounds(grg_ctx *c, uint64_t max_rounds, grg_stats &S, double &joi
         if ((st = ensure_cand(c, 2 * nd_last))) return st;    // a full candidate buffer falls back to direct inserts
         if ((st = ensure_rbuf(c, retry_room(c, c->gbuf_cap + (c->rt.nol ? c->vbuf_cap : 0))))) return st;
         if ((st = ensure_sbuf(c))) return st;
+        if ((st = ensure_tiles(c))) return st;
         if ((st = build_round_graph(c, rs))) return st;
         c->cb = 0;
         // the delta index starts clear: inside the graph each round clears what the previous
@@ -4536,7 +5200,7 @@ int grg_batch_admit(grg_ctx *c, uint32_t job, uint32_t base, uint32_t num_vars, 
                                                                 c->tmask);
     for (int l = 1; l <= c->L; l++)
         if ((eps_mask >> (l - 1)) & 1ull) k_eps_hist<<<grid_for(c, num_vars, 256), 256, 0, s>>>(d, (uint32_t)l, base, num_vars);
-    k_load_alloc<<<grid_for(c, (uint64_t)c->L * num_vars, 256), 256, 0, s>>>(d, base, num_vars, (uint32_t)c->L, mc,
+    k_load_alloc<<<alloc_grid(c->sms, (uint32_t)c->L, num_vars), ALLOC_ROWS, 0, s>>>(d, base, num_vars, (uint32_t)c->L, mc,
                                                                               nullptr);
     st = read_ctr(c);
     if (st) return st;
@@ -4668,6 +5332,8 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH
 // Device address of g_noalloc_scratch per device ordinal, looked up once per
 // device with that device current (the host-side symbol is not a device address).
 static void *g_noalloc_addr[256];
+
+constexpr uint64_t NOALLOC_TILE_MIN = 512;   // records of a round that goes through k_tile
 
 static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -4802,13 +5468,12 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
     NA_CUDA(cudaMemsetAsync(d.dvm, 0, (uint64_t)num_labels * vwords * 4, s));
 
     // load (grg_load_edges)
-    const uint64_t nlab = (uint64_t)num_labels * num_vars;
     if (num_edges) k_load_hist<<<grid(num_edges, 256, 8), 256, 0, s>>>(d, d_src, d_dst, d_label, num_edges, 0, num_vars, (uint32_t)num_labels, 0ull);
     for (int q = 0; q < num_rules; q++)
         if (rules[3 * q + 1] == 0) k_eps_hist<<<grid(num_vars, 256, 8), 256, 0, s>>>(d, (uint32_t)rules[3 * q], 0, num_vars);
     MinCap mc;
     memset(&mc, 0, sizeof mc);
-    k_load_alloc<<<grid(nlab, 256, 8), 256, 0, s>>>(d, 0, num_vars, (uint32_t)num_labels, mc, nullptr);
+    k_load_alloc<<<alloc_grid(sms, (uint32_t)num_labels, num_vars), ALLOC_ROWS, 0, s>>>(d, 0, num_vars, (uint32_t)num_labels, mc, nullptr);
     if ((st = na_read(h, d.ctr, s))) return st;
     if (h[C_BADIN] & ERR_IN_LABEL) return GRG_E_LABEL;
     if (h[C_BADIN] & ERR_IN_RANGE) return GRG_E_RANGE;
@@ -4838,6 +5503,8 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
         k_scan_sums<<<1, 1024, 0, s>>>(csum, nb, nullptr);
         k_scan_add<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(coff, csum, nchunks, nullptr);
         uint32_t nd32 = 0;
+        NA_CUDA(cudaMemsetAsync(d.ctr + C_DIRTY_N, 0, 8, s));
+        NA_CUDA(cudaMemcpyAsync(d.ctr + C_DIRTY_N, csum + nb, 4, cudaMemcpyDeviceToDevice, s));
         NA_CUDA(cudaMemcpyAsync(&nd32, csum + nb, 4, cudaMemcpyDeviceToHost, s));
         NA_CUDA(cudaStreamSynchronize(s));
         const uint64_t nd = nd32;
@@ -4866,7 +5533,13 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
         for (int pass = 0;; pass++) {
             const int g = grid((n + RB - 1) / RB, JOIN_WARPS, 16);
             // each join launch pulls 32-record batches from a queue that starts at 0
-            if (pass == 0) {
+            if (pass == 0 && rt.nol && nd + nv >= NOALLOC_TILE_MIN) {
+                // gslot and rbuf[1] are free in this pass: the tile list and the records left to k_join
+                launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0], tile_rows_lg(nd + nv));
+                NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
+                k_join<WIN, WIN_LO><<<grid((nd + nv + RB - 1) / RB, JOIN_WARPS, 16), JOIN_WARPS * 32, 0, s>>>(
+                    d, rbuf[1], 0, C_LN, rbuf[0]);
+            } else if (pass == 0) {
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
                 k_join<WIN, WIN_LO><<<g, JOIN_WARPS * 32, 0, s>>>(d, gbuf, nd, -1, rbuf[0]);
                 if (nv) {

@@ -30,3 +30,31 @@ def test_counts_and_hash_by_row_groups(grg_mod, oracle_mod, nv):
     assert np.sum([p[0] for p in parts], axis=0).tolist() == counts
     assert sum(p[1] for p in parts) % (1 << 64) == r.set_hash
     ctx.close()
+
+
+@pytest.mark.parametrize("nv,block,density", [(40, 40, 3), (700, 129, 4), (9_000, 1000, 4), (30_000, 383, 3),
+                                              (3_500, 0, 2), (60_000, 1100, 2)])
+def test_tiled_joins(grg_mod, oracle_mod, nv, block, density):
+    """Grammars with a derivable second symbol join tiles of neighbouring rows. Blocks of a few ids,
+    of more ids than one window of 8 elements holds (unconfined rows and their further windows), and
+    of fewer records than a tile pays for give the oracle's closure, whole, alone and in a batch."""
+    w = G.alias(seed=nv + block, num_vars=nv, num_base_edges=density * nv, block=block or None)
+    r = oracle_mod.closure(nv, w.rule_ids(), w.num_labels, 0, w.src, w.dst, w.lab)
+    want = (r.label_counts().tolist(), r.set_hash)
+    for dev in (True, False):
+        ctx = grg_mod.Context(0)
+        ctx.set_device_rounds(dev)
+        ctx.transfer_rules(w.rule_ids(), w.num_labels)
+        ctx.load_edges(nv, w.src, w.dst, w.lab)
+        ctx.closure(0)
+        assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
+        ctx.close()
+    ctx = grg_mod.Context(0)
+    b = grg_mod.Batch(ctx, 2 * nv, 2, [(w.rules, w.labels)], 0)
+    for j in (0, 1):
+        b.admit(j, j * nv, 0, nv, w.src, w.dst, w.lab)
+    b.step(0)
+    for j in (0, 1):
+        c, h = b.result(j, 0)
+        assert (c.tolist(), h) == want
+    ctx.close()
