@@ -1,6 +1,7 @@
 // grg_engine.cu -- CUDA kernels and the C ABI of the closure engine (sm_103a).
 //
 // Hot path (reference: src/kernel.cu):
+//   k_rows    the same joins for grammars whose right-hand labels are all static (CSR copies).
 //   k_tile    the same joins for grammars with a derivable right-hand label, over tiles of
 //             neighbouring rows (dense rows, read once a tile); leaves the rest to k_join.
 //   k_join    binary joins A ::= B C for a round's delta records, delta-left
@@ -2169,6 +2170,286 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
     flush_counters();
 }
 
+// ---------------------------------------------------------------- row joins
+//
+// Grammars without old-left joins (dataflow: N ::= N e) join every record with short static rows:
+// a few destinations an intermediate, in the labels' CSR copies. k_join spends 17 warp instructions
+// on such a (record, k) pair -- the search for the record of a flattened task, the choice between
+// item forms, a division a destination, a hash for what its window of 12 elements cannot hold. k_rows
+// does only what these joins need: a batch's set bits are written down as a list of tasks once, the
+// destinations of 32 tasks at a time are dealt over the lanes, and a destination's place in a window
+// is its distance from the window's first id. The warp's ROWS_ELEMS window elements are split over
+// the batch's runs of a row's records: 8 windows of 12 elements (4 of 24 when they are few) for rows
+// within a procedure, and all 96 for a row whose records spread wider (an unconfined graph's row of
+// 52 elements, or one that reaches several blocks, sent most of its items to k_join's hash). What
+// even that leaves out becomes a candidate of one bit. Bound by integer issue (2.3 of 2-4 warp
+// instructions a clock, 13 a pair). Closures: 10k vertices unconfined 11.1 -> 7.8 ms, 97k in blocks
+// 6.2 -> 5.8 ms, 2M in blocks 53.5 -> 48.7 ms (at 8 blocks a SM 48.8, at 6 51.3, at 10 56.4).
+constexpr int ROWS_WARPS = 4;
+constexpr int ROWS_ELEMS = 96;
+constexpr int ROWS_LIST = 512;                 // tasks listed at once
+constexpr int ROWS_QUEUE = 96;                 // destinations outside the windows held for a common write
+constexpr int ROWS_NEAR = 7;                   // elements of a narrow run: a procedure of 1,000 ids
+#ifndef GRG_ROWS_MINB
+#define GRG_ROWS_MINB 7
+#endif
+
+struct __align__(16) RowsSmem {
+    uint32_t win[ROWS_ELEMS * EW];
+    uint4 rows[32];                            // a chunk's non-empty right rows: where its items are, the
+                                               // run's window (first id, first bit in win), record
+    uint2 beyond[ROWS_QUEUE];                  // destinations outside the windows: id, record
+    uint16_t list[ROWS_LIST];                  // record << 8 | position of its bit
+    uint8_t first[8];                          // the first record of each window's run
+};
+
+__global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
+    k_rows(Dev d, const uint4 *__restrict__ recs, uint64_t n, int n_ctr, uint4 *retry_out)
+{
+    if (d.ctr[C_HALT]) return;
+    if (n_ctr >= 0) n = d.ctr[n_ctr];
+    __shared__ RowsSmem smem[ROWS_WARPS];
+    RowsSmem &w = smem[threadIdx.x >> 5];
+    const uint32_t lane = lane_id();
+    for (int j = lane; j < ROWS_ELEMS * EW; j += 32) w.win[j] = 0;
+    __syncwarp();
+    const uint32_t nbases = (d.V + EIDS - 1) / EIDS;
+    const unsigned lt = (1u << lane) - 1u, le = 0xFFFFFFFFu >> (31 - lane);
+    uint32_t n_left = 0, n_right = 0, n_out = 0, inserts = 0;
+    auto flush_counters = [&]() {
+        unsigned long long s[4] = {inserts, n_left, n_right, n_out};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            for (int o = 16; o; o >>= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+        if (lane == 0) {
+            if (s[0]) atomicAdd(&d.ctr[C_INSERTS], s[0]);
+            if (s[1]) atomicAdd(&d.ctr[C_LEFT], s[1]);
+            if (s[2]) atomicAdd(&d.ctr[C_RIGHT], s[2]);
+            if (s[3]) atomicAdd(&d.ctr[C_WOUT], s[3]);
+        }
+        inserts = n_left = n_right = n_out = 0;
+    };
+    const uint64_t nbatch = (n + RB - 1) / RB;
+    uint64_t bt = 0;
+    if (lane == 0) bt = atomicAdd(&d.ctr[C_JQ], 1ull);
+    bt = __shfl_sync(0xffffffffu, bt, 0);
+    for (; bt < nbatch; bt = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(&d.ctr[C_JQ], 1ull) : 0ull, 0)) {
+        const uint64_t ri = bt * RB + lane;
+        const bool have = ri < n;
+        uint4 ra = make_uint4(0, 0, 0, 0), rb = make_uint4(0, 0, EMPTY, 0);
+        if (have) ld32(recs + 2 * ri, ra, rb);
+        const Bits bits = {{ra.x, ra.y, ra.z, ra.w, rb.x, rb.y}};
+        const uint32_t key = rb.z, row = rb.w, lab = key >> KEY_SHIFT, base = key & BASE_MASK;
+        const bool real = have && lab >= 1 && lab <= (uint32_t)d.rt.L;
+        const uint32_t B = real ? lab : 0;
+        // runs of records of one row and label (a table's records are contiguous)
+        const uint32_t prow = __shfl_up_sync(0xffffffffu, row, 1), pB = __shfl_up_sync(0xffffffffu, B, 1);
+        const bool start = lane == 0 || !have || B == 0 || prow != row || pB != B;
+        const unsigned sm = __ballot_sync(0xffffffffu, start);
+        const uint32_t lead = 31 - __clz(sm & (0xFFFFFFFFu >> (31 - lane)));
+        // the lowest and highest block of intermediates of each run
+        const uint32_t nlead = sm & (0xFFFFFFFEu << lane) ? __ffs(sm & (0xFFFFFFFEu << lane)) - 1 : 32u;  // next run
+        uint32_t lo = base, hi = base;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t l2 = __shfl_down_sync(0xffffffffu, lo, o), h2 = __shfl_down_sync(0xffffffffu, hi, o);
+            if (lane + o < nlead) {
+                lo = min(lo, l2);
+                hi = max(hi, h2);
+            }
+        }
+        lo = __shfl_sync(0xffffffffu, lo, lead);
+        hi = __shfl_sync(0xffffffffu, hi, lead);
+        // windows: a run's destinations are taken to lie as far around its intermediates as a group of
+        // ROWS_NEAR elements that holds them all reaches; runs in more than that get the warp's
+        // whole window to themselves, in a pass of their own
+        const bool wide = hi - lo >= (uint32_t)ROWS_NEAR;
+        const uint32_t narrow = __popc(__ballot_sync(0xffffffffu, start && real && !wide));
+        bool ok = true;
+        unsigned fail = 0;                         // first records of runs with a failed insert
+        // unary rules A ::= B
+        const uint32_t nu = real ? d.rt.un_start[B + 1] - d.rt.un_start[B] : 0;
+        const uint32_t maxu = __reduce_max_sync(0xffffffffu, nu);
+        for (uint32_t u = 0; u < maxu; u++)
+            if (u < nu) {
+                const uint32_t A = d.rt.un_A[d.rt.un_start[B] + u];
+                ok &= g_insert(d, A, row, base, bits, d.rt.track[A]);
+                inserts++;
+            }
+        const uint32_t nbr_rec = real ? d.rt.bin_start[B + 1] - d.rt.bin_start[B] : 0;
+        const uint32_t nbits = popc6(bits), k0 = base * EIDS;
+        // passes: the narrow runs, 8 (or, when they are few, 4) at a time, then each wide run
+        const unsigned nm = __ballot_sync(0xffffffffu, start && real && !wide), wm = __ballot_sync(0xffffffffu, start && real && wide);
+        const uint32_t nrank = __popc(nm & ((1u << lead) - 1u)), wrank = __popc(wm & ((1u << lead) - 1u));
+        const uint32_t nslots = narrow <= 4 ? 4u : 8u, npass = (narrow + nslots - 1) / nslots;
+        for (uint32_t pass = 0; pass < npass + __popc(wm); pass++) {
+            const bool wpass = pass >= npass;
+            const uint32_t slots = wpass ? 1u : nslots, width = ROWS_ELEMS / slots;
+            const uint32_t slot = wpass ? wrank - (pass - npass) : nrank - pass * nslots;   // (huge: another pass's)
+            const bool act = real && wide == wpass && slot < slots;
+            const uint32_t nbr = act ? nbr_rec : 0;
+            const uint32_t maxb = __reduce_max_sync(0xffffffffu, nbr);
+            if (!maxb) continue;
+            // the first element of the run's window. Windows lie one after the other in w.win as plain
+            // bitmaps (an element is 6 words), so a destination's place is its distance from the window's
+            // first id: no division by 192
+            const uint32_t room = wpass ? (uint32_t)ROWS_ELEMS - min(hi - lo + 1, (uint32_t)ROWS_ELEMS) : 0u;
+            const uint32_t ws = wpass ? (nbases <= (uint32_t)ROWS_ELEMS ? 0u : lo - room / 2)
+                                      : hi - (ROWS_NEAR - 1) - (width - 2 * ROWS_NEAR + 2) / 2;
+            const uint32_t id0 = ws * EIDS, span = width * EIDS, at0 = slot * span;
+            if (start && act) w.first[slot] = (uint8_t)lane;
+            for (uint32_t rho = 0; rho < maxb; rho++) {
+                const bool hr = rho < nbr;
+                const uint32_t q = d.rt.bin_start[B] + rho;
+                const uint32_t A = hr ? d.rt.bin_A[q] : 0, myC = hr ? d.rt.bin_C[q] : 0;
+                n_left += hr;
+                // one right-hand label at a time (nearly always the only one)
+                for (unsigned todo = __ballot_sync(0xffffffffu, hr); todo;) {
+                    const uint32_t C = __shfl_sync(0xffffffffu, myC, __ffs(todo) - 1);
+                    const bool mine = hr && myC == C;
+                    todo &= ~__ballot_sync(0xffffffffu, mine);
+                    const uint2 *rowp = d.rt.csr_row[C];
+                    const uint32_t *colp = d.rt.csr_col[C];
+                    const uint32_t my_cnt = mine ? nbits : 0;
+                    uint32_t incl = my_cnt;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= (uint32_t)o) incl += y;
+                    }
+                    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                    uint32_t nx = incl - my_cnt;                   // my next task
+                    uint32_t m[EW];
+#pragma unroll
+                    for (int x = 0; x < EW; x++) m[x] = mine ? bits.w[x] : 0;
+                    // destinations outside the windows: candidates of one bit
+                    uint32_t nq = 0;
+                    auto flush_beyond = [&]() {
+                        __syncwarp();
+                        for (uint32_t i = 0; i < nq; i += 32) {
+                            const bool v = i + lane < nq;
+                            const uint2 e = v ? w.beyond[i + lane] : make_uint2(0, 0);
+                            const uint32_t oA = __shfl_sync(0xffffffffu, A, e.y), orow = __shfl_sync(0xffffffffu, row, e.y);
+                            const uint64_t ci = cand_reserve(d, v);
+                            if (!v) continue;
+                            const uint32_t b = e.x / EIDS, o = e.x - b * EIDS;
+                            Bits ob;
+#pragma unroll
+                            for (int x = 0; x < EW; x++) ob.w[x] = (uint32_t)x == (o >> 5) ? 1u << (o & 31) : 0u;
+                            n_out++;
+                            if (ci != ~0ull) {
+                                cand_write(d, ci, ob, (oA << KEY_SHIFT) | b, orow);
+                            } else {
+                                inserts++;
+                                if (!g_insert(d, oA, orow, b, ob, d.rt.track[oA])) fail |= 1u << e.y;
+                            }
+                        }
+                        __syncwarp();
+                        nq = 0;
+                    };
+                    for (uint32_t t0 = 0; t0 < total; t0 += ROWS_LIST) {
+                        __syncwarp();
+#pragma unroll
+                        for (int x = 0; x < EW; x++)
+                            while (m[x] && nx - t0 < (uint32_t)ROWS_LIST) {
+                                w.list[nx - t0] = (uint16_t)(lane << 8 | (x * 32 + __ffs(m[x]) - 1));
+                                m[x] &= m[x] - 1;
+                                nx++;
+                            }
+                        __syncwarp();
+                        const uint32_t nt = min(total - t0, (uint32_t)ROWS_LIST);
+                        for (uint32_t f = 0; f < nt; f += 32) {
+                            const bool valid = f + lane < nt;
+                            const uint32_t e = valid ? w.list[f + lane] : 0, r = e >> 8;
+                            const uint32_t k = __shfl_sync(0xffffffffu, k0, r) + (e & 0xFFu);
+                            const uint32_t tid0 = __shfl_sync(0xffffffffu, id0, r), tat0 = __shfl_sync(0xffffffffu, at0, r);
+                            uint2 rw = make_uint2(0, 0);
+                            if (valid) rw = __ldg(rowp + k);
+                            const uint32_t deg = rw.y & 0xFFFFFFu;
+                            n_right += rw.y >> 24;
+                            // the rows' destinations, dealt over the lanes: item g of the chunk belongs to the
+                            // last non-empty row that starts at or before it
+                            uint32_t inc = deg;
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                                if (lane >= (uint32_t)o) inc += y;
+                            }
+                            const uint32_t items = __shfl_sync(0xffffffffu, inc, 31), s1 = inc - deg;
+                            const unsigned some = __ballot_sync(0xffffffffu, deg != 0);
+                            __syncwarp();
+                            if (deg) w.rows[__popc(some & lt)] = make_uint4(rw.x - s1, tid0, tat0, r);
+                            __syncwarp();
+                            int at = -1;                       // the last row that starts before item g0
+                            for (uint32_t g0 = 0; g0 < items; g0 += 32) {
+                                const unsigned st = __reduce_or_sync(0xffffffffu, deg && s1 - g0 < 32u ? 1u << (s1 - g0) : 0u);
+                                const uint4 rr = w.rows[at + __popc(st & le)];
+                                at += __popc(st);
+                                const bool v = g0 + lane < items;
+                                uint32_t id = 0;
+                                if (v) id = __ldg(colp + (uint32_t)(rr.x + g0 + lane));
+                                const uint32_t rel = id - rr.y;
+                                const bool in = rel < span;
+                                if (v && in) atomicOr(&w.win[(rel + rr.z) >> 5], 1u << (rel & 31));
+                                const unsigned out = __ballot_sync(0xffffffffu, v && !in);
+                                if (out) {
+                                    if (v && !in) w.beyond[nq + __popc(out & lt)] = make_uint2(id, rr.w);
+                                    nq += __popc(out);
+                                    if (nq > ROWS_QUEUE - 32) flush_beyond();
+                                }
+                            }
+                        }
+                    }
+                    if (nq) flush_beyond();
+                }
+                // the windows' elements go out as candidates (or, without room, into the tables)
+                __syncwarp();
+                uint32_t nz = 0;
+#pragma unroll
+                for (int it = 0; it < ROWS_ELEMS / 32; it++) {
+                    const uint2 *p = reinterpret_cast<const uint2 *>(w.win + (it * 32 + lane) * EW);
+                    const uint2 p0 = p[0], p1 = p[1], p2 = p[2];
+                    if (p0.x | p0.y | p1.x | p1.y | p2.x | p2.y) nz |= 1u << it;
+                }
+                uint64_t ci = cand_reserve(d, __popc(nz));
+#pragma unroll 1
+                for (int it = 0; it < ROWS_ELEMS / 32; it++) {
+                    const uint32_t el = it * 32 + lane, sl = el / width, fr = w.first[min(sl, slots - 1)] & 31u;
+                    const uint32_t oA = __shfl_sync(0xffffffffu, A, fr), orow = __shfl_sync(0xffffffffu, row, fr);
+                    const uint32_t ob = __shfl_sync(0xffffffffu, ws, fr) + (el - sl * width);
+                    if (!((nz >> it) & 1u)) continue;
+                    uint2 *p = reinterpret_cast<uint2 *>(w.win + el * EW);
+                    const uint2 p0 = p[0], p1 = p[1], p2 = p[2];
+                    p[0] = p[1] = p[2] = make_uint2(0, 0);
+                    const Bits b = {{p0.x, p0.y, p1.x, p1.y, p2.x, p2.y}};
+                    if (ci != ~0ull) {
+                        cand_write(d, ci++, b, (oA << KEY_SHIFT) | ob, orow);
+                    } else {
+                        inserts++;
+                        if (!g_insert(d, oA, orow, ob, b, d.rt.track[oA])) fail |= 1u << fr;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        // a failed insert re-runs the records of its run (of the record, for a unary rule or a
+        // destination outside the window)
+        fail = __reduce_or_sync(0xffffffffu, fail);
+        const bool failed = have && (!ok || ((fail >> lead) & 1u) || ((fail >> lane) & 1u));
+        const unsigned fm = __ballot_sync(0xffffffffu, failed);
+        if (fm) {
+            unsigned long long p = 0;
+            if (lane == (uint32_t)(__ffs(fm) - 1)) p = atomicAdd(&d.ctr[C_RETRY_N], (unsigned long long)__popc(fm));
+            p = __shfl_sync(0xffffffffu, p, __ffs(fm) - 1);
+            const uint64_t o = p + __popc(fm & ((1u << lane) - 1u));
+            if (failed && o < d.retry_cap) st32(retry_out + 2 * o, ra, rb);
+        }
+        if (__any_sync(0xffffffffu, (n_left | n_right | n_out | inserts) >> 30)) flush_counters();
+        __syncwarp();
+    }
+    flush_counters();
+}
+
 // Tables of labels 1..L by log2 of their occupied elements (buckets 0..7, the
 // last open-ended) into C_DH0..C_DH0+7: the degree distribution that keys the
 // join-window tuning.
@@ -2785,6 +3066,7 @@ struct grg_ctx {
     int items_mode = 2;                    // 0 ids, 1 elements, 2 tuned per degree key, 3 re-measured
     bool join_elems = false;               // the form of this closure
     bool tuned_elems = false;
+    bool join_rows = false;                // this closure's joins run k_rows (see rows_possible)
     float items_ms[2] = {0, 0};            // measured (ids, elements) when tuned in this closure
     bool tune_pending = false;             // measure both windows in the first large round
     uint64_t tune_key = 0;
@@ -3617,10 +3899,26 @@ __global__ void k_tmark(unsigned long long *ctr, int t0_slot, int acc_slot, int 
 // an SM. Earlier layouts, measured on one box (2M-vertex dataflow / 1M alias
 // closure): 16 slots with runs past the 16th in the hash, 10-element windows, 7
 // blocks 54.4 / 317 ms; 32 slots (one per record) at 5 blocks 66.3 / 334 ms.
+// Joins that k_rows can run: no old-left joins (so no derivable right-hand label), no pushes, and a
+// CSR copy of every right-hand label (a batch has none, nor a label with a row of 2^24 ids). A fixed
+// window or item form is k_join's.
+static bool rows_possible(const grg_ctx *c)
+{
+    if (c->rt.nol || c->need_push) return false;
+    bool any = false;
+    for (int B = 1; B <= c->L; B++)
+        for (int q = c->rt.bin_start[B]; q < c->rt.bin_start[B + 1]; q++) {
+            if (!c->rt.csr_row[c->rt.bin_C[q]]) return false;
+            any = true;
+        }
+    return any;
+}
+
 static void choose_window(grg_ctx *c)
 {
     c->join_wide = c->join_window_mode >= 2 ? c->tuned_wide : c->join_window_mode != 0;
     c->join_elems = c->items_mode >= 2 ? c->tuned_elems : c->items_mode != 0;
+    c->join_rows = c->join_window_mode >= 2 && c->items_mode >= 2 && rows_possible(c);
     c->push_flat = c->push_mode >= 2 ? c->tuned_flat : c->push_mode != 0;
 }
 
@@ -3631,13 +3929,18 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
 {
     const Dev *dp = &d;
     Dev de;
-    if (c->join_elems) {
+    if (c->join_elems && !c->join_rows) {
         de = d;
         for (int l = 0; l <= MAX_LABELS; l++) de.rt.csr_row[l] = nullptr;
         dp = &de;
     }
     // the launch's work queue starts at batch 0; the grid is what the SMs hold at once
     cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s);
+    if (c->join_rows) {
+        const int g = std::min(grid, c->sms * GRG_ROWS_MINB);
+        k_rows<<<g, ROWS_WARPS * 32, 0, s>>>(d, recs, n, n_ctr, retry_out);
+        return;
+    }
     const int resident = c->sms * (c->join_wide ? GRG_JOIN_MINB_WIDE : GRG_JOIN_MINB);
     if (grid > resident) grid = resident;
     if (c->join_wide)
@@ -3652,6 +3955,7 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
 static bool use_tiles(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
 
 // The tiles of a round's gathered and virtual records (counts on the device): list, then join.
+// sh: log2 of a tile's rows, 0 = from the device.
 static void launch_tiles(int sms, cudaStream_t s, const Dev &d, const uint4 *grecs, const uint4 *vrecs, uint32_t *list,
                          uint4 *left, uint64_t cap, uint4 *retry_out, uint32_t sh)
 {
@@ -3820,7 +4124,8 @@ static int tune_first_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, u
     // right-hand label has a CSR copy; an untimed pass, then every combination twice,
     // interleaved, keeping each one's best time
     const bool tw = c->join_window_mode >= 2, ti = c->items_mode >= 2 && any_csr(c);
-    const bool fix_wide = c->join_wide, fix_elems = c->join_elems;
+    const bool fix_wide = c->join_wide, fix_elems = c->join_elems, rows = c->join_rows;
+    c->join_rows = false;                    // (k_rows has neither windows nor item forms to choose)
     float best[2][2] = {{1e30f, 1e30f}, {1e30f, 1e30f}};        // [wide][elems]
     for (int rep = -1; rep < 2; rep++)
         for (int w = 0; w < 2; w++)
@@ -3840,6 +4145,7 @@ static int tune_first_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, u
                 GRG_CUDA(c, cudaEventElapsedTime(&ms, c->ev_t0, c->ev_t1));
                 best[w][e] = std::min(best[w][e], ms);
             }
+    c->join_rows = rows;
     // the statistics count the round's own pass only
     for (int i = 0; i < 5; i++) {
         c->h_ctr[kept[i]] = keep[i];
@@ -4246,7 +4552,7 @@ static std::vector<uint64_t> round_graph_key(const grg_ctx *c, uint32_t rs, uint
                                (uint64_t)c->elem_loaded, (uint64_t)c->rt.nol, (uint64_t)c->row_job,
                                (uint64_t)c->job_cnt, c->max_jobs, (uint64_t)c->join_wide, (uint64_t)c->sbuf,
                                (uint64_t)c->need_join, (uint64_t)c->need_push, (uint64_t)c->push_flat,
-                               (uint64_t)c->join_elems, (uint64_t)c->lbuf, (uint64_t)c->tlist, c->lbuf_cap};
+                               (uint64_t)c->join_elems, (uint64_t)c->join_rows, (uint64_t)c->lbuf, (uint64_t)c->tlist, c->lbuf_cap};
     for (int l = 1; l <= c->L; l++) k.push_back(c->rt.dindex[l]);
     // the rule table is a parameter of every recorded launch
     uint64_t w[(sizeof(RuleTable) + 7) / 8] = {0};

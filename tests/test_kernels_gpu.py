@@ -58,3 +58,28 @@ def test_tiled_joins(grg_mod, oracle_mod, nv, block, density):
         c, h = b.result(j, 0)
         assert (c.tolist(), h) == want
     ctx.close()
+
+
+@pytest.mark.parametrize("kind,nv,block,ne,f", [
+    ("small", 50, 0, 120, 0),            # one element a row
+    ("small", 3_000, 0, 9_000, 0),       # 16 elements a row: two runs a batch, one window of 96
+    ("small", 19_500, 0, 40_000, 0),     # rows of more elements than the widest window
+    ("blocks", 64, 500, 1500, 1),        # narrow rows, and exits that reach five blocks
+    ("blocks", 40, 1001, 3003, 0),
+])
+def test_row_joins(grg_mod, oracle_mod, kind, nv, block, ne, f):
+    """Grammars with static right-hand rows: every window width, rows wider than all of them, small
+    rounds cut into sub-records, and pools small enough that inserts fail and run again."""
+    w = (G.dataflow_small(seed=nv, num_vars=nv, num_edges=ne) if kind == "small"
+         else G.dataflow_blocks(seed=nv, num_blocks=nv, block=block, num_edges=ne * nv, seed_n=f == 1))
+    r = oracle_mod.closure(w.num_vars, w.rule_ids(), w.num_labels, f, w.src, w.dst, w.lab)
+    want = (r.label_counts().tolist(), r.set_hash)
+    for dev, pool in ((True, 0), (False, 0), (True, 1 << 18)):
+        ctx = grg_mod.Context(0)
+        ctx.set_device_rounds(dev)
+        ctx.transfer_rules(w.rule_ids(), w.num_labels)
+        ctx.allocate_pool(pool)
+        ctx.load_edges(w.num_vars, w.src, w.dst, w.lab)
+        st = ctx.closure(f)
+        assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
+        ctx.close()
