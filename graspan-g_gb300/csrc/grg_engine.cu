@@ -575,28 +575,34 @@ __global__ void k_dindex_clear(Dev d, const uint4 *__restrict__ recs, int n_ctr)
 // masked to the vertices k whose row C[k] has deltas this round, becomes a
 // virtual delta record (label slot OL_SLOT0 + q). The 192 ids of an element are
 // exactly 6 words of the dirty-vertex bitmap. Records past cap are counted only.
-// A block takes OL_ROWS consecutive rows and writes their records together, in
-// row order (the joins merge a row's records and share right-hand rows between
-// neighbouring rows): it counts them, reserves room once, and writes them, the
-// slots of a warp's 32 rows dealt over its lanes both times.
-constexpr int OL_ROWS = 256;
-__global__ void __launch_bounds__(OL_ROWS) k_oldleft(Dev d, uint32_t q, uint4 *out, uint64_t cap,
-                                                     const uint32_t *__restrict__ row_job,
-                                                     const uint32_t *__restrict__ job_cnt)
+// A block takes 8 << lg consecutive rows of one rule and writes their records
+// together, in row order (the joins merge a row's records and share right-hand
+// rows between neighbouring rows): it counts them, reserves room once, and writes
+// them, the slots of a warp's 1 << lg rows dealt over its lanes both times. All
+// rules go in one launch; small graphs take fewer rows a warp, so that a
+// 600-vertex graph (6 rules, 43 us a round in a launch a rule) fills more than
+// three blocks.
+constexpr int OL_WARPS = 8;
+__global__ void __launch_bounds__(OL_WARPS * 32) k_oldleft(Dev d, uint32_t lg, uint4 *out, uint64_t cap,
+                                                           const uint32_t *__restrict__ row_job,
+                                                           const uint32_t *__restrict__ job_cnt)
 {
     if (d.ctr[C_HALT]) return;
-    __shared__ uint32_t warp_n[OL_ROWS / 32];
+    __shared__ uint32_t warp_n[OL_WARPS];
     __shared__ unsigned long long base_s;
-    __shared__ uint8_t own_s[OL_ROWS / 32][32];
-    const uint32_t B = d.rt.ol_B[q], C = d.rt.ol_C[q], lane = lane_id(), wid = threadIdx.x >> 5;
-    const uint32_t *dv = d.dvm + (size_t)(C - 1) * d.vwords;
-    const uint32_t vkey = (OL_SLOT0 + q) << KEY_SHIFT;
+    __shared__ uint8_t own_s[OL_WARPS][32];
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, rows = OL_WARPS << lg;
+    const uint64_t groups = ((uint64_t)d.V + rows - 1) / rows;
     uint8_t *own = own_s[wid];
-    for (uint64_t b0 = blockIdx.x * (uint64_t)OL_ROWS; b0 < d.V; b0 += (uint64_t)gridDim.x * OL_ROWS) {
-        const uint64_t v = b0 + threadIdx.x;
-        const uint64_t de = v < d.V ? d.desc[(size_t)(B - 1) * d.V + v] : 0ull;
+    for (uint64_t u = blockIdx.x; u < groups * d.rt.nol; u += gridDim.x) {
+        const uint32_t q = (uint32_t)(u / groups), B = d.rt.ol_B[q], C = d.rt.ol_C[q];
+        const uint32_t *dv = d.dvm + (size_t)(C - 1) * d.vwords;
+        const uint32_t vkey = (OL_SLOT0 + q) << KEY_SHIFT;
+        const uint64_t v0 = u % groups * rows + ((uint64_t)wid << lg), v = v0 + lane;
+        const bool mine = lane < (1u << lg) && v < d.V;
+        const uint64_t de = mine ? d.desc[(size_t)(B - 1) * d.V + v] : 0ull;
         uint32_t cap_v = (uint32_t)(de >> 32);
-        if (v < d.V && prefix_table(d, B, cap_v)) cap_v = min(cap_v, d.cnt[(size_t)(B - 1) * d.V + v]);
+        if (mine && prefix_table(d, B, cap_v)) cap_v = min(cap_v, d.cnt[(size_t)(B - 1) * d.V + v]);
         // batched jobs: a job without delta records this round adds no virtual records
         if (row_job && cap_v) {
             const uint32_t job = row_job[v];
@@ -641,7 +647,7 @@ __global__ void __launch_bounds__(OL_ROWS) k_oldleft(Dev d, uint32_t q, uint4 *o
                     const uint64_t p = pos + n + __popc(em & ((1u << lane) - 1u));
                     if (p < cap) {
                         out[2 * p] = make_uint4(m.w[0], m.w[1], m.w[2], m.w[3]);
-                        out[2 * p + 1] = make_uint4(m.w[4], m.w[5], vkey | base, (uint32_t)(b0 + wid * 32 + o));
+                        out[2 * p + 1] = make_uint4(m.w[4], m.w[5], vkey | base, (uint32_t)(v0 + o));
                     }
                 }
                 n += __popc(em);
@@ -651,7 +657,7 @@ __global__ void __launch_bounds__(OL_ROWS) k_oldleft(Dev d, uint32_t q, uint4 *o
             __syncthreads();
             if (threadIdx.x == 0) {
                 uint32_t sum = 0;
-                for (int w = 0; w < OL_ROWS / 32; w++) {
+                for (int w = 0; w < OL_WARPS; w++) {
                     const uint32_t c = warp_n[w];
                     warp_n[w] = sum;
                     sum += c;
@@ -664,6 +670,17 @@ __global__ void __launch_bounds__(OL_ROWS) k_oldleft(Dev d, uint32_t q, uint4 *o
         }
         __syncthreads();
     }
+}
+
+// Virtual records of every old-left rule.
+static void launch_oldleft(int sms, cudaStream_t s, const Dev &d, uint4 *out, uint64_t cap, const uint32_t *row_job,
+                           const uint32_t *job_cnt)
+{
+    uint32_t lg = 5;
+    while (lg > 2 && (uint64_t)d.rt.nol * (d.V >> lg) < (uint64_t)sms * OL_WARPS * 4) lg--;
+    const uint64_t groups = ((uint64_t)d.V + (OL_WARPS << lg) - 1) / (OL_WARPS << lg) * (uint64_t)d.rt.nol;
+    const int grid = (int)std::max<uint64_t>(std::min<uint64_t>(groups, (uint64_t)sms * 8), 1);
+    k_oldleft<<<grid, OL_WARPS * 32, 0, s>>>(d, lg, out, cap, row_job, job_cnt);
 }
 
 // Per-warp shared memory of the join, for a dense window of W elements per
@@ -1780,61 +1797,81 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
 // as they are. The choice is made here, on the device: the joins read their
 // counts from C_JN1 / C_JN2 / C_SPLIT_N.
 constexpr uint32_t SPLIT_MAX = 32768;
+// The same line for rounds that otherwise go through k_tile: it depends on how many old-left rules
+// the round's records are spread over. 3,000-vertex alias graph (2 rules), in the static scratch:
+// 6.1 ms with the line at 8,192 records, 8.2 ms at 32,768; 600-vertex points-to graph (6 rules):
+// 3.8 ms at 8,192 and 3.2 ms at 32,768.
+constexpr uint32_t TILE_MIN_RULE = 5461;
+__host__ __device__ inline uint64_t tile_min(int nol)
+{
+    const uint64_t n = (uint64_t)TILE_MIN_RULE * (uint64_t)nol;
+    return n < SPLIT_MAX ? n : SPLIT_MAX;
+}
 constexpr uint32_t SPLIT_BITS = 8;
 constexpr uint32_t SPLIT_PARTS = (EIDS + SPLIT_BITS - 1) / SPLIT_BITS;
 
 // tile: the rounds that are not split go through k_tile (C_TS: its rows), not k_join.
-__global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out, int tile)
+// A thread cuts one bitmap word of a record (up to 4 parts), and a warp reserves its parts' room
+// at once, in record order: a thread a record took 14 us for the 192 bits of a dense one.
+__global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out, int tile,
+                        uint64_t split_max)
 {
     if (d.ctr[C_HALT]) return;
     const uint64_t nd = d.ctr[C_DIRTY_N], nv = d.ctr[C_VN];
-    const bool split = nd + nv < SPLIT_MAX;
+    const bool split = nd + nv < split_max;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         d.ctr[C_JN1] = split || tile ? 0 : nd;
         d.ctr[C_JN2] = split || tile ? 0 : nv;
         d.ctr[C_TS] = split || !tile ? 0 : tile_rows_lg(nd + nv);
     }
     if (!split) return;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nd + nv;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint4 *r = i < nd ? grecs + 2 * i : vrecs + 2 * (i - nd);
-        const uint4 a = r[0], b = r[1];
-        const uint32_t w[EW] = {a.x, a.y, a.z, a.w, b.x, b.y};
-        uint32_t p = 0;
-#pragma unroll
-        for (int x = 0; x < EW; x++) p += __popc(w[x]);
-        const uint32_t lab = b.z >> KEY_SHIFT;
-        if (p && lab <= (uint32_t)MAX_LABELS && d.rt.tpose[lab]) {
-            // a column's record is pushed whole (its bits cost nothing extra): never split
-            const uint64_t pos = atomicAdd(&d.ctr[C_SPLIT_N], 1ull);
-            out[2 * pos] = a;
-            out[2 * pos + 1] = b;
-            continue;
-        }
-        const uint32_t parts = (p + SPLIT_BITS - 1) / SPLIT_BITS;
-        if (!parts) continue;
-        uint64_t pos = atomicAdd(&d.ctr[C_SPLIT_N], (unsigned long long)parts);
-        uint32_t cur[EW] = {0, 0, 0, 0, 0, 0}, c = 0;
-#pragma unroll
-        for (int x = 0; x < EW; x++) {
-            uint32_t m = w[x];
-            while (m) {
-                const uint32_t bit = m & (0u - m);
-                m ^= bit;
-                cur[x] |= bit;
-                if (++c == SPLIT_BITS) {
-                    out[2 * pos] = make_uint4(cur[0], cur[1], cur[2], cur[3]);
-                    out[2 * pos + 1] = make_uint4(cur[4], cur[5], b.z, b.w);
-                    pos++;
-                    c = 0;
-#pragma unroll
-                    for (int y = 0; y < EW; y++) cur[y] = 0;
+    const uint64_t total = (nd + nv) * EW, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t lane = lane_id();
+    for (uint64_t u0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); u0 < total; u0 += stride) {
+        const uint64_t u = u0 + lane, i = u / EW;
+        const uint32_t x = (uint32_t)(u % EW);
+        uint32_t m = 0, parts = 0;
+        uint2 key = make_uint2(EMPTY, 0);
+        uint4 whole0 = make_uint4(0, 0, 0, 0), whole1 = whole0;
+        bool whole = false;
+        if (u < total) {
+            const uint32_t *r = reinterpret_cast<const uint32_t *>(i < nd ? grecs + 2 * i : vrecs + 2 * (i - nd));
+            key = *reinterpret_cast<const uint2 *>(r + 6);
+            const uint32_t lab = key.x >> KEY_SHIFT;
+            if (lab <= (uint32_t)MAX_LABELS && d.rt.tpose[lab]) {
+                // a column's record is pushed whole (its bits cost nothing extra): never split
+                if (x == 0) {
+                    ld32(r, whole0, whole1);
+                    whole = (whole0.x | whole0.y | whole0.z | whole0.w | whole1.x | whole1.y) != 0;
+                    parts = whole;
                 }
+            } else {
+                m = r[x];
+                parts = (__popc(m) + SPLIT_BITS - 1) / SPLIT_BITS;
             }
         }
-        if (c) {                      // the last, partial part
-            out[2 * pos] = make_uint4(cur[0], cur[1], cur[2], cur[3]);
-            out[2 * pos + 1] = make_uint4(cur[4], cur[5], b.z, b.w);
+        uint32_t incl = parts;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        unsigned long long pos = 0;
+        if (lane == 31 && incl) pos = atomicAdd(&d.ctr[C_SPLIT_N], (unsigned long long)incl);
+        pos = __shfl_sync(0xffffffffu, pos, 31) + incl - parts;
+        if (whole) st32(out + 2 * pos, whole0, whole1);
+        while (m) {
+            uint32_t part = m;                    // the lowest SPLIT_BITS bits of m
+            if (__popc(m) > (int)SPLIT_BITS) {
+                uint32_t rest = m;
+#pragma unroll
+                for (uint32_t k = 0; k < SPLIT_BITS; k++) rest &= rest - 1;
+                part = m ^ rest;
+            }
+            m ^= part;
+            st32(out + 2 * pos,
+                 make_uint4(x == 0 ? part : 0, x == 1 ? part : 0, x == 2 ? part : 0, x == 3 ? part : 0),
+                 make_uint4(x == 4 ? part : 0, x == 5 ? part : 0, key.x, key.y));
+            pos++;
         }
     }
 }
@@ -4291,11 +4328,8 @@ static int round_oldleft(grg_ctx *c, uint64_t *nv_out)
         for (int attempt = 0; attempt < 2; attempt++) {
             Dev d = make_dev(c);
             GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_VN, 0, 8, s));
-            for (int q = 0; q < c->rt.nol; q++) {
-                k_oldleft<<<grid_for(c, c->V, 256), 256, 0, s>>>(d, (uint32_t)q, c->vbuf, c->vbuf_cap, c->row_job,
-                                                                 c->job_cnt);
-                c->launches++;
-            }
+            launch_oldleft(c->sms, s, d, c->vbuf, c->vbuf_cap, c->row_job, c->job_cnt);
+            c->launches++;
             int st = read_ctr(c);
             if (st) return st;
             nv = c->h_ctr[C_VN];
@@ -4313,6 +4347,7 @@ static int round_oldleft(grg_ctx *c, uint64_t *nv_out)
 // pass are re-run until nothing fails.
 // Retry list size for a round of n records: retries come only from tables at
 // their load limit, a small share; a round with more is re-run whole.
+static uint64_t split_max(const grg_ctx *c) { return use_tiles(c) ? tile_min(c->rt.nol) : SPLIT_MAX; }
 static uint64_t retry_room(const grg_ctx *c, uint64_t n) { return std::max<uint64_t>(c->retry_min, n / 8); }
 
 // The first join pass of a round over its records: the parts of a small round
@@ -4432,7 +4467,7 @@ static int ensure_tiles(grg_ctx *c)
 static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, double &join_ms, uint64_t &joins)
 {
     cudaStream_t s = c->stream;
-    const bool split = nd + nv < SPLIT_MAX;
+    const bool split = nd + nv < split_max(c);
     int st = ensure_rbuf(c, retry_room(c, nd + nv));
     if (st) return st;
     if (split && (st = ensure_sbuf(c))) return st;
@@ -4442,7 +4477,7 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
     if (split) {
         // few records: their parts spread the join over more warps
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_SPLIT_N, 0, 8, s));
-        k_split<<<grid_for(c, nd + nv, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, 0);
+        k_split<<<grid_for(c, (nd + nv) * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, 0, split_max(c));
         c->launches++;
     }
     if (c->tune_pending && c->need_join && !split && nd >= TUNE_MIN_RECORDS) {
@@ -4620,11 +4655,9 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
         nk++;
     }
     if (c->rt.nol) {
-        for (int q = 0; q < c->rt.nol; q++)
-            k_oldleft<<<grid_for(c, c->V, 256), 256, 0, s>>>(d, (uint32_t)q, c->vbuf, c->vbuf_cap, c->row_job,
-                                                             c->job_cnt);
+        launch_oldleft(c->sms, s, d, c->vbuf, c->vbuf_cap, c->row_job, c->job_cnt);
         k_gate_oldleft<<<1, 32, 0, s>>>(ctr, c->vbuf_cap, h);
-        nk += c->rt.nol + 1;
+        nk += 2;
     }
     if (c->timing) {
         k_tmark<<<1, 32, 0, s>>>(ctr, C_JT0, C_JNS, 0);
@@ -4633,7 +4666,7 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
     const int jgrid = grid_for(c, ~0u, JOIN_WARPS, 16);
     cudaMemsetAsync(ctr + C_SPLIT_N, 0, 8, s);
     const bool tiles = use_tiles(c);
-    k_split<<<grid_for(c, SPLIT_MAX, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles);
+    k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles, split_max(c));
     nk++;
     {
         const uint64_t launches0 = c->launches;
@@ -4769,7 +4802,7 @@ static int run_rounds(grg_ctx *c, uint64_t max_rounds, grg_stats &S, double &joi
         } else if (halt == HALT_RETRY) {
             const uint64_t nd = c->h_ctr[C_DIRTY_N], nv = c->h_ctr[C_VN];
             if ((st = round_retries(c, c->h_ctr[C_RETRY_N], c->cand_cap ? c->h_ctr[C_AFAIL] : 0, S, join_ms, joins,
-                                    nd, nv, nd + nv < SPLIT_MAX)))
+                                    nd, nv, nd + nv < split_max(c))))
                 return st;
         } else if (halt == HALT_LIMIT) {
             // a launch that ran this long without a halt is not trusted: host-driven rounds from here
@@ -5639,8 +5672,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH
 // device with that device current (the host-side symbol is not a device address).
 static void *g_noalloc_addr[256];
 
-constexpr uint64_t NOALLOC_TILE_MIN = 512;   // records of a round that goes through k_tile
-
 static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace grg
@@ -5669,10 +5700,12 @@ struct DeviceGuard {
 };
 }  // namespace
 
-extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, const int *rules, int num_labels,
-                                   uint32_t filter, uint32_t num_vars, uint64_t num_edges, const uint32_t *d_src,
-                                   const uint32_t *d_dst, const uint8_t *d_label, uint64_t *d_label_counts,
-                                   uint64_t *d_set_hash, uint64_t *rounds_out)
+// presize (in: allowed; out: done): derived rows start with DERIVED_MIN_CAP slots, as in
+// grg_load_edges, when that takes no more than half of the array's slots.
+static int noalloc_closure(int device, void *stream, int num_rules, const int *rules, int num_labels, uint32_t filter,
+                           uint32_t num_vars, uint64_t num_edges, const uint32_t *d_src, const uint32_t *d_dst,
+                           const uint8_t *d_label, uint64_t *d_label_counts, uint64_t *d_set_hash, uint64_t *rounds_out,
+                           bool *presize)
 {
     if (device < 0 || device >= 256 || num_rules < 0 || num_rules > GRG_MAX_RULES || (num_rules && !rules) ||
         num_labels < 1 || num_labels > GRG_MAX_LABELS || filter > 1 || !d_label_counts ||
@@ -5779,6 +5812,14 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
         if (rules[3 * q + 1] == 0) k_eps_hist<<<grid(num_vars, 256, 8), 256, 0, s>>>(d, (uint32_t)rules[3 * q], 0, num_vars);
     MinCap mc;
     memset(&mc, 0, sizeof mc);
+    if (*presize) {
+        bool lhs[MAX_LABELS + 1] = {false};
+        uint64_t nder = 0;
+        for (int q = 0; q < num_rules; q++) lhs[rules[3 * q]] = true;
+        for (int l = 1; l <= num_labels; l++) nder += lhs[l];
+        *presize = nder * num_vars * DERIVED_MIN_CAP <= pool / 2;
+        for (int l = 1; l <= num_labels; l++) mc.cap[l] = *presize && lhs[l] ? DERIVED_MIN_CAP : 0;
+    }
     k_load_alloc<<<alloc_grid(sms, (uint32_t)num_labels, num_vars), ALLOC_ROWS, 0, s>>>(d, 0, num_vars, (uint32_t)num_labels, mc, nullptr);
     if ((st = na_read(h, d.ctr, s))) return st;
     if (h[C_BADIN] & ERR_IN_LABEL) return GRG_E_LABEL;
@@ -5827,8 +5868,7 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
         uint64_t nv = 0;
         if (rt.nol) {
             NA_CUDA(cudaMemsetAsync(d.ctr + C_VN, 0, 8, s));
-            for (int q = 0; q < rt.nol; q++)
-                k_oldleft<<<grid(num_vars, 256, 8), 256, 0, s>>>(d, (uint32_t)q, vbuf, pool, nullptr, nullptr);
+            launch_oldleft(sms, s, d, vbuf, pool, nullptr, nullptr);
             if ((st = na_read(h, d.ctr, s))) return st;
             nv = h[C_VN];
             if (nd + nv > pool) return GRG_E_NOMEM;                // records (and their retries) outgrew the scratch
@@ -5839,23 +5879,22 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
         for (int pass = 0;; pass++) {
             const int g = grid((n + RB - 1) / RB, JOIN_WARPS, 16);
             // each join launch pulls 32-record batches from a queue that starts at 0
-            if (pass == 0 && rt.nol && nd + nv >= NOALLOC_TILE_MIN) {
+            if (pass == 0 && nd + nv < (rt.nol ? tile_min(rt.nol) : (uint64_t)SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
+                // few records: their parts (in rbuf[1], free in this pass)
+                NA_CUDA(cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
+                k_split<<<grid((nd + nv) * EW, 256, 8), 256, 0, s>>>(d, gbuf, vbuf, rbuf[1], 0, ~0ull);
+                NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
+                k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_SPLIT_N, rbuf[0]);
+            } else if (pass == 0 && rt.nol) {
                 // gslot and rbuf[1] are free in this pass: the tile list and the records left to k_join
                 launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0], tile_rows_lg(nd + nv));
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
-                k_join<WIN, WIN_LO><<<grid((nd + nv + RB - 1) / RB, JOIN_WARPS, 16), JOIN_WARPS * 32, 0, s>>>(
-                    d, rbuf[1], 0, C_LN, rbuf[0]);
-            } else if (pass == 0) {
-                NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
-                k_join<WIN, WIN_LO><<<g, JOIN_WARPS * 32, 0, s>>>(d, gbuf, nd, -1, rbuf[0]);
-                if (nv) {
-                    NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
-                    k_join<WIN, WIN_LO><<<grid((nv + RB - 1) / RB, JOIN_WARPS, 16), JOIN_WARPS * 32, 0, s>>>(d, vbuf, nv,
-                                                                                                        -1, rbuf[0]);
-                }
+                k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_LN, rbuf[0]);
             } else {
+                // the round's records (pass 0, no virtual ones), or those that failed in the last pass
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
-                k_join<WIN, WIN_LO><<<g, JOIN_WARPS * 32, 0, s>>>(d, rbuf[rb], n, -1, rbuf[rb ^ 1]);
+                k_join<WIN2, WIN2_LO><<<std::min(g, sms * GRG_JOIN_MINB_WIDE), JOIN_WARPS * 32, 0, s>>>(
+                    d, pass == 0 ? gbuf : rbuf[rb], n, -1, pass == 0 ? rbuf[0] : rbuf[rb ^ 1]);
             }
             NA_CUDA(cudaGetLastError());
             if ((st = na_read(h, d.ctr, s))) return st;
@@ -5883,4 +5922,22 @@ extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, cons
     NA_CUDA(cudaStreamSynchronize(s));
     if (rounds_out) *rounds_out = rounds;
     return GRG_OK;
+}
+
+extern "C" int grg_closure_noalloc(int device, void *stream, int num_rules, const int *rules, int num_labels,
+                                   uint32_t filter, uint32_t num_vars, uint64_t num_edges, const uint32_t *d_src,
+                                   const uint32_t *d_dst, const uint8_t *d_label, uint64_t *d_label_counts,
+                                   uint64_t *d_set_hash, uint64_t *rounds_out)
+{
+    // with presized rows few tables grow; a graph whose closure then outgrows the array is closed
+    // again with rows as small as its edges need (nothing has been written to the outputs)
+    bool presize = true;
+    int st = noalloc_closure(device, stream, num_rules, rules, num_labels, filter, num_vars, num_edges, d_src, d_dst, d_label,
+                             d_label_counts, d_set_hash, rounds_out, &presize);
+    if (st == GRG_E_NOMEM && presize) {
+        presize = false;
+        st = noalloc_closure(device, stream, num_rules, rules, num_labels, filter, num_vars, num_edges, d_src, d_dst, d_label,
+                             d_label_counts, d_set_hash, rounds_out, &presize);
+    }
+    return st;
 }
