@@ -2953,6 +2953,7 @@ __global__ void k_export_elems(Dev d, uint32_t v0, uint32_t v1, uint32_t L, uint
     const uint32_t lane = lane_id();
     const uint64_t nv = v1 - v0, ntab = (uint64_t)L * nv;
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    uint32_t counted = 0;                        // without a buffer: one addition a warp, at the end
     for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < ntab; u += nwarps) {
         const uint32_t lab = (uint32_t)(u / nv) + 1, row = v0 + (uint32_t)(u % nv);
         const uint64_t de = d.desc[(size_t)(lab - 1) * d.V + row];
@@ -2963,15 +2964,19 @@ __global__ void k_export_elems(Dev d, uint32_t v0, uint32_t v1, uint32_t L, uint
             if (t < cap) {
                 const uint4 *e = reinterpret_cast<const uint4 *>(d.elems + (size_t)(off + t) * 8);
                 e1 = e[1];
-                if (e1.z != EMPTY) e0 = e[0];
+                if (out && e1.z != EMPTY) e0 = e[0];
             }
             const bool have = e1.z != EMPTY;
             const unsigned m = __ballot_sync(0xffffffffu, have);
             if (!m) continue;
+            if (!out) {
+                counted += __popc(m);
+                continue;
+            }
             unsigned long long p0 = 0;
             if (lane == 0) p0 = atomicAdd(&d.ctr[C_EXPORT], (unsigned long long)__popc(m));
             p0 = __shfl_sync(0xffffffffu, p0, 0);
-            if (have && out) {
+            if (have) {
                 const uint64_t p = p0 + __popc(m & ((1u << lane) - 1u));
                 if (p < cap_out) {
                     out[2 * p] = e0;
@@ -2981,6 +2986,7 @@ __global__ void k_export_elems(Dev d, uint32_t v0, uint32_t v1, uint32_t L, uint
             }
         }
     }
+    if (counted && lane == 0) atomicAdd(&d.ctr[C_EXPORT], (unsigned long long)counted);
 }
 
 // Partitions that rows [v0, v1) reach through labels in label_mask:
@@ -5200,8 +5206,8 @@ static int export_csr5_split(grg_ctx *c, uint32_t a, uint32_t b, uint64_t total,
     if (csr5_footprint(total, n) <= budget || b - a <= 1) return export_csr5_piece(c, a, b, total, edges, degree);
     const uint32_t mid = a + (b - a) / 2;
     std::vector<uint64_t> counts(c->L + 1, 0);
-    uint64_t h = 0, t1 = 0;
-    if ((st = grg_range_counts(c, a, mid, counts.data(), &h))) return st;
+    uint64_t t1 = 0;
+    if ((st = grg_range_counts(c, a, mid, counts.data(), nullptr))) return st;
     for (int l = 0; l < c->L; l++) t1 += counts[l];
     if ((st = export_csr5_split(c, a, mid, t1, budget, edges, degree))) return st;
     return export_csr5_split(c, mid, b, total - t1, budget, edges + t1 * 5, degree + (mid - a));
@@ -5217,8 +5223,8 @@ int grg_export_csr5(grg_ctx *c, uint32_t v_begin, uint32_t v_end, uint64_t cap, 
     if (int rs = rows_by_source(c)) return rs;
     // the stream's length is the range's popcount
     std::vector<uint64_t> counts(c->L + 1, 0);
-    uint64_t h = 0, total = 0;
-    int st = grg_range_counts(c, v_begin, v_end, counts.data(), &h);
+    uint64_t total = 0;
+    int st = grg_range_counts(c, v_begin, v_end, counts.data(), nullptr);
     if (st) return st;
     for (int l = 0; l < c->L; l++) total += counts[l];
     *num_edges = total;

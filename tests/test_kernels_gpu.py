@@ -1,9 +1,12 @@
 """Kernels at the sizes where they can go wrong -- edges of tiles and groups, remainders, the
 smallest and largest of a range -- against the CPU oracle. Sets of edges: every comparison is exact."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import grg_gen as G
+from test_csr5 import pack_csr5
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +86,35 @@ def test_row_joins(grg_mod, oracle_mod, kind, nv, block, ne, f):
         st = ctx.closure(f)
         assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
         ctx.close()
+
+
+@pytest.mark.parametrize("shift", [0, 1, 3])
+@pytest.mark.parametrize("ne,fill", [(1, 0), (15, 0), (17, 0), (64, 1), (4_095, 0), (4_096, 1), (4_097, 0), (20_001, 1)])
+def test_stream_edges_of_tiles(grg_mod, ne, fill, shift):
+    """Streams of about a tile of 4,096 edges, of one full element (fill) and sparse ones, read from the
+    device at an odd address too and written back as they were."""
+    import torch
+
+    rng = np.random.default_rng(ne + fill)
+    V = 5_000
+    src = rng.integers(0, V, ne) if not fill else rng.integers(0, 1 + ne // 700, ne) * 31
+    dst = rng.integers(0, V if not fill else 400, ne)
+    if fill:                                             # one element with all of its 192 ids
+        src, dst = np.append(src, np.full(192, V - 1)), np.append(dst, np.arange(384, 576))
+    lab = rng.integers(1, 3, len(src))
+    e = np.unique(np.stack([src, lab, dst], 1), axis=0)
+    want, deg = pack_csr5(e[:, 0], e[:, 2], e[:, 1], 0, V)
+    buf = torch.zeros(len(want) + shift, dtype=torch.uint8, device="cuda")
+    buf[shift:] = torch.from_numpy(want).cuda()
+    ddeg = torch.from_numpy(deg.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    ctx = grg_mod.Context(0)
+    ctx.transfer_rules(np.array([[1, 2, 1]], np.int32), 2)
+    ctx._check(ctx._L.grg_load_csr5(ctx._h, V, 0, V, ctypes.c_void_p(ddeg.data_ptr()), len(e),
+                                    ctypes.c_void_p(buf.data_ptr() + shift), 1), "load_csr5")
+    assert [int(x) for x in ctx.label_counts()] == [int((e[:, 1] == k).sum()) for k in (1, 2)]
+    for lo, hi in ((0, V), (0, V - 1)):
+        got, gdeg = ctx.export_csr5(lo, hi)
+        w, d = pack_csr5(e[:, 0], e[:, 2], e[:, 1], lo, hi)
+        assert np.array_equal(got, w) and np.array_equal(gdeg, d)
+    ctx.close()
