@@ -1259,8 +1259,8 @@ __global__ void __launch_bounds__(PUSH_WARPS * 32, 4) k_push_flat(Dev d, const u
 //  - a record whose panel's union adds nothing to A[i] is done at once: late rounds (0.9M (i, k)
 //    pairs a block and round in the old-left joins, against a few thousand new edges) cost a
 //    compare a record instead of a pass over C's rows.
-// 1M-vertex alias closure: right-hand elements read 2.3e10 -> 5.4e8, closure 189 -> 82.5 ms;
-// 37k vertices 13.4 -> 7.5 ms. A block holds one tile a SM (214 KB), bound by the lookups' shared
+// 1M-vertex alias closure: right-hand elements read 2.3e10 -> 5.4e8, closure 189 -> 70.9 ms;
+// 37k vertices 13.4 -> 6.0 ms. A block holds one tile a SM (214 KB), bound by the lookups' shared
 // memory reads (21 of 16 bytes a lane and record in the mean) and by the waits between its phases.
 // Only accumulator words that changed are inserted. Right-hand elements outside the window of
 // TILE_W elements are joined in further windows (up to TILE_WINDOWS, each from the lowest base
@@ -1276,11 +1276,13 @@ constexpr int TILE_G = EIDS / 4;               // groups of 4 intermediates
 constexpr int TILE_RECS = 2048;                // records a tile holds at once (more are taken in turns)
 constexpr int TILE_KB = 32;                    // distinct blocks of intermediates at once
 constexpr int TILE_WINDOWS = 8;
-#ifndef GRG_TILE_BITS
-#define GRG_TILE_BITS 128
-#endif
-constexpr uint32_t TILE_MIN_BITS = GRG_TILE_BITS;  // (record, k) pairs that pay for reading a panel
-constexpr uint32_t TILE_MIN_RECS = 4;
+// Pairs (record, k) of a tile that pay for reading a panel; records of blocks with fewer go to k_join,
+// whose warps share them out over the chip. A panel holds an SM for some 7,000 clocks whatever it joins,
+// k_join takes a pair at a time: 4 pairs a row of the tile. Closures (ms) with 128 pairs at every size,
+// 1,024 at 256 rows, and 4,096: 1M-vertex alias 82.6, 70.8, 69.3; 300k 28.3, 25.0, 25.2; 37k vertices
+// 6.8, 6.0, 8.9; tiles of 64 rows and fewer (3,000 vertices) 5.5 with 128, 6.3 with 512.
+__device__ __forceinline__ uint32_t tile_min_bits(uint32_t sh) { return 4u << sh; }
+constexpr uint32_t TILE_MIN_RECS = 2;
 
 // Rows of a tile for a round of n records (some 6 a row): as many as leave every SM two tiles or more.
 __host__ __device__ inline uint32_t tile_rows_lg(uint64_t n)
@@ -1463,7 +1465,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
             __syncthreads();
             // ---- order by block; blocks with few pairs are left to k_join
             if (wid == 0) {
-                const bool heavy = w.kb[lane] != EMPTY && w.kbits[lane] >= TILE_MIN_BITS && w.kcnt[lane] >= TILE_MIN_RECS;
+                const bool heavy = w.kb[lane] != EMPTY && w.kbits[lane] >= tile_min_bits(sh) && w.kcnt[lane] >= TILE_MIN_RECS;
                 const uint32_t c = heavy ? w.kcnt[lane] : 0;
                 uint32_t incl = c;
                 for (int o = 1; o < 32; o <<= 1) {
@@ -1809,22 +1811,32 @@ __host__ __device__ inline uint64_t tile_min(int nol)
 }
 constexpr uint32_t SPLIT_BITS = 8;
 constexpr uint32_t SPLIT_PARTS = (EIDS + SPLIT_BITS - 1) / SPLIT_BITS;
+// Records that tiles leave to k_join are cut too: a warp that takes 32 of them whole is done long after
+// the others (0.5 to 1.1 ms a round, whatever their number). Up to SPLIT_MAX of them go in parts of
+// SPLIT_BITS, more by bitmap word, up to as many as the buffer holds 6 parts of. 37k-vertex alias
+// closure 6.8 -> 6.0 ms.
+constexpr int SPLIT_LEFT = 2;
+constexpr uint64_t SPLIT_LEFT_MAX = (uint64_t)SPLIT_MAX * SPLIT_PARTS / EW;
 
-// tile: the rounds that are not split go through k_tile (C_TS: its rows), not k_join.
+// tile: 1: the rounds that are not split go through k_tile (C_TS: its rows), not k_join; SPLIT_LEFT: the
+// records are those that k_tile left (C_LN of grecs), and those not split are joined as they are (C_JN1).
 // A thread cuts one bitmap word of a record (up to 4 parts), and a warp reserves its parts' room
 // at once, in record order: a thread a record took 14 us for the 192 bits of a dense one.
 __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out, int tile,
                         uint64_t split_max)
 {
     if (d.ctr[C_HALT]) return;
-    const uint64_t nd = d.ctr[C_DIRTY_N], nv = d.ctr[C_VN];
+    const bool left = tile == SPLIT_LEFT;
+    const uint64_t nd = d.ctr[left ? C_LN : C_DIRTY_N], nv = left ? 0 : d.ctr[C_VN];
     const bool split = nd + nv < split_max;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        d.ctr[C_JN1] = split || tile ? 0 : nd;
+        d.ctr[C_JN1] = split || tile == 1 ? 0 : nd;
         d.ctr[C_JN2] = split || tile ? 0 : nv;
-        d.ctr[C_TS] = split || !tile ? 0 : tile_rows_lg(nd + nv);
+        if (!left) d.ctr[C_TS] = split || !tile ? 0 : tile_rows_lg(nd + nv);
     }
     if (!split) return;
+    // bits of a part: 8, or a word's when more records are left than the buffer holds 24 parts of
+    const uint32_t part_bits = left && nd >= SPLIT_MAX ? 32u : SPLIT_BITS;
     const uint64_t total = (nd + nv) * EW, stride = (uint64_t)gridDim.x * blockDim.x;
     const uint32_t lane = lane_id();
     for (uint64_t u0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); u0 < total; u0 += stride) {
@@ -1847,7 +1859,7 @@ __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__r
                 }
             } else {
                 m = r[x];
-                parts = (__popc(m) + SPLIT_BITS - 1) / SPLIT_BITS;
+                parts = (__popc(m) + part_bits - 1) / part_bits;
             }
         }
         uint32_t incl = parts;
@@ -1861,7 +1873,7 @@ __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__r
         if (whole) st32(out + 2 * pos, whole0, whole1);
         while (m) {
             uint32_t part = m;                    // the lowest SPLIT_BITS bits of m
-            if (__popc(m) > (int)SPLIT_BITS) {
+            if ((uint32_t)__popc(m) > part_bits) {
                 uint32_t rest = m;
 #pragma unroll
                 for (uint32_t k = 0; k < SPLIT_BITS; k++) rest &= rest - 1;
@@ -4368,9 +4380,12 @@ static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv,
     }
     if (use_tiles(c)) {
         launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], tile_rows_lg(nd + nv));
-        launch_join(c, grid_for(c, (nd + nv + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_LN, c->rbuf[0]);
-        c->launches += 3;
-        joins += 2;
+        cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s);
+        k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX);
+        launch_join(c, grid_for(c, (nd + nv + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
+        launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB, JOIN_WARPS, 16), s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0]);
+        c->launches += 5;
+        joins += 3;
         return;
     }
     launch_pass(c, grid_for(c, (nd + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
@@ -4476,7 +4491,7 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
     const bool split = nd + nv < split_max(c);
     int st = ensure_rbuf(c, retry_room(c, nd + nv));
     if (st) return st;
-    if (split && (st = ensure_sbuf(c))) return st;
+    if ((split || use_tiles(c)) && (st = ensure_sbuf(c))) return st;
     if ((st = ensure_tiles(c))) return st;
     Dev d = make_dev(c);
     if (c->timing) GRG_CUDA(c, cudaEventRecord(c->ev_c, s));
@@ -4679,8 +4694,9 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
         uint64_t unused = 0;
         if (tiles) {
             launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], 0);
-            launch_join(c, jgrid, s, d, c->lbuf, 0, C_LN, c->rbuf[0]);
-            nk += 3;
+            k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX);
+            launch_join(c, jgrid, s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
+            nk += 4;
         } else {
             launch_pass(c, jgrid, s, d, c->gbuf, 0, C_JN1, c->rbuf[0], unused);
         }

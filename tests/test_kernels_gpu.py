@@ -36,7 +36,7 @@ def test_counts_and_hash_by_row_groups(grg_mod, oracle_mod, nv):
 
 
 @pytest.mark.parametrize("nv,block,density", [(40, 40, 3), (700, 129, 4), (9_000, 1000, 4), (30_000, 383, 3),
-                                              (3_500, 0, 2), (60_000, 1100, 2)])
+                                              (3_500, 0, 2), (60_000, 1100, 2), (24_000, 1000, 4)])
 def test_tiled_joins(grg_mod, oracle_mod, nv, block, density):
     """Grammars with a derivable second symbol join tiles of neighbouring rows. Blocks of a few ids,
     of more ids than one window of 8 elements holds (unconfined rows and their further windows), and
