@@ -433,27 +433,12 @@ __global__ void k_mark_all(Dev d, uint64_t begin, uint64_t end)   // begin: mult
 
 // ---------------------------------------------------------------- rounds
 
-// Dirty records per chunk of 1024 slots (one warp per chunk of 32 bitmap words).
 // Dirty-bitmap words below the pool top. Launches recorded once and replayed
 // (round graphs, dyn != 0) read the top from the device counter, bounded by
 // nwords = the words the buffers were sized for; others get the host's figure.
 __device__ __forceinline__ uint64_t dyn_words(uint64_t nwords, const unsigned long long *ctr, int dyn)
 {
     return dyn ? min(nwords, (uint64_t)(ctr[C_POOL_TOP] + 31) / 32) : nwords;
-}
-
-__global__ void k_dcount(Dev d, uint64_t nwords, uint32_t *chunk_cnt, int dyn)
-{
-    if (d.ctr[C_HALT]) return;
-    nwords = dyn_words(nwords, d.ctr, dyn);
-    const uint64_t nchunks = (nwords + 31) / 32;
-    const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t c = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); c < nchunks; c += nwarps) {
-        const uint64_t wi = c * 32 + lane_id();
-        uint32_t n = wi < nwords ? __popc(d.dmap[wi]) : 0;
-        for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-        if (lane_id() == 0) chunk_cnt[c] = n;
-    }
 }
 
 // Position of the n-th (0-based) set bit of a 32-bit word (broadword select, no loop).
@@ -475,8 +460,8 @@ __device__ __forceinline__ uint32_t select32(uint32_t w, uint32_t n)
 // Gather, pass 1: the dirty slots of the round, in slot order (a table's
 // records stay contiguous), as a dense array of slot ids; the dirty bits are
 // cleared. Lanes walk their own bitmap word: stores only, nothing to wait for.
-__global__ void k_gather_slots(Dev d, uint64_t nwords, const uint32_t *__restrict__ chunk_off, uint32_t *slots,
-                               int dyn)
+__global__ void k_gather_slots(Dev d, uint64_t nwords, const uint32_t *__restrict__ chunk_off,
+                               const uint32_t *__restrict__ block_off, uint32_t *slots, int dyn)
 {
     if (d.ctr[C_HALT]) return;
     nwords = dyn_words(nwords, d.ctr, dyn);
@@ -486,7 +471,7 @@ __global__ void k_gather_slots(Dev d, uint64_t nwords, const uint32_t *__restric
     for (uint64_t c = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); c < nchunks; c += nwarps) {
         const uint64_t wi = c * 32 + lane;
         uint32_t m = wi < nwords ? d.dmap[wi] : 0;
-        const uint64_t base_pos = chunk_off[c];
+        const uint64_t base_pos = chunk_off[c] + block_off[c >> 10];
         const uint32_t cnt = __popc(m);
         uint32_t incl = cnt;
         for (int o = 1; o < 32; o <<= 1) {
@@ -2537,23 +2522,10 @@ __global__ void k_csr_count(Dev d, uint32_t slot, uint32_t *deg, uint2 *row)
     }
 }
 
-// Block-wise exclusive scan of n values (1024 per block); block totals to sums.
-// dyn != null: a scan of the gather's chunk counts whose length follows the
-// pool top in the device counters (round graphs), at most n; blocks past it return.
-__device__ __forceinline__ uint64_t dyn_chunks(uint64_t n, const unsigned long long *dyn)
+// Exclusive scan of a block's 1,024 values v; the total goes to *sum.
+__device__ __forceinline__ uint32_t scan_block(uint32_t v, uint32_t *sum)
 {
-    return dyn ? min(n, (uint64_t)(dyn[C_POOL_TOP] + 1023) / 1024) : n;
-}
-
-__global__ void k_scan_blocks(const uint32_t *in, uint32_t *out, uint32_t *sums, uint64_t n,
-                              const unsigned long long *dyn)
-{
-    if (dyn && dyn[C_HALT]) return;
-    n = dyn_chunks(n, dyn);
-    if (blockIdx.x * 1024ull >= n && n) return;
     __shared__ uint32_t wsum[32];
-    const uint64_t i = blockIdx.x * 1024ull + threadIdx.x;
-    const uint32_t v = i < n ? in[i] : 0;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t incl = v;
     for (int o = 1; o < 32; o <<= 1) {
@@ -2569,54 +2541,75 @@ __global__ void k_scan_blocks(const uint32_t *in, uint32_t *out, uint32_t *sums,
             if (lane >= (uint32_t)o) si += y;
         }
         wsum[lane] = si - s;
-        if (lane == 31) sums[blockIdx.x] = si;
+        if (lane == 31) *sum = si;
     }
     __syncthreads();
-    if (i < n) out[i] = incl - v + wsum[wid];
+    return incl - v + wsum[wid];
+}
+
+// Block-wise exclusive scan of n values (1024 per block); block totals to sums.
+__global__ void k_scan_blocks(const uint32_t *in, uint32_t *out, uint32_t *sums, uint64_t n)
+{
+    const uint64_t i = blockIdx.x * 1024ull + threadIdx.x;
+    const uint32_t excl = scan_block(i < n ? in[i] : 0, &sums[blockIdx.x]);
+    if (i < n) out[i] = excl;
+}
+
+// Chunks of 1,024 slots below the pool top: the host's figure, or (dyn, round graphs) the device
+// counter's, at most n.
+__device__ __forceinline__ uint64_t dyn_chunks(uint64_t n, const unsigned long long *ctr, int dyn)
+{
+    return dyn ? min(n, (uint64_t)(ctr[C_POOL_TOP] + 1023) / 1024) : n;
+}
+
+// Dirty records per chunk of 1,024 slots (a thread per chunk: its 32 bitmap words are one line),
+// scanned over the 1,024 chunks of a block; block totals to sums. Counting, scanning blocks, scanning
+// the totals, adding them back and the loop's gate were five launches a round, most of a small round's
+// gather (3-4 us each); they are two, and k_gather_slots adds the totals.
+__global__ void __launch_bounds__(1024) k_dscan(Dev d, uint64_t nwords, uint32_t *off, uint32_t *sums, int dyn)
+{
+    if (d.ctr[C_HALT]) return;
+    const uint64_t n = dyn_chunks((nwords + 31) / 32, d.ctr, dyn);
+    if (blockIdx.x * 1024ull >= n && n) return;
+    nwords = dyn_words(nwords, d.ctr, dyn);
+    const uint64_t c = blockIdx.x * 1024ull + threadIdx.x;
+    uint32_t v = 0;
+    if (c * 32 + 32 <= nwords) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(d.dmap + c * 32);
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            const uint4 m = p[x];
+            v += __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+        }
+    } else {
+        for (uint64_t w = c * 32; w < nwords; w++) v += __popc(d.dmap[w]);
+    }
+    const uint32_t excl = scan_block(v, &sums[blockIdx.x]);
+    if (c < n) off[c] = excl;
 }
 
 // Exclusive scan of the block totals (one block, sequential over chunks of 1024); total at sums[nb].
-__global__ void k_scan_sums(uint32_t *sums, uint64_t nb, const unsigned long long *dyn)
+__device__ __forceinline__ void scan_sums(uint32_t *sums, uint64_t nb)
 {
-    if (dyn && dyn[C_HALT]) return;
-    if (dyn) nb = min(nb, (dyn_chunks(~0ull, dyn) + 1023) / 1024);
-    __shared__ uint32_t wsum[32];
-    __shared__ uint32_t carry;
+    __shared__ uint32_t carry, total;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (uint64_t c0 = 0; c0 < nb; c0 += 1024) {
         const uint64_t i = c0 + threadIdx.x;
-        const uint32_t v = i < nb ? sums[i] : 0;
-        uint32_t incl = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (uint32_t)o) incl += y;
-        }
-        if (lane == 31) wsum[wid] = incl;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t s = wsum[lane], si = s;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, si, o);
-                if (lane >= (uint32_t)o) si += y;
-            }
-            wsum[lane] = si - s;
-        }
-        __syncthreads();
+        const uint32_t excl = scan_block(i < nb ? sums[i] : 0, &total);
         const uint32_t base = carry;
-        if (i < nb) sums[i] = base + incl - v + wsum[wid];
+        if (i < nb) sums[i] = base + excl;
         __syncthreads();
-        if (threadIdx.x == 1023) carry = base + wsum[wid] + incl;
+        if (threadIdx.x == 0) carry = base + total;
         __syncthreads();
     }
     if (threadIdx.x == 0) sums[nb] = carry;
 }
 
-__global__ void k_scan_add(uint32_t *out, const uint32_t *sums, uint64_t n, const unsigned long long *dyn)
+__global__ void k_scan_sums(uint32_t *sums, uint64_t nb) { scan_sums(sums, nb); }
+
+__global__ void k_scan_add(uint32_t *out, const uint32_t *sums, uint64_t n)
 {
-    if (dyn && dyn[C_HALT]) return;
-    n = dyn_chunks(n, dyn);
     const uint64_t i = blockIdx.x * 1024ull + threadIdx.x;
     if (i < n) out[i] += sums[blockIdx.x];
 }
@@ -3074,7 +3067,7 @@ struct grg_ctx {
     uint32_t *elems = nullptr;
     uint32_t *dbits = nullptr;                 // delta bitmaps (32 B per slot)
     uint32_t *dmap = nullptr;                  // dirty bitmap (1 bit per slot)
-    uint32_t *chunk = nullptr;                 // dirty counts / offsets per 1024 slots (+ scan sums)
+    uint32_t *chunk = nullptr;                 // offsets of dirty slots per 1024 slots (+ scan sums)
     uint64_t chunk_cap = 0;
     uint64_t *desc = nullptr;
     uint32_t *cnt = nullptr, *want = nullptr, *grow = nullptr;
@@ -3344,10 +3337,10 @@ int alloc_pool(grg_ctx *c, uint64_t elems)
     return GRG_OK;
 }
 
-// Chunk counters of the dirty-bitmap gather: one per 1024 slots, plus scan sums.
+// Chunk offsets of the dirty-bitmap gather: one per 1024 slots, plus scan sums.
 int ensure_chunks(grg_ctx *c, uint64_t nchunks)
 {
-    const uint64_t need = 2 * (nchunks + 1) + (nchunks + 1023) / 1024 + 2;
+    const uint64_t need = nchunks + 1 + (nchunks + 1023) / 1024 + 2;
     if (need <= c->chunk_cap) return GRG_OK;
     cudaFree(c->chunk);
     c->chunk = nullptr;
@@ -3945,15 +3938,6 @@ __global__ void k_tmark(unsigned long long *ctr, int t0_slot, int acc_slot, int 
 // not fit after growing its tables. The pieces are separate so a round the
 // device-driven loop hands back can be finished where it stopped.
 
-// Window of this closure's joins. Measured on dataflow, alias, points-to and
-// small alias jobs, the wide window was fastest or within 1.5% on every one, so
-// it is the default; the narrow window stays selectable. Wide is 12 elements
-// (5 below the run's base). A warp has 8 window slots, one per run of a row's
-// records, and joins a batch of more runs in passes; a block takes 22 KB of
-// shared memory, and at 64 registers a thread (some bytes spilled) 8 blocks fit
-// an SM. Earlier layouts, measured on one box (2M-vertex dataflow / 1M alias
-// closure): 16 slots with runs past the 16th in the hash, 10-element windows, 7
-// blocks 54.4 / 317 ms; 32 slots (one per record) at 5 blocks 66.3 / 334 ms.
 // Joins that k_rows can run: no old-left joins (so no derivable right-hand label), no pushes, and a
 // CSR copy of every right-hand label (a batch has none, nor a label with a row of 2^24 ids). A fixed
 // window or item form is k_join's.
@@ -3969,6 +3953,15 @@ static bool rows_possible(const grg_ctx *c)
     return any;
 }
 
+// Window of this closure's joins. Measured on dataflow, alias, points-to and
+// small alias jobs, the wide window was fastest or within 1.5% on every one, so
+// it is the default; the narrow window stays selectable. Wide is 12 elements
+// (5 below the run's base). A warp has 8 window slots, one per run of a row's
+// records, and joins a batch of more runs in passes; a block takes 22 KB of
+// shared memory, and at 64 registers a thread (some bytes spilled) 8 blocks fit
+// an SM. Earlier layouts, measured on one box (2M-vertex dataflow / 1M alias
+// closure): 16 slots with runs past the 16th in the hash, 10-element windows, 7
+// blocks 54.4 / 317 ms; 32 slots (one per record) at 5 blocks 66.3 / 334 ms.
 static void choose_window(grg_ctx *c)
 {
     c->join_wide = c->join_window_mode >= 2 ? c->tuned_wide : c->join_window_mode != 0;
@@ -4005,8 +3998,8 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
 }
 
 // Rounds go through k_tile where a rule's second symbol is derivable (old-left joins): their right
-// rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 82.5 ms).
-// With static second symbols a right row is 1-2 elements and k_join's windows stay.
+// rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 70.9 ms).
+// With static second symbols a right row is 1-2 elements, too few to pay for a panel: k_rows or k_join.
 static bool use_tiles(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
 
 // The tiles of a round's gathered and virtual records (counts on the device): list, then join.
@@ -4296,15 +4289,13 @@ static int round_head(grg_ctx *c, uint32_t rs, grg_stats &S, uint64_t *nd_out)
     const uint64_t nchunks = (nwords + 31) / 32;
     int st = ensure_chunks(c, nchunks);
     if (st) return st;
-    uint32_t *ccnt = c->chunk, *coff = c->chunk + nchunks + 1, *csum = c->chunk + 2 * (nchunks + 1);
+    uint32_t *coff = c->chunk, *csum = c->chunk + nchunks + 1;
     const uint64_t nb = (nchunks + 1023) / 1024;
     Dev d = make_dev(c);
     if (c->timing) k_tmark<<<1, 32, 0, s>>>(c->ctr, C_GT0, C_GNS, 0);
-    k_dcount<<<grid_for(c, nchunks * 32, 256), 256, 0, s>>>(d, nwords, ccnt, 0);
-    k_scan_blocks<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(ccnt, coff, csum, nchunks, nullptr);
-    k_scan_sums<<<1, 1024, 0, s>>>(csum, nb, nullptr);
-    k_scan_add<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(coff, csum, nchunks, nullptr);
-    c->launches += 4;
+    k_dscan<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(d, nwords, coff, csum, 0);
+    k_scan_sums<<<1, 1024, 0, s>>>(csum, nb);
+    c->launches += 2;
     GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_DIRTY_N, 0, 8, s));
     GRG_CUDA(c, cudaMemcpyAsync(c->ctr + C_DIRTY_N, csum + nb, 4, cudaMemcpyDeviceToDevice, s));
     GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_RETRY_N, 0, 16, s));   // retry + grow counters
@@ -4330,7 +4321,7 @@ static int round_head(grg_ctx *c, uint32_t rs, grg_stats &S, uint64_t *nd_out)
             GRG_CUDA(c, cudaMemsetAsync(c->drc + t0, 0, (size_t)c->V * 4, s));
             GRG_CUDA(c, cudaMemsetAsync(c->dvm + (size_t)(l - 1) * vw, 0, vw * 4, s));
         }
-    k_gather_slots<<<grid_for(c, nchunks * 32, 256), 256, 0, s>>>(d, nwords, coff, c->gslot, 0);
+    k_gather_slots<<<grid_for(c, nchunks * 32, 256), 256, 0, s>>>(d, nwords, coff, csum, c->gslot, 0);
     k_gather_recs<<<grid_for(c, nd, 256), 256, 0, s>>>(d, c->gslot, c->gbuf, nd, -1, c->row_job, c->job_cnt, rs);
     c->launches += 2;
     if (c->timing) k_tmark<<<1, 32, 0, s>>>(c->ctr, C_GT0, C_GNS, 1);
@@ -4540,17 +4531,22 @@ enum : unsigned long long {
 };
 constexpr uint64_t GATE_MAX_ITERS = 1u << 20;   // iterations of one graph launch; past it the host takes over
 
-__global__ void k_gate_gather(unsigned long long *ctr, const uint32_t *csum, uint64_t max_chunks, uint64_t gbuf_cap,
-                              uint64_t max_iters, cudaGraphConditionalHandle h)
+// Also scans the gather's block totals and zeroes the counters that the round's kernels add to
+// (retries and grown tables, candidates and failed ones, virtual records, sub-records).
+__global__ void __launch_bounds__(1024) k_gate_gather(unsigned long long *ctr, uint32_t *csum, uint64_t max_chunks,
+                                                      uint64_t gbuf_cap, uint64_t max_iters,
+                                                      cudaGraphConditionalHandle h)
 {
+    const uint64_t nb = (dyn_chunks(max_chunks, ctr, 1) + 1023) / 1024;
+    if (!ctr[C_HALT]) scan_sums(csum, nb);       // the same for all threads: written below, past its barriers
     if (threadIdx.x != 0) return;
+    ctr[C_RETRY_N] = ctr[C_GROW_N] = ctr[C_CAND_N] = ctr[C_AFAIL] = ctr[C_VN] = ctr[C_SPLIT_N] = 0;
     const unsigned long long it = ++ctr[C_ITERS];
     if (ctr[C_HALT] || it > max_iters) {
         if (!ctr[C_HALT]) ctr[C_HALT] = HALT_LIMIT;
         cudaGraphSetConditional(h, 0);
         return;
     }
-    const uint64_t nb = (dyn_chunks(max_chunks, ctr) + 1023) / 1024;
     const uint64_t nd = csum[nb];
     ctr[C_DIRTY_N] = nd;
     const unsigned long long halt = nd == 0 ? HALT_FIXPOINT : nd > gbuf_cap ? HALT_CAPACITY : 0;
@@ -4643,7 +4639,7 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
     c->cb = 0;
     Dev d = make_dev(c);
     c->cb = saved_cb;
-    uint32_t *ccnt = c->chunk, *coff = c->chunk + nchunks + 1, *csum = c->chunk + 2 * (nchunks + 1);
+    uint32_t *coff = c->chunk, *csum = c->chunk + nchunks + 1;
     unsigned long long *ctr = c->ctr;
     int nk = 0;
     bool any_dindex = false;
@@ -4653,21 +4649,15 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
         k_dindex_clear<<<grid_for(c, c->gbuf_cap, 256), 256, 0, s>>>(d, c->gbuf, C_DIRTY_N);
         nk++;
     }
-    cudaMemsetAsync(ctr + C_RETRY_N, 0, 16, s);
-    cudaMemsetAsync(ctr + C_CAND_N, 0, 16, s);
     if (c->job_cnt) cudaMemsetAsync(c->job_cnt, 0, (size_t)c->max_jobs * 4, s);
     if (c->timing) {
         k_tmark<<<1, 32, 0, s>>>(ctr, C_GT0, C_GNS, 0);
         nk++;
     }
-    k_dcount<<<grid_for(c, nchunks * 32, 256), 256, 0, s>>>(d, nwords, ccnt, 1);
-    k_scan_blocks<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(ccnt, coff, csum, nchunks, ctr);
-    k_scan_sums<<<1, 1024, 0, s>>>(csum, nb, ctr);
-    k_scan_add<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(coff, csum, nchunks, ctr);
-    k_gate_gather<<<1, 32, 0, s>>>(ctr, csum, nchunks, c->gbuf_cap, GATE_MAX_ITERS, h);
-    nk += 5;
-    cudaMemsetAsync(ctr + C_VN, 0, 8, s);
-    k_gather_slots<<<grid_for(c, nchunks * 32, 256), 256, 0, s>>>(d, nwords, coff, c->gslot, 1);
+    k_dscan<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(d, nwords, coff, csum, 1);
+    k_gate_gather<<<1, 1024, 0, s>>>(ctr, csum, nchunks, c->gbuf_cap, GATE_MAX_ITERS, h);
+    nk += 2;
+    k_gather_slots<<<grid_for(c, nchunks * 32, 256), 256, 0, s>>>(d, nwords, coff, csum, c->gslot, 1);
     k_gather_recs<<<grid_for(c, c->gbuf_cap, 256), 256, 0, s>>>(d, c->gslot, c->gbuf, 0, C_DIRTY_N, c->row_job,
                                                                 c->job_cnt, rs);
     nk += 2;
@@ -4685,7 +4675,6 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
         nk++;
     }
     const int jgrid = grid_for(c, ~0u, JOIN_WARPS, 16);
-    cudaMemsetAsync(ctr + C_SPLIT_N, 0, 8, s);
     const bool tiles = use_tiles(c);
     k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles, split_max(c));
     nk++;
@@ -4896,9 +4885,9 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
         uint2 *row = cb.row;
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_ERR, 0, 8, s));
         k_csr_count<<<grid_for(c, c->V, 256), 256, 0, s>>>(d, (uint32_t)l, ptr, row);
-        k_scan_blocks<<<(unsigned)nb, 1024, 0, s>>>(ptr, ptr, sums, c->V, nullptr);
-        k_scan_sums<<<1, 1024, 0, s>>>(sums, nb, nullptr);
-        k_scan_add<<<(unsigned)nb, 1024, 0, s>>>(ptr, sums, c->V, nullptr);
+        k_scan_blocks<<<(unsigned)nb, 1024, 0, s>>>(ptr, ptr, sums, c->V);
+        k_scan_sums<<<1, 1024, 0, s>>>(sums, nb);
+        k_scan_add<<<(unsigned)nb, 1024, 0, s>>>(ptr, sums, c->V);
         st = read_ctr(c);
         if (st) return st;
         if (c->h_ctr[C_ERR]) continue;                 // a row too long for the packed CSR: keep elements
@@ -5765,7 +5754,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
     const size_t o_vbuf = off; off = align256(off + pool * 32);
     const size_t o_rbuf0 = off; off = align256(off + pool * 32);
     const size_t o_rbuf1 = off; off = align256(off + pool * 32);
-    const size_t o_chunk = off; off = align256(off + (2 * (pchunks + 1) + pnb + 2) * 4);
+    const size_t o_chunk = off; off = align256(off + (pchunks + 1 + pnb + 2) * 4);
     if (off > NOALLOC_SCRATCH_BYTES) return GRG_E_RANGE;
 
     RuleTable rt;
@@ -5866,11 +5855,9 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
         if ((st = na_read(h, d.ctr, s))) return st;
         const uint64_t nwords = (h[C_POOL_TOP] + 31) / 32, nchunks = (nwords + 31) / 32;
         const uint64_t nb = (nchunks + 1023) / 1024;
-        uint32_t *ccnt = chunk, *coff = chunk + nchunks + 1, *csum = chunk + 2 * (nchunks + 1);
-        k_dcount<<<grid(nchunks * 32, 256, 8), 256, 0, s>>>(d, nwords, ccnt, 0);
-        k_scan_blocks<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(ccnt, coff, csum, nchunks, nullptr);
-        k_scan_sums<<<1, 1024, 0, s>>>(csum, nb, nullptr);
-        k_scan_add<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(coff, csum, nchunks, nullptr);
+        uint32_t *coff = chunk, *csum = chunk + nchunks + 1;
+        k_dscan<<<(unsigned)std::max<uint64_t>(nb, 1), 1024, 0, s>>>(d, nwords, coff, csum, 0);
+        k_scan_sums<<<1, 1024, 0, s>>>(csum, nb);
         uint32_t nd32 = 0;
         NA_CUDA(cudaMemsetAsync(d.ctr + C_DIRTY_N, 0, 8, s));
         NA_CUDA(cudaMemcpyAsync(d.ctr + C_DIRTY_N, csum + nb, 4, cudaMemcpyDeviceToDevice, s));
@@ -5885,7 +5872,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
                 NA_CUDA(cudaMemsetAsync(d.drc + (size_t)(l - 1) * num_vars, 0, (size_t)num_vars * 4, s));
                 NA_CUDA(cudaMemsetAsync(d.dvm + (size_t)(l - 1) * vwords, 0, vwords * 4, s));
             }
-        k_gather_slots<<<grid(nchunks * 32, 256, 8), 256, 0, s>>>(d, nwords, coff, gslot, 0);
+        k_gather_slots<<<grid(nchunks * 32, 256, 8), 256, 0, s>>>(d, nwords, coff, csum, gslot, 0);
         k_gather_recs<<<grid(nd, 256, 8), 256, 0, s>>>(d, gslot, gbuf, nd, -1, nullptr, nullptr, 0);
         uint64_t nv = 0;
         if (rt.nol) {
