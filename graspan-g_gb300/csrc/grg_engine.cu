@@ -180,6 +180,7 @@ static void set_columns(RuleTable &rt, uint64_t tmask, int L)
 #endif
 constexpr int JOIN_WARPS = GRG_JOIN_WARPS;  // warps per join block
 constexpr int RB = 32;            // delta records per warp batch (one per lane)
+constexpr int RB_MIN = 8;         // and the fewest (see batch_records)
 constexpr int WIN = GRG_WIN;      // dense accumulator window: elements base-WIN_LO .. base+WIN-1-WIN_LO
 constexpr int WIN_LO = GRG_WIN_LO;
 #ifndef GRG_WIN2
@@ -1873,7 +1874,18 @@ __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__r
     }
 }
 
-// One warp per batch of RB delta records (label B, row i, base, bits); lane r
+// Records of a batch: 32, fewer while a warp would get less than 4 batches: the last batches of 32
+// dense records ran 1.3 to 2.5 ms after the rest. Closures (ms) with batches of 32 always, down to 16,
+// 8 and 4: 600-vertex points-to 3.3, 2.8, 2.7, 2.9; 37k-vertex alias 6.1, 5.6, 5.8, 5.9; 120k 8.7, 8.2,
+// 7.8, 8.1; 3,000 vertices in the static scratch 6.2, 5.7, 4.5, 4.5; 8 partitions of 200k 175, 158, 152, 152.
+__device__ __forceinline__ uint32_t batch_records(uint64_t n, uint64_t warps)
+{
+    uint32_t rb = RB;
+    while (rb > (uint32_t)RB_MIN && n < 4 * warps * rb) rb >>= 1;
+    return rb;
+}
+
+// One warp per batch of up to RB delta records (label B, row i, base, bits); lane r
 // owns record r for per-record work, and (record, k) tasks and their right-hand
 // items are flattened over the lanes so every phase keeps 32 independent memory
 // operations in flight.
@@ -1918,16 +1930,17 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
     unsigned long long ph[5] = {0, 0, 0, 0, 0};
     long long ph_t = clock64();
 #endif
-    // a persistent grid: each warp pulls its next batch of 32 records from the launch's
+    // a persistent grid: each warp pulls its next batch of records from the launch's
     // device queue (C_JQ, zeroed before the launch), so warps that drew light batches take
     // more of them instead of idling behind the ones that drew heavy records
-    const uint64_t nbatch = (n + RB - 1) / RB;
+    const uint32_t rb = batch_records(n, (uint64_t)gridDim.x * JOIN_WARPS);
+    const uint64_t nbatch = (n + rb - 1) / rb;
     uint64_t bt = 0;
     if (lane == 0) bt = atomicAdd(&d.ctr[C_JQ], 1ull);
     bt = __shfl_sync(0xffffffffu, bt, 0);
     for (; bt < nbatch; bt = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(&d.ctr[C_JQ], 1ull) : 0ull, 0)) {
-        const uint64_t ri = bt * RB + lane;
-        const bool have = ri < n;
+        const uint64_t ri = bt * rb + lane;
+        const bool have = lane < rb && ri < n;
         Bits rb;
         uint32_t key = EMPTY, row = 0;
         if (have) {
@@ -4365,7 +4378,7 @@ static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv,
 {
     cudaStream_t s = c->stream;
     if (split) {
-        launch_pass(c, grid_for(c, ((nd + nv) * SPLIT_PARTS + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->sbuf, 0,
+        launch_pass(c, grid_for(c, ((nd + nv) * SPLIT_PARTS + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0,
                     C_SPLIT_N, c->rbuf[0], joins);
         return;
     }
@@ -4373,16 +4386,16 @@ static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv,
         launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], tile_rows_lg(nd + nv));
         cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s);
         k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX);
-        launch_join(c, grid_for(c, (nd + nv + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
-        launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB, JOIN_WARPS, 16), s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0]);
+        launch_join(c, grid_for(c, (nd + nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
+        launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0]);
         c->launches += 5;
         joins += 3;
         return;
     }
-    launch_pass(c, grid_for(c, (nd + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
+    launch_pass(c, grid_for(c, (nd + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
     if (nv) {
         // virtual old-left records: joined by source rows only
-        launch_join(c, grid_for(c, (nv + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->vbuf, nv, -1, c->rbuf[0]);
+        launch_join(c, grid_for(c, (nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->vbuf, nv, -1, c->rbuf[0]);
         c->launches++;
         joins++;
     }
@@ -4430,7 +4443,7 @@ static int round_retries(grg_ctx *c, uint64_t nr, uint64_t nf, grg_stats &S, dou
             first_pass_joins(c, d, nd, nv, split, joins);
             rb = 0;
         } else if (nr) {
-            launch_pass(c, grid_for(c, (nr + RB - 1) / RB, JOIN_WARPS, 16), s, d, c->rbuf[rb], nr, -1, c->rbuf[rb ^ 1],
+            launch_pass(c, grid_for(c, (nr + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->rbuf[rb], nr, -1, c->rbuf[rb ^ 1],
                         joins);
             rb ^= 1;
         }
@@ -5886,7 +5899,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
         uint64_t n = nd;
         int rb = 0;
         for (int pass = 0;; pass++) {
-            const int g = grid((n + RB - 1) / RB, JOIN_WARPS, 16);
+            const int g = grid((n + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16);
             // each join launch pulls 32-record batches from a queue that starts at 0
             if (pass == 0 && nd + nv < (rt.nol ? tile_min(rt.nol) : (uint64_t)SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
                 // few records: their parts (in rbuf[1], free in this pass)
