@@ -63,7 +63,7 @@ enum : int {
     C_MAXR = C_LABEL0 + MAX_SLOTS + 3,  // rounds a device-driven launch may run (0 = until the fixpoint)
     C_WOUT = C_LABEL0 + MAX_SLOTS + 4,  // right-hand items the join's dense window could not hold
     C_SPLIT_N = C_LABEL0 + MAX_SLOTS + 5,  // sub-records of a small round (k_split)
-    C_JN1 = C_LABEL0 + MAX_SLOTS + 6,   // records the join reads from the gathered buffer this round
+    C_JN1 = C_LABEL0 + MAX_SLOTS + 6,   // records the join reads from the gathered buffer (or, after k_tile, as it left them) this round
     C_JN2 = C_LABEL0 + MAX_SLOTS + 7,   // records the join reads from the virtual-record buffer this round
     C_GT0 = C_LABEL0 + MAX_SLOTS + 8,   // start time of the current gather (kernel timing)
     C_GNS = C_LABEL0 + MAX_SLOTS + 9,   // gather nanoseconds (kernel timing)

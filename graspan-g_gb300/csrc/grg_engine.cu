@@ -1877,7 +1877,8 @@ __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__r
 // Records of a batch: 32, fewer while a warp would get less than 4 batches: the last batches of 32
 // dense records ran 1.3 to 2.5 ms after the rest. Closures (ms) with batches of 32 always, down to 16,
 // 8 and 4: 600-vertex points-to 3.3, 2.8, 2.7, 2.9; 37k-vertex alias 6.1, 5.6, 5.8, 5.9; 120k 8.7, 8.2,
-// 7.8, 8.1; 3,000 vertices in the static scratch 6.2, 5.7, 4.5, 4.5; 8 partitions of 200k 175, 158, 152, 152.
+// 7.8, 8.1; 3,000 vertices in the static scratch 6.2, 5.7, 4.5, 4.5; 8 partitions of 200k 175, 158, 152, 152;
+// dataflow (k_rows) 97k vertices 5.42, 5.20, 5.19, 5.27; 10k vertices in 52-element rows 7.37, 7.12, 7.20, 7.31.
 __device__ __forceinline__ uint32_t batch_records(uint64_t n, uint64_t warps)
 {
     uint32_t rb = RB;
@@ -2276,13 +2277,14 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
         }
         inserts = n_left = n_right = n_out = 0;
     };
-    const uint64_t nbatch = (n + RB - 1) / RB;
+    const uint32_t batch = batch_records(n, (uint64_t)gridDim.x * ROWS_WARPS);
+    const uint64_t nbatch = (n + batch - 1) / batch;
     uint64_t bt = 0;
     if (lane == 0) bt = atomicAdd(&d.ctr[C_JQ], 1ull);
     bt = __shfl_sync(0xffffffffu, bt, 0);
     for (; bt < nbatch; bt = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(&d.ctr[C_JQ], 1ull) : 0ull, 0)) {
-        const uint64_t ri = bt * RB + lane;
-        const bool have = ri < n;
+        const uint64_t ri = bt * batch + lane;
+        const bool have = lane < batch && ri < n;
         uint4 ra = make_uint4(0, 0, 0, 0), rb = make_uint4(0, 0, EMPTY, 0);
         if (have) ld32(recs + 2 * ri, ra, rb);
         const Bits bits = {{ra.x, ra.y, ra.z, ra.w, rb.x, rb.y}};
@@ -2738,8 +2740,8 @@ __global__ void k_grow(Dev d, uint64_t n)
 // slots are then taken one by one, a lane per bit of a bitmap word, so a dense word's 32 terms
 // are computed at once; a lane walking its own element's bits had 5 of 32 lanes at work (a row of
 // ~6 elements in 16 slots). The hash is bound by integer issue (64 lanes a clock a SM): ~50
-// instructions a term. Hash of the 2M-vertex dataflow closure (1.6e9 edges) 21.8 -> 4.1 ms, of
-// the 1M-vertex alias closure (2.3e9 edges) 30.7 -> 5 ms. All labels go in one launch: a
+// instructions a term. Hash of the 2M-vertex dataflow closure (1.6e9 edges) 21.8 -> 5.3 ms, of
+// the 1M-vertex alias closure (2.3e9 edges) 30.7 -> 7.1 ms. All labels go in one launch: a
 // points-to graph has 13, and a closure call counts three or four times.
 constexpr int COUNT_WARPS = 8;
 template <bool HASH>
