@@ -49,8 +49,8 @@ sys.path[:0] = [ROOT, os.path.join(ROOT, "graspan-g_gb300")]
 import numpy as np  # noqa: E402
 
 # DRAM bytes (read + write) per join pass measured by ncu on the named workload, with the file
-# that records the capture
-TRAFFIC = {("dataflow", 2000): (559.0e6, "profiles/traffic_dataflow_blocks_2000.md")}
+# that records the capture: none of the row and tile joins yet
+TRAFFIC = {}
 METRIC = "closure_edges_per_sec"
 UNIT = "edges/s"
 WORKLOAD = ("dataflow_blocks: 2000 blocks x 1000 vertices, 6M 'e' edges + 6M 'N' seeds, "
@@ -514,9 +514,7 @@ def main():
         join_ms = statistics.mean(x["join_ms"] for x in stats)
         launches = s["rounds"]
         achieved = alg_bytes / (join_ms * 1e-3) / 1e9 if (join_ms > 0 and alg_bytes) else None
-        # DRAM bytes per join pass (k_join + k_apply) of the headline closure, from a one-pass
-        # ncu capture of every launch of one closure (profiles/traffic_dataflow_blocks_2000.md);
-        # other workloads have no capture
+        # DRAM bytes per join pass, from a one-pass ncu capture of every launch of one closure
         traffic = TRAFFIC.get((args.workload, args.blocks)) if not s["column_labels"] else None
         cb = None if args.no_cpu_baseline else cpu_baseline(w)
         # the other configurations run once, on a single GPU (replica runs hold every GPU meanwhile)
@@ -557,7 +555,7 @@ def main():
             "e2e": {"value": world * total / (e2e_max * 1e-3), "unit": UNIT,
                     "h2d_bytes_per_step": int(w.num_edges * 9), "d2h_bytes_per_step": int(w.num_labels * 8)},
             "roofline": {"bound": "hbm",
-                         "kernel": "join pass (" + ("k_push" if s["column_labels"] else "k_join + k_apply") + ")",
+                         "kernel": "join pass (" + ("k_push" if s["column_labels"] else "k_rows, k_tile or k_join + k_apply") + ")",
                          "achieved": achieved, "peak": hbm,
                          "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": (achieved / hbm) if achieved else None,

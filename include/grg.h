@@ -56,7 +56,8 @@ typedef struct grg_stats {
     uint64_t rounds;               /* semi-naive rounds to the fixpoint */
     uint64_t delta_elems;          /* delta elements joined (sum over rounds) */
     uint64_t left_elems;           /* left-operand elements read by binary joins */
-    uint64_t right_elems;          /* right-operand elements read by binary joins */
+    uint64_t right_elems;          /* right-operand elements read by binary joins (a tile of rows
+                                      that shares its right-hand rows reads them once) */
     uint64_t out_elems;            /* elements written as new deltas */
     uint64_t retry_records;        /* delta records re-run after a table grew */
     uint64_t grow_rows;            /* rows whose table grew */
@@ -133,8 +134,11 @@ int grg_set_device_rounds(grg_ctx *ctx, int on);
  * narrow wins by 10% on a trial of at least 0.25 ms), and later closures with
  * the key reuse the choice (a process-wide cache). Mode 3 measures again even
  * when the key is cached, and updates the cache. Environment
- * GRG_JOIN_WINDOW=narrow / wide / tuned selects the default. Results are
- * identical in every mode. */
+ * GRG_JOIN_WINDOW=narrow / wide / tuned selects the default. Grammars with a
+ * derivable right-hand label join tiles of rows instead and use the window for
+ * small rounds and for what the tiles leave; with static right-hand rows, mode
+ * 2 or 3 here and for the items below joins by rows, whose window follows the
+ * width of each row. Results are identical in every mode. */
 int grg_set_join_window(grg_ctx *ctx, int mode);
 /* Right-hand items of labels that have a CSR copy (never derived, read as a
  * binary rule's second symbol): mode 0 reads destination ids (4 bytes each,
