@@ -512,6 +512,10 @@ def main():
             alg = s["left_elems"] + s["right_elems"] + s["out_elems"]
         alg_bytes = 32.0 * alg if alg is not None else None
         join_ms = statistics.mean(x["join_ms"] for x in stats)
+        joins = ctx.last_joins()
+        join_kernel = ("k_push" if s["column_labels"] else
+                       ("k_rows" if joins["rows"] else "k_tile + k_join" if joins["tiles"] else "k_join") +
+                       ("" if s["direct_inserts"] else " + k_apply"))
         launches = s["rounds"]
         achieved = alg_bytes / (join_ms * 1e-3) / 1e9 if (join_ms > 0 and alg_bytes) else None
         # DRAM bytes per join pass, from a one-pass ncu capture of every launch of one closure
@@ -533,15 +537,17 @@ def main():
                        "join_launches": s["join_launches"], "retry_records": s["retry_records"],
                        "grow_rows": s["grow_rows"], "delta_elems": s["delta_elems"],
                        "pool_elems_used": s["pool_elems_used"],
-                       "join_window": ("wide (12 elements)" if s["wide_window"] else "narrow (8 elements)") +
+                       "join_kernel": join_kernel,
+                       "join_window": "as wide as a row's records, up to 96 elements" if joins["rows"] else
+                       ("wide (12 elements)" if s["wide_window"] else "narrow (8 elements)") +
                        {0: ", fixed", 1: ", measured in this step", 2: ", tuned (degree-key cache)"}[
                            int(s["window_tuned"])],
                        "join_items": "table elements" if s["join_elements"] else "destination ids",
                        # one closure's join work: (record, rule) pairs, right-hand elements read, the
-                       # items ORed into the hash accumulator instead of a dense window, new elements
+                       # items outside the dense windows, new elements
                        "join_work": {"left_records": s["left_elems"], "right_elems": s["right_elems"],
-                                     "hash_items": s["window_out_elems"],
-                                     "hash_items_no_slot": s["window_noslot_items"], "out_elems": s["out_elems"],
+                                     "window_out_items": s["window_out_elems"],
+                                     "window_out_no_slot": s["window_noslot_items"], "out_elems": s["out_elems"],
                                      "candidates": s["candidates"], "join_inserts": s["join_inserts"],
                                      "direct_inserts": bool(s["direct_inserts"])},
                        # the first closure's trial passes (ms): windows [narrow, wide], item forms [ids, elements]
@@ -555,7 +561,7 @@ def main():
             "e2e": {"value": world * total / (e2e_max * 1e-3), "unit": UNIT,
                     "h2d_bytes_per_step": int(w.num_edges * 9), "d2h_bytes_per_step": int(w.num_labels * 8)},
             "roofline": {"bound": "hbm",
-                         "kernel": "join pass (" + ("k_push" if s["column_labels"] else "k_rows, k_tile or k_join + k_apply") + ")",
+                         "kernel": "join pass (" + join_kernel + ")",
                          "achieved": achieved, "peak": hbm,
                          "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": (achieved / hbm) if achieved else None,

@@ -77,7 +77,10 @@ enum : int {
     C_TQ = C_LABEL0 + MAX_SLOTS + 24,     // work queue of k_tile: next tile
     C_LN = C_LABEL0 + MAX_SLOTS + 25,     // records k_tile left to k_join
     C_TS = C_LABEL0 + MAX_SLOTS + 26,     // log2 of the rows of a tile in a device-driven round (0 = not tiled)
-    NCTR = C_LABEL0 + MAX_SLOTS + 27
+    C_TSUM = C_LABEL0 + MAX_SLOTS + 27,   // tiles joined over the closure
+    C_LSUM = C_LABEL0 + MAX_SLOTS + 28,   // records they left to k_join over the closure
+    C_JCNT = C_LABEL0 + MAX_SLOTS + 29,   // join launches of the device-driven rounds (grg_stats.join_launches)
+    NCTR = C_LABEL0 + MAX_SLOTS + 30
 };
 // error bits of C_ERR; ERR_IN_* (in C_BADIN) flag input edges that were refused
 // (label outside 1..L, vertex id outside the graph) and never touched a table

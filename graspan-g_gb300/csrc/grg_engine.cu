@@ -25,6 +25,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -1367,6 +1368,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
     if (!sh) sh = (uint32_t)d.ctr[C_TS];
     if (!sh) return;
     const uint64_t ntiles = min((uint64_t)d.ctr[C_TN], list_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr[C_TSUM] += ntiles;
     const uint64_t nd = d.ctr[C_DIRTY_N], nv = d.ctr[C_VN];
     const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, rows = 1u << sh;
     // in the joins, lanes 0-11 and 16-27 hold a row's 12 quads of 16 bytes (12-15 and 28-31 repeat the last)
@@ -1802,14 +1804,21 @@ constexpr uint32_t SPLIT_PARTS = (EIDS + SPLIT_BITS - 1) / SPLIT_BITS;
 // SPLIT_BITS, more by bitmap word, up to as many as the buffer holds 6 parts of. 37k-vertex alias
 // closure 6.8 -> 6.0 ms.
 constexpr int SPLIT_LEFT = 2;
+// Launches of a round's first join pass that have records to join: the parts of a small round, the tiles
+// and the two lists they leave, or the gathered and the virtual records. passes: kernels of a pass.
+__host__ __device__ inline uint32_t join_launches(bool split, bool tiles, uint64_t nv, uint32_t passes)
+{
+    return split ? passes : tiles ? 3u : passes + (nv ? 1u : 0u);
+}
 constexpr uint64_t SPLIT_LEFT_MAX = (uint64_t)SPLIT_MAX * SPLIT_PARTS / EW;
 
 // tile: 1: the rounds that are not split go through k_tile (C_TS: its rows), not k_join; SPLIT_LEFT: the
 // records are those that k_tile left (C_LN of grecs), and those not split are joined as they are (C_JN1).
 // A thread cuts one bitmap word of a record (up to 4 parts), and a warp reserves its parts' room
 // at once, in record order: a thread a record took 14 us for the 192 bits of a dense one.
+// passes (round graphs, else 0): join kernels of a pass, for the count of their launches (C_JCNT).
 __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out, int tile,
-                        uint64_t split_max)
+                        uint64_t split_max, uint32_t passes)
 {
     if (d.ctr[C_HALT]) return;
     const bool left = tile == SPLIT_LEFT;
@@ -1819,6 +1828,8 @@ __global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__r
         d.ctr[C_JN1] = split || tile == 1 ? 0 : nd;
         d.ctr[C_JN2] = split || tile ? 0 : nv;
         if (!left) d.ctr[C_TS] = split || !tile ? 0 : tile_rows_lg(nd + nv);
+        if (left) d.ctr[C_LSUM] += nd;
+        if (passes) d.ctr[C_JCNT] += join_launches(split, tile != 0, nv, passes);
     }
     if (!split) return;
     // bits of a part: 8, or a word's when more records are left than the buffer holds 24 parts of
@@ -3130,9 +3141,11 @@ struct grg_ctx {
     bool join_elems = false;               // the form of this closure
     bool tuned_elems = false;
     bool join_rows = false;                // this closure's joins run k_rows (see rows_possible)
+    bool tuned_rows = true;                // false: measured slower than k_join on this degree key
+    grg_join_info joins{};                 // what the joins of the last closure ran
     float items_ms[2] = {0, 0};            // measured (ids, elements) when tuned in this closure
     bool tune_pending = false;             // measure both windows in the first large round
-    uint64_t tune_key = 0;
+    uint64_t tune_key = 0, tune_input = 0; // degree key; its part that needs no look at the tables
     int tune_source = 0;                   // grg_stats.window_tuned
     float tune_ms[2] = {0, 0};
     cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
@@ -3981,7 +3994,7 @@ static void choose_window(grg_ctx *c)
 {
     c->join_wide = c->join_window_mode >= 2 ? c->tuned_wide : c->join_window_mode != 0;
     c->join_elems = c->items_mode >= 2 ? c->tuned_elems : c->items_mode != 0;
-    c->join_rows = c->join_window_mode >= 2 && c->items_mode >= 2 && rows_possible(c);
+    c->join_rows = c->tuned_rows && c->join_window_mode >= 2 && c->items_mode >= 2 && rows_possible(c);
     c->push_flat = c->push_mode >= 2 ? c->tuned_flat : c->push_mode != 0;
 }
 
@@ -4058,6 +4071,8 @@ static void set_passes(grg_ctx *c)
     }
 }
 
+static uint32_t pass_kernels(const grg_ctx *c) { return (c->need_join ? 1u : 0u) + (c->need_push ? 1u : 0u); }
+
 // One join pass over n records (or the device count n_ctr): the kernels the rule
 // table needs, each taking its own records and skipping the others'.
 static void launch_pass(grg_ctx *c, int grid, cudaStream_t s, const Dev &d, const uint4 *recs, uint64_t n, int n_ctr,
@@ -4090,8 +4105,9 @@ static void launch_pass(grg_ctx *c, int grid, cudaStream_t s, const Dev &d, cons
 // applying a candidate or re-running a record twice adds nothing.
 
 static std::mutex g_tune_mu;
-struct JoinChoice { bool wide, elems; };
+struct JoinChoice { bool wide, elems, rows; };
 static std::map<uint64_t, JoinChoice> g_tune_cache;    // degree key -> the faster window and item form
+static std::set<uint64_t> g_rows_measured;             // input keys with a measured choice against k_rows
 static std::map<uint64_t, bool> g_push_cache;          // degree key -> flattened push faster
 constexpr uint64_t TUNE_MIN_RECORDS = 1u << 16;        // smaller first rounds are not timed
 // The narrow window replaces the wide default only when the wide trial pass takes at least
@@ -4099,6 +4115,20 @@ constexpr uint64_t TUNE_MIN_RECORDS = 1u << 16;        // smaller first rounds a
 // swap places by more than the 10% margin from run to run, and the narrow window then
 // costs ~11% over the closure
 constexpr float TUNE_WINDOW_MIN_MS = 0.25f;
+
+// The part of the key that needs no look at the tables: grammar, filter, vertex count.
+static uint64_t input_key(const grg_ctx *c, uint32_t filter)
+{
+    uint64_t h = 1469598103934665603ull;
+    auto mix = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
+    mix((uint64_t)c->L);
+    mix(filter);
+    for (int q = 0; q < 3 * c->R; q++) mix((uint64_t)c->rules[q]);
+    uint32_t vb = 0;
+    while ((1ull << vb) < c->V) vb++;
+    mix(vb);
+    return h;
+}
 
 static int degree_key(grg_ctx *c, uint32_t filter, uint64_t *key)
 {
@@ -4108,14 +4138,8 @@ static int degree_key(grg_ctx *c, uint32_t filter, uint64_t *key)
     c->launches++;
     int st = read_ctr(c);
     if (st) return st;
-    uint64_t h = 1469598103934665603ull, tot = 0;
+    uint64_t h = input_key(c, filter), tot = 0;
     auto mix = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
-    mix((uint64_t)c->L);
-    mix(filter);
-    for (int q = 0; q < 3 * c->R; q++) mix((uint64_t)c->rules[q]);
-    uint32_t vb = 0;
-    while ((1ull << vb) < c->V) vb++;
-    mix(vb);
     for (int b = 0; b < 8; b++) tot += c->h_ctr[C_DH0 + b];
     for (int b = 0; b < 8; b++) mix(tot ? c->h_ctr[C_DH0 + b] * 8 / tot : 0);
     *key = h;
@@ -4131,8 +4155,18 @@ static int tune_begin(grg_ctx *c, uint32_t filter)
     c->items_ms[0] = c->items_ms[1] = 0;
     c->push_ms[0] = c->push_ms[1] = 0;
     // only the choices this closure's pass kernels make are tuned (the window is
-    // k_join's; the push kernel is timed only when the pass is pushes alone)
-    const bool tune_window = (c->join_window_mode >= 2 || c->items_mode >= 2) && c->need_join;
+    // k_join's; the push kernel is timed only when the pass is pushes alone). Where
+    // k_rows can run it does, untimed, unless a mode of 3 has it measured against
+    // k_join, now or in an earlier closure of the process
+    c->tuned_rows = true;
+    c->tune_input = input_key(c, filter);
+    const bool again = c->join_window_mode == 3 || c->items_mode == 3;
+    const bool rows = c->join_window_mode >= 2 && c->items_mode >= 2 && rows_possible(c);
+    bool tune_window = (c->join_window_mode >= 2 || c->items_mode >= 2) && c->need_join;
+    if (rows && !again) {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        tune_window = g_rows_measured.count(c->tune_input) > 0;
+    }
     const bool tune_push = c->push_mode >= 2 && c->need_push && !c->need_join;
     if (!tune_window && !tune_push) return GRG_OK;
     int st = degree_key(c, filter, &c->tune_key);
@@ -4140,14 +4174,15 @@ static int tune_begin(grg_ctx *c, uint32_t filter)
     std::lock_guard<std::mutex> lk(g_tune_mu);
     if (tune_window) {
         auto it = g_tune_cache.find(c->tune_key);
-        if (it != g_tune_cache.end() && c->join_window_mode != 3 && c->items_mode != 3) {
+        if (it != g_tune_cache.end() && !again) {
             c->tuned_wide = it->second.wide;
             c->tuned_elems = it->second.elems;
+            c->tuned_rows = it->second.rows;
             c->tune_source = 2;
         } else {
             c->tuned_wide = true;
             c->tuned_elems = false;
-            c->tune_pending = true;
+            c->tune_pending = !rows || again;
         }
     }
     if (tune_push) {
@@ -4188,27 +4223,33 @@ static int tune_first_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, u
     // interleaved, keeping each one's best time
     const bool tw = c->join_window_mode >= 2, ti = c->items_mode >= 2 && any_csr(c);
     const bool fix_wide = c->join_wide, fix_elems = c->join_elems, rows = c->join_rows;
-    c->join_rows = false;                    // (k_rows has neither windows nor item forms to choose)
-    float best[2][2] = {{1e30f, 1e30f}, {1e30f, 1e30f}};        // [wide][elems]
-    for (int rep = -1; rep < 2; rep++)
+    float best[2][2] = {{1e30f, 1e30f}, {1e30f, 1e30f}}, best_rows = 1e30f;        // [wide][elems], k_rows
+    auto trial = [&](bool timed, float &ms_best) -> int {
+        if (timed) GRG_CUDA(c, cudaEventRecord(c->ev_t0, s));
+        launch_join(c, grid, s, d, c->gbuf, nt, -1, c->rbuf[0]);
+        c->launches++;
+        joins++;
+        if (!timed) return GRG_OK;
+        float ms = 0;
+        GRG_CUDA(c, cudaEventRecord(c->ev_t1, s));
+        GRG_CUDA(c, cudaEventSynchronize(c->ev_t1));
+        GRG_CUDA(c, cudaEventElapsedTime(&ms, c->ev_t0, c->ev_t1));
+        ms_best = std::min(ms_best, ms);
+        return GRG_OK;
+    };
+    for (int rep = -1; rep < 2; rep++) {
+        if (rows && (st = trial(rep >= 0, best_rows))) return st;
+        c->join_rows = false;
         for (int w = 0; w < 2; w++)
             for (int e = 0; e < 2; e++) {
                 if ((!tw && w != (int)fix_wide) || (!ti && e != (int)fix_elems)) continue;
                 if (rep < 0 && !(w == 1 || !tw)) continue;         // one untimed (wide) pass per item form
                 c->join_wide = w == 1;
                 c->join_elems = e == 1;
-                if (rep >= 0) GRG_CUDA(c, cudaEventRecord(c->ev_t0, s));
-                launch_join(c, grid, s, d, c->gbuf, nt, -1, c->rbuf[0]);
-                c->launches++;
-                joins++;
-                if (rep < 0) continue;
-                float ms = 0;
-                GRG_CUDA(c, cudaEventRecord(c->ev_t1, s));
-                GRG_CUDA(c, cudaEventSynchronize(c->ev_t1));
-                GRG_CUDA(c, cudaEventElapsedTime(&ms, c->ev_t0, c->ev_t1));
-                best[w][e] = std::min(best[w][e], ms);
+                if ((st = trial(rep >= 0, best[w][e]))) return st;
             }
-    c->join_rows = rows;
+        c->join_rows = rows;
+    }
     // the statistics count the round's own pass only
     for (int i = 0; i < 5; i++) {
         c->h_ctr[kept[i]] = keep[i];
@@ -4236,11 +4277,16 @@ static int tune_first_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, u
     c->items_ms[1] = ti ? t_of[1] : 0.f;
     c->tuned_wide = c->join_wide = wide;
     c->tuned_elems = c->join_elems = elems;
+    // k_rows stays unless k_join beats it by a margin (its windows follow the rows of later rounds,
+    // which are wider than the first's)
+    c->tuned_rows = !rows || !(t_of[elems ? 1 : 0] < 0.9f * best_rows);
+    c->join_rows = rows && c->tuned_rows;
     c->tune_pending = false;
     c->tune_source = 1;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tune_cache[c->tune_key] = JoinChoice{wide, elems};
+        g_tune_cache[c->tune_key] = JoinChoice{wide, elems, c->tuned_rows};
+        if (rows) g_rows_measured.insert(c->tune_input);
     }
     first_pass_joins(c, d, nd, nv, false, joins);
     return GRG_OK;
@@ -4387,11 +4433,11 @@ static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv,
     if (use_tiles(c)) {
         launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], tile_rows_lg(nd + nv));
         cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s);
-        k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX);
+        k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX, 0);
         launch_join(c, grid_for(c, (nd + nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
         launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0]);
         c->launches += 5;
-        joins += 3;
+        joins += join_launches(false, true, nv, pass_kernels(c));
         return;
     }
     launch_pass(c, grid_for(c, (nd + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
@@ -4504,7 +4550,7 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
     if (split) {
         // few records: their parts spread the join over more warps
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_SPLIT_N, 0, 8, s));
-        k_split<<<grid_for(c, (nd + nv) * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, 0, split_max(c));
+        k_split<<<grid_for(c, (nd + nv) * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, 0, split_max(c), 0);
         c->launches++;
     }
     if (c->tune_pending && c->need_join && !split && nd >= TUNE_MIN_RECORDS) {
@@ -4691,14 +4737,15 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
     }
     const int jgrid = grid_for(c, ~0u, JOIN_WARPS, 16);
     const bool tiles = use_tiles(c);
-    k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles, split_max(c));
+    k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles, split_max(c),
+                                                            pass_kernels(c));
     nk++;
     {
         const uint64_t launches0 = c->launches;
         uint64_t unused = 0;
         if (tiles) {
             launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], 0);
-            k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX);
+            k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX, 0);
             launch_join(c, jgrid, s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
             nk += 4;
         } else {
@@ -4797,7 +4844,8 @@ static int run_rounds(grg_ctx *c, uint64_t max_rounds, grg_stats &S, double &joi
         const unsigned long long halt = c->h_ctr[C_HALT], rounds = c->h_ctr[C_GROUNDS];
         S.rounds += rounds;
         S.delta_elems += c->h_ctr[C_GDSUM];
-        joins += rounds * ((c->need_join ? 1 : 0) + (c->need_push ? 1 : 0) + (c->rt.nol ? 1 : 0));
+        joins += c->h_ctr[C_JCNT];
+        GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_JCNT, 0, 8, s));
         c->launches += c->h_ctr[C_ITERS] * c->rg_kernels;
         join_ms += c->h_ctr[C_JNS] * 1e-6;
         done_rounds += rounds;
@@ -4850,7 +4898,6 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
     if (!c || filter > 1) return GRG_E_ARG;
     if (!c->loaded) return fail(c, GRG_E_STATE, "grg_load_edges must come first");
     c->run_stamp = run_stamp;
-    choose_window(c);
     if (c->closed) return fail(c, GRG_E_STATE, "closure already computed; reload the graph");
     cudaSetDevice(c->device);
     RuleTable rt;
@@ -4862,8 +4909,6 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
     grg_stats S;
     memset(&S, 0, sizeof S);
     GRG_CUDA(c, cudaEventRecord(c->ev_a, s));
-    if ((st = tune_begin(c, filter))) return st;
-    choose_window(c);
     Dev d = make_dev(c);
     // labels never inserted into after the load are packed
     bool derivable[MAX_LABELS + 1] = {false};
@@ -4925,6 +4970,7 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
     }
     c->rt = rt;
     set_passes(c);
+    if ((st = tune_begin(c, filter))) return st;     // (which joins can run depends on the copies)
     st = read_ctr(c);
     if (st) return st;
     const uint64_t top = c->h_ctr[C_POOL_TOP];
@@ -4958,12 +5004,15 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
     S.join_inserts = c->h_ctr[C_INSERTS];
     S.direct_inserts = c->cand_cap == 0;
     S.gather_ms = c->h_ctr[C_GNS] * 1e-6;
-    S.wide_window = c->join_wide ? 1 : 0;
+    S.wide_window = c->join_wide && !c->join_rows ? 1 : 0;
     S.window_tuned = (uint64_t)c->tune_source;
     S.window_trial_ms[0] = c->tune_ms[0];
     S.window_trial_ms[1] = c->tune_ms[1];
     S.column_labels = c->tmask;
-    S.join_elements = c->need_join && c->join_elems && any_csr(c) ? 1 : 0;
+    S.join_elements = c->need_join && !c->join_rows && c->join_elems && any_csr(c) ? 1 : 0;
+    c->joins.rows = c->join_rows ? 1 : 0;
+    c->joins.tiles = c->h_ctr[C_TSUM];
+    c->joins.tile_left = c->h_ctr[C_LSUM];
     S.items_trial_ms[0] = c->items_ms[0];
     S.items_trial_ms[1] = c->items_ms[1];
     S.push_flat = c->need_push && c->push_flat ? 1 : 0;
@@ -4984,6 +5033,13 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
     for (int l = 0; l < c->L; l++) S.total_edges += counts[l];
     S.kernel_launches = c->launches;
     if (stats) *stats = S;
+    return GRG_OK;
+}
+
+int grg_last_joins(const grg_ctx *c, grg_join_info *out)
+{
+    if (!c || !out) return GRG_E_ARG;
+    *out = c->joins;
     return GRG_OK;
 }
 
@@ -5906,7 +5962,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
             if (pass == 0 && nd + nv < (rt.nol ? tile_min(rt.nol) : (uint64_t)SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
                 // few records: their parts (in rbuf[1], free in this pass)
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
-                k_split<<<grid((nd + nv) * EW, 256, 8), 256, 0, s>>>(d, gbuf, vbuf, rbuf[1], 0, ~0ull);
+                k_split<<<grid((nd + nv) * EW, 256, 8), 256, 0, s>>>(d, gbuf, vbuf, rbuf[1], 0, ~0ull, 0);
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
                 k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_SPLIT_N, rbuf[0]);
             } else if (pass == 0 && rt.nol) {

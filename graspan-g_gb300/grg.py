@@ -35,7 +35,7 @@ EXPORTS = (
     "grg_part_destroy", "grg_part_load_edges", "grg_part_run", "grg_part_label_counts", "grg_part_bounds",
     "grg_set_device_rounds", "grg_range_reach", "grg_set_join_window", "grg_export_csr5", "grg_load_csr5",
     "grg_part_export_csr5", "grg_part_save", "grg_part_restore", "grg_part_set_checkpoint", "grg_part_set_run_budget",
-    "grg_set_layout", "grg_set_push", "grg_set_join_items",
+    "grg_set_layout", "grg_set_push", "grg_set_join_items", "grg_last_joins",
 )
 
 
@@ -68,6 +68,10 @@ class Stats(ctypes.Structure):
         d["push_trial_ms"] = list(d["push_trial_ms"])
         d["items_trial_ms"] = list(d["items_trial_ms"])
         return d
+
+
+class JoinInfo(ctypes.Structure):
+    _fields_ = [("rows", ctypes.c_uint64), ("tiles", ctypes.c_uint64), ("tile_left", ctypes.c_uint64)]
 
 
 class PartStats(ctypes.Structure):
@@ -117,6 +121,7 @@ def load_library(path: str = LIB_PATH):
     L.grg_allocate_pool.argtypes = [P, U64]
     L.grg_load_edges.argtypes = [P, U32, U64, P, P, P, I]
     L.grg_closure.argtypes = [P, U32, ctypes.POINTER(Stats)]
+    L.grg_last_joins.argtypes = [P, ctypes.POINTER(JoinInfo)]
     L.grg_label_counts.argtypes = [P, P]
     L.grg_get_degree.argtypes = [P, U32, U32, P]
     L.grg_set_hash.argtypes = [P, ctypes.POINTER(U64)]
@@ -304,6 +309,12 @@ class Context:
         s = Stats()
         self._check(self._L.grg_closure(self._h, filter_flag, ctypes.byref(s)), "closure")
         return s.as_dict()
+
+    def last_joins(self) -> dict:
+        """What the last closure's joins ran: by rows (0 / 1), tiles, records the tiles left."""
+        j = JoinInfo()
+        self._check(self._L.grg_last_joins(self._h, ctypes.byref(j)), "last_joins")
+        return {k: getattr(j, k) for k, _ in j._fields_}
 
     def label_counts(self) -> np.ndarray:
         out = np.zeros(self.num_labels, dtype=np.uint64)

@@ -65,18 +65,21 @@ typedef struct grg_stats {
     uint64_t pool_elems_cap;       /* pool slots allocated */
     double closure_ms;             /* device time from resident graph to fixpoint known */
     double join_ms;                /* sum of join-kernel durations (when kernel timing is on) */
-    uint64_t join_launches;        /* join-kernel launches (first pass + retries) */
+    uint64_t join_launches;        /* join-kernel launches for a list of records (first pass +
+                                      retries; a round that goes through tiles counts three) */
     uint64_t kernel_launches;      /* all kernel launches of the closure */
     uint64_t join_phase_cycles[5]; /* join-kernel cycles per phase (record load, unary,
                                       binary join, flush, retry list) when built with
                                       -DGRG_PHASE_TIMERS; 0 otherwise */
-    uint64_t window_out_elems;     /* right-hand items the join ORed into its hash
-                                      accumulator: beyond the record's dense window, or of a
-                                      run of records left without a window slot */
-    uint64_t wide_window;          /* 1 = the closure ended on the wide join window */
+    uint64_t window_out_elems;     /* right-hand items outside the join's dense windows: ORed into
+                                      the hash accumulator (k_join; also those of a run of records
+                                      left without a window slot), written as candidates of one
+                                      bit (joins by rows) */
+    uint64_t wide_window;          /* 1 = the closure ended on the wide join window (0 when it
+                                      joined by rows, see grg_last_joins) */
     double gather_ms;              /* time of the rounds' gathers (when kernel timing is on) */
-    uint64_t window_tuned;         /* how the join window was chosen: 0 fixed by grg_set_join_window,
-                                      1 measured in this closure, 2 taken from the tuning cache */
+    uint64_t window_tuned;         /* how the join window was chosen: 0 fixed by grg_set_join_window
+                                      or nothing to choose (joins by rows), 1 measured in this closure, 2 taken from the tuning cache */
     double window_trial_ms[2];     /* the measured trial passes (narrow, wide) when window_tuned = 1 */
     uint64_t column_labels;        /* labels stored by destination in this closure (bit l-1 = label l;
                                       grg_set_layout); their joins are pushes, so right_elems then
@@ -100,6 +103,14 @@ typedef struct grg_stats {
                                       environment GRG_DIRECT_INSERTS=0 / 1 overrides), 0 = they
                                       wrote candidates that k_apply inserted */
 } grg_stats;
+
+/* What the joins of the context's last closure ran. */
+typedef struct grg_join_info {
+    uint64_t rows;                 /* 1 = joins by rows (k_rows: static right-hand rows) */
+    uint64_t tiles;                /* tiles of neighbouring rows joined (k_tile: grammars with a
+                                      derivable right-hand label) */
+    uint64_t tile_left;            /* records the tiles left to the plain join */
+} grg_join_info;
 
 /* Error text of a status code, and the last detailed message of a context. */
 const char *grg_error_string(int status);
@@ -217,6 +228,8 @@ int grg_closure(grg_ctx *ctx, uint32_t filter, grg_stats *stats);
  * closes the loaded vertex ranges together, like one spagpu_s/spagpu_b/spagpu
  * pass over a partition or a pair of partitions (src/kernel.cu:466-780). */
 int grg_closure_ex(grg_ctx *ctx, uint32_t filter, uint32_t run_stamp, grg_stats *stats);
+/* Which join kernels the last closure of the context ran. */
+int grg_last_joins(const grg_ctx *ctx, grg_join_info *info);
 
 /* Per-label closure edge counts: counts[l-1] for label l (num_labels values). */
 int grg_label_counts(grg_ctx *ctx, uint64_t *counts);

@@ -118,3 +118,47 @@ def test_stream_edges_of_tiles(grg_mod, ne, fill, shift):
         w, d = pack_csr5(e[:, 0], e[:, 2], e[:, 1], lo, hi)
         assert np.array_equal(got, w) and np.array_equal(gdeg, d)
     ctx.close()
+
+
+@pytest.mark.parametrize("device_rounds", [True, False])
+def test_joins_by_rows_are_reported(grg_mod, oracle_mod, device_rounds):
+    """A closure that joins by rows times no window and no item form of the plain join and reports none;
+    one that measures them (mode 3) may keep either kernel and says which; fixed ones run the plain join."""
+    w = G.dataflow_blocks(seed=31, num_blocks=70 + 65 * device_rounds, block=1000, num_edges=210_000 + 195_000 * device_rounds)
+    # a grammar of its own (X ::= N e beside N ::= N e): no other test has measured it in this process
+    n, e = w.labels.index("N") + 1, w.labels.index("e") + 1
+    rules, nl = np.array([[n, n, e], [w.num_labels + 1, n, e]], np.int32), w.num_labels + 1
+    r = oracle_mod.closure(w.num_vars, rules, nl, w.filter_flag, w.src, w.dst, w.lab)
+    want = (r.label_counts().tolist(), r.set_hash)
+    rows = []
+    for window, items in ((2, 2), (3, 3), (2, 2), (1, 1)):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(device_rounds)
+            ctx.set_join_window(window)
+            ctx.set_join_items(items)
+            ctx.transfer_rules(rules, nl)
+            ctx.load_edges(w.num_vars, w.src, w.dst, w.lab)
+            st = ctx.closure(w.filter_flag)
+            assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
+            j = ctx.last_joins()
+        assert (j["tiles"], j["tile_left"]) == (0, 0)
+        if j["rows"]:
+            assert st["wide_window"] == 0 and st["join_elements"] == 0
+        rows.append((j["rows"], st["window_tuned"], st["window_trial_ms"]))
+    assert rows[0] == (1, 0, [0.0, 0.0])                  # nothing to choose, nothing timed
+    assert rows[1][1] == 1 and min(rows[1][2]) > 0
+    assert rows[2] == (rows[1][0], 2, [0.0, 0.0])         # the measured choice holds for later closures
+    assert rows[3][:2] == (0, 0)
+
+
+def test_join_launches_are_those_with_records(grg_mod):
+    """A round of few records is joined in one launch, whether the host or the device drives it."""
+    w = G.alias(seed=8, num_vars=300, num_base_edges=900, block=100)
+    for dev in (True, False):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(dev)
+            ctx.transfer_rules(w.rule_ids(), w.num_labels)
+            ctx.load_edges(w.num_vars, w.src, w.dst, w.lab)
+            st = ctx.closure(0)
+            assert st["retry_records"] == 0 and ctx.last_joins()["tiles"] == 0
+            assert st["join_launches"] == st["rounds"]
