@@ -768,8 +768,11 @@ int run_once(grg_part *p, uint32_t filter, const RunInput &in, uint32_t run_stam
         if ((st = grg_closure_ex(p->ctx, filter, run_stamp, &cs))) return st;
     }
     // partitions of one graph share its degree distribution: the window the first tuned
-    // run chose holds for the rest (no trial per partition)
-    if (cs.window_tuned && !p->window_pinned) {
+    // run chose holds for the rest (no trial per partition). Joins by rows have no window,
+    // and a fixed one would keep later runs from them
+    grg_join_info ji;
+    if ((st = grg_last_joins(p->ctx, &ji))) return st;
+    if (cs.window_tuned && !ji.rows && !p->window_pinned) {
         grg_set_join_window(p->ctx, cs.wide_window ? 1 : 0);
         grg_set_join_items(p->ctx, cs.join_elements ? 1 : 0);
         p->window_pinned = true;

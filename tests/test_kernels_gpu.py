@@ -162,3 +162,19 @@ def test_join_launches_are_those_with_records(grg_mod):
             st = ctx.closure(0)
             assert st["retry_records"] == 0 and ctx.last_joins()["tiles"] == 0
             assert st["join_launches"] == st["rounds"]
+
+
+def test_partitions_keep_the_row_join(grg_mod, oracle_mod):
+    """Runs of a partitioned graph choose their joins as a single closure does: none of them fixes the window
+    of the plain join for the runs after it."""
+    w = G.dataflow_blocks(seed=12, num_blocks=160, block=1000, num_edges=480_000)
+    r = oracle_mod.closure(w.num_vars, w.rule_ids(), w.num_labels, w.filter_flag, w.src, w.dst, w.lab)
+    with grg_mod.Context(0) as ctx:
+        ctx.transfer_rules(w.rule_ids(), w.num_labels)
+        p = grg_mod.Partitioned(ctx, w.num_vars, 2)
+        p.load_edges(w.src, w.dst, w.lab)
+        assert p.run(w.filter_flag)["runs"] >= 2
+        counts, h = p.label_counts()
+        p.close()
+        assert (counts.tolist(), h) == (r.label_counts().tolist(), r.set_hash)
+        assert ctx.last_joins()["rows"] == 1
