@@ -3130,6 +3130,8 @@ struct grg_ctx {
     uint64_t xcap = 0;
     uint64_t pool_limit = 0;               // maximum pool slots (0 = what the device holds)
     uint64_t retry_min = 1ull << 20;       // smallest retry list (records; GRG_RETRY_ROOM)
+    uint64_t tile_room = ~0ull;            // records the tile lists may hold (GRG_TILE_ROOM)
+    bool tiles_off = false;                // the loaded graph needed their memory
     uint64_t prefix_mask = 0;              // labels with prefix-filled small tables (Dev::prefix_mask)
     // join window: narrow (WIN) or wide (WIN2, the default)
     bool join_wide = true;
@@ -3306,6 +3308,30 @@ int read_ctr(grg_ctx *c)
     return GRG_OK;
 }
 
+// Gives the tile lists back (the joins then run without tiles); whether there were any. cudaFree waits
+// for the work that uses them.
+bool free_tiles(grg_ctx *c)
+{
+    const bool had = c->lbuf || c->tlist;
+    cudaFree(c->lbuf);
+    cudaFree(c->tlist);
+    c->lbuf = nullptr;
+    c->tlist = nullptr;
+    c->lbuf_cap = 0;
+    return had;
+}
+
+// cudaMalloc for what a closure cannot do without: the tile lists make room before it fails.
+template <class T>
+cudaError_t must_alloc(grg_ctx *c, T **p, uint64_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !free_tiles(c)) return e;
+    cudaGetLastError();
+    c->tiles_off = true;                   // this graph's later rounds leave the memory alone too
+    return cudaMalloc(p, bytes);
+}
+
 // Device staging of num_edges input edges (src and dst in d_in32, labels in d_in8).
 static int ensure_input(grg_ctx *c, uint64_t num_edges)
 {
@@ -3313,8 +3339,8 @@ static int ensure_input(grg_ctx *c, uint64_t num_edges)
     cudaFree(c->d_in32); cudaFree(c->d_in8);
     c->d_in32 = nullptr; c->d_in8 = nullptr;
     c->in_cap = 0;
-    GRG_CUDA(c, cudaMalloc(&c->d_in32, num_edges * 8));
-    GRG_CUDA(c, cudaMalloc(&c->d_in8, num_edges));
+    GRG_CUDA(c, must_alloc(c, &c->d_in32, num_edges * 8));
+    GRG_CUDA(c, must_alloc(c, &c->d_in8, num_edges));
     c->in_cap = num_edges;
     return GRG_OK;
 }
@@ -3338,8 +3364,8 @@ int alloc_pool(grg_ctx *c, uint64_t elems)
     if (elems > 0xFFFFFFE0ull) elems = 0xFFFFFFE0ull;
     const uint64_t words = elems / 32 + 2;
     uint32_t *e = nullptr, *b = nullptr, *m = nullptr, *t = nullptr;
-    if (cudaMalloc(&e, elems * 32) != cudaSuccess || cudaMalloc(&b, elems * 32) != cudaSuccess ||
-        cudaMalloc(&m, words * 4) != cudaSuccess || (c->stamp_on && cudaMalloc(&t, elems * 4) != cudaSuccess)) {
+    if (must_alloc(c, &e, elems * 32) != cudaSuccess || must_alloc(c, &b, elems * 32) != cudaSuccess ||
+        must_alloc(c, &m, words * 4) != cudaSuccess || (c->stamp_on && must_alloc(c, &t, elems * 4) != cudaSuccess)) {
         cudaGetLastError();
         cudaFree(e); cudaFree(b); cudaFree(m); cudaFree(t);
         return fail(c, GRG_E_NOMEM, "cannot allocate element pool of " + std::to_string(elems) + " slots");
@@ -3372,7 +3398,7 @@ int ensure_chunks(grg_ctx *c, uint64_t nchunks)
     if (need <= c->chunk_cap) return GRG_OK;
     cudaFree(c->chunk);
     c->chunk = nullptr;
-    GRG_CUDA(c, cudaMalloc(&c->chunk, need * 2 * 4));
+    GRG_CUDA(c, must_alloc(c, &c->chunk, need * 2 * 4));
     c->chunk_cap = need * 2;
     return GRG_OK;
 }
@@ -3383,6 +3409,10 @@ int grow_pool(grg_ctx *c, uint64_t min_elems)
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
     uint64_t fit = (uint64_t)((double)fr * 0.9) / POOL_BYTES_PER_SLOT;
+    if (want > fit && free_tiles(c)) {     // the tile lists count as free
+        cudaMemGetInfo(&fr, &tot);
+        fit = (uint64_t)((double)fr * 0.9) / POOL_BYTES_PER_SLOT;
+    }
     if (want > fit) want = fit;
     if (c->pool_limit && want > c->pool_limit) want = c->pool_limit;
     if (want <= c->pool_cap) return fail(c, GRG_E_NOMEM, "element pool exhausted and device memory is full");
@@ -3443,7 +3473,7 @@ int ensure_buf(grg_ctx *c, uint4 **buf, uint64_t *cap, uint64_t n)
     cudaFree(*buf);
     *buf = nullptr;
     *cap = 0;
-    GRG_CUDA(c, cudaMalloc(buf, nc * 32));
+    GRG_CUDA(c, must_alloc(c, buf, nc * 32));
     *cap = nc;
     return GRG_OK;
 }
@@ -3457,7 +3487,7 @@ int ensure_gather(grg_ctx *c, uint64_t n)
     cudaFree(c->gslot);
     c->gslot = nullptr;
     c->gslot_cap = 0;
-    GRG_CUDA(c, cudaMalloc(&c->gslot, c->gbuf_cap * 4));
+    GRG_CUDA(c, must_alloc(c, &c->gslot, c->gbuf_cap * 4));
     c->gslot_cap = c->gbuf_cap;
     return GRG_OK;
 }
@@ -3472,7 +3502,7 @@ int ensure_rbuf(grg_ctx *c, uint64_t n)
         c->rbuf[i] = nullptr;
     }
     c->rbuf_cap = 0;
-    for (int i = 0; i < 2; i++) GRG_CUDA(c, cudaMalloc(&c->rbuf[i], cap * 32));
+    for (int i = 0; i < 2; i++) GRG_CUDA(c, must_alloc(c, &c->rbuf[i], cap * 32));
     c->rbuf_cap = cap;
     return GRG_OK;
 }
@@ -3482,9 +3512,9 @@ int alloc_dindex(grg_ctx *c)
 {
     const uint64_t nt = (uint64_t)c->L * c->V, vw = (uint64_t)c->L * ((c->V + 31) / 32);
     c->dvm_alloc = std::max<uint64_t>(vw, 1);
-    GRG_CUDA(c, cudaMalloc(&c->drs, std::max<uint64_t>(nt, 1) * 4));
-    GRG_CUDA(c, cudaMalloc(&c->drc, std::max<uint64_t>(nt, 1) * 4));
-    GRG_CUDA(c, cudaMalloc(&c->dvm, std::max<uint64_t>(vw, 1) * 4));
+    GRG_CUDA(c, must_alloc(c, &c->drs, std::max<uint64_t>(nt, 1) * 4));
+    GRG_CUDA(c, must_alloc(c, &c->drc, std::max<uint64_t>(nt, 1) * 4));
+    GRG_CUDA(c, must_alloc(c, &c->dvm, std::max<uint64_t>(vw, 1) * 4));
     GRG_CUDA(c, cudaMemsetAsync(c->drs, 0xFF, std::max<uint64_t>(nt, 1) * 4, c->stream));
     GRG_CUDA(c, cudaMemsetAsync(c->drc, 0, std::max<uint64_t>(nt, 1) * 4, c->stream));
     GRG_CUDA(c, cudaMemsetAsync(c->dvm, 0, std::max<uint64_t>(vw, 1) * 4, c->stream));
@@ -3540,6 +3570,8 @@ int grg_create(grg_ctx **out, int device)
     c->device_rounds = !(dr && dr[0] == '0');
     const char *rr = getenv("GRG_RETRY_ROOM");         // smallest retry list, in records
     if (rr && atoll(rr) > 0) c->retry_min = (uint64_t)atoll(rr);
+    const char *tr = getenv("GRG_TILE_ROOM");          // most records the tile lists may hold (0: no tile joins)
+    if (tr) c->tile_room = (uint64_t)atoll(tr);
     const char *jw = getenv("GRG_JOIN_WINDOW");        // "narrow" / "wide"; otherwise chosen per closure
     if (jw) c->join_window_mode = !strcmp(jw, "narrow") ? 0 : !strcmp(jw, "wide") ? 1 : 2;
     const char *ly = getenv("GRG_LAYOUT");             // "columns": labels the grammar allows by destination
@@ -3564,8 +3596,7 @@ void grg_destroy(grg_ctx *c)
     cudaFree(c->gslot);
     cudaFree(c->vbuf);
     cudaFree(c->sbuf);
-    cudaFree(c->lbuf);
-    cudaFree(c->tlist);
+    free_tiles(c);
     cudaFree(c->xbuf);
     cudaFree(c->xst);
     cudaFree(c->rowmark);
@@ -3724,10 +3755,10 @@ int setup_tables(grg_ctx *c, uint32_t num_vars)
     if (c->ntables_alloc < nt_all || c->batch ||
         c->dvm_alloc < (uint64_t)c->L * ((num_vars + 31) / 32)) {
         free_graph(c);
-        GRG_CUDA(c, cudaMalloc(&c->desc, std::max<uint64_t>(nt_all, 1) * 8));
-        GRG_CUDA(c, cudaMalloc(&c->cnt, std::max<uint64_t>(nt_all, 1) * 4));
-        GRG_CUDA(c, cudaMalloc(&c->want, std::max<uint64_t>(nt_all, 1) * 4));
-        GRG_CUDA(c, cudaMalloc(&c->grow, std::max<uint64_t>(nt_all, 1) * 4));
+        GRG_CUDA(c, must_alloc(c, &c->desc, std::max<uint64_t>(nt_all, 1) * 8));
+        GRG_CUDA(c, must_alloc(c, &c->cnt, std::max<uint64_t>(nt_all, 1) * 4));
+        GRG_CUDA(c, must_alloc(c, &c->want, std::max<uint64_t>(nt_all, 1) * 4));
+        GRG_CUDA(c, must_alloc(c, &c->grow, std::max<uint64_t>(nt_all, 1) * 4));
         c->ntables_alloc = nt_all;
         int st0 = alloc_dindex(c);
         if (st0) return st0;
@@ -3739,6 +3770,7 @@ int setup_tables(grg_ctx *c, uint32_t num_vars)
     GRG_CUDA(c, cudaMemsetAsync(c->ctr, 0, sizeof(unsigned long long) * NCTR, s));
     c->loaded = false;
     c->closed = false;
+    c->tiles_off = false;
     return GRG_OK;
 }
 
@@ -3902,8 +3934,8 @@ int grg_load_elements(grg_ctx *c, uint32_t num_vars, uint64_t num_elems, const u
             c->xbuf = nullptr; c->xst = nullptr;
             c->xcap = 0;
             const uint64_t cap = num_elems + num_elems / 4;
-            GRG_CUDA(c, cudaMalloc(&c->xbuf, cap * 32));
-            GRG_CUDA(c, cudaMalloc(&c->xst, cap * 4));
+            GRG_CUDA(c, must_alloc(c, &c->xbuf, cap * 32));
+            GRG_CUDA(c, must_alloc(c, &c->xst, cap * 4));
             c->xcap = cap;
         }
         GRG_CUDA(c, cudaMemcpyAsync(c->xbuf, elems, num_elems * 32, cudaMemcpyHostToDevice, s));
@@ -3918,7 +3950,7 @@ int grg_load_elements(grg_ctx *c, uint32_t num_vars, uint64_t num_elems, const u
         cudaFree(c->rowmark);
         c->rowmark = nullptr;
         c->rowmark_cap = 0;
-        GRG_CUDA(c, cudaMalloc(&c->rowmark, mwords * 4));
+        GRG_CUDA(c, must_alloc(c, &c->rowmark, mwords * 4));
         c->rowmark_cap = mwords;
     }
     auto hist = [&](Dev d) {
@@ -4028,7 +4060,9 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
 // Rounds go through k_tile where a rule's second symbol is derivable (old-left joins): their right
 // rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 70.9 ms).
 // With static second symbols a right row is 1-2 elements, too few to pay for a panel: k_rows or k_join.
-static bool use_tiles(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
+// They do while there was room for the tile lists (ensure_tiles); k_join needs none.
+static bool tiles_wanted(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
+static bool use_tiles(const grg_ctx *c) { return tiles_wanted(c) && c->lbuf_cap > 0; }
 
 // The tiles of a round's gathered and virtual records (counts on the device): list, then join.
 // sh: log2 of a tile's rows, 0 = from the device.
@@ -4516,35 +4550,35 @@ static int round_retries(grg_ctx *c, uint64_t nr, uint64_t nf, grg_stats &S, dou
 static int ensure_sbuf(grg_ctx *c)
 {
     if (c->sbuf) return GRG_OK;
-    GRG_CUDA(c, cudaMalloc(&c->sbuf, (size_t)SPLIT_MAX * SPLIT_PARTS * 32));
+    GRG_CUDA(c, must_alloc(c, &c->sbuf, (size_t)SPLIT_MAX * SPLIT_PARTS * 32));
     return GRG_OK;
 }
 
-// Buffers of k_tile: a tile starts at one record, and a record is left to k_join once at most.
-static int ensure_tiles(grg_ctx *c)
+// Lists of k_tile for rounds of n records: a tile starts at one record, and a record is left to k_join
+// once at most. 36 bytes a record on top of the records themselves: without room for them (or past
+// GRG_TILE_ROOM) the closure goes on without tiles.
+static void ensure_tiles(grg_ctx *c, uint64_t n)
 {
-    const uint64_t n = c->gbuf_cap + c->vbuf_cap;
-    if (!use_tiles(c) || n <= c->lbuf_cap) return GRG_OK;
-    cudaFree(c->lbuf);
-    cudaFree(c->tlist);
-    c->lbuf = nullptr;
-    c->tlist = nullptr;
-    c->lbuf_cap = 0;
-    GRG_CUDA(c, cudaMalloc(&c->lbuf, n * 32));
-    GRG_CUDA(c, cudaMalloc(&c->tlist, n * 4));
+    if (!tiles_wanted(c) || (c->lbuf_cap && n <= c->lbuf_cap)) return;
+    free_tiles(c);
+    if (n > c->tile_room || c->tiles_off) return;
+    if (cudaMalloc(&c->lbuf, n * 32) != cudaSuccess || cudaMalloc(&c->tlist, n * 4) != cudaSuccess) {
+        cudaGetLastError();
+        free_tiles(c);
+        return;
+    }
     c->lbuf_cap = n;
-    return GRG_OK;
 }
 
 // First join pass of a round over its nd gathered and nv virtual records, then retries.
 static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, double &join_ms, uint64_t &joins)
 {
     cudaStream_t s = c->stream;
-    const bool split = nd + nv < split_max(c);
     int st = ensure_rbuf(c, retry_room(c, nd + nv));
     if (st) return st;
+    if (nd + nv >= tile_min(c->rt.nol)) ensure_tiles(c, nd + nv + (nd + nv) / 2);
+    const bool split = nd + nv < split_max(c);
     if ((split || use_tiles(c)) && (st = ensure_sbuf(c))) return st;
-    if ((st = ensure_tiles(c))) return st;
     Dev d = make_dev(c);
     if (c->timing) GRG_CUDA(c, cudaEventRecord(c->ev_c, s));
     if (split) {
@@ -4823,7 +4857,7 @@ static int run_rounds(grg_ctx *c, uint64_t max_rounds, grg_stats &S, double &joi
         if ((st = ensure_cand(c, 2 * nd_last))) return st;    // a full candidate buffer falls back to direct inserts
         if ((st = ensure_rbuf(c, retry_room(c, c->gbuf_cap + (c->rt.nol ? c->vbuf_cap : 0))))) return st;
         if ((st = ensure_sbuf(c))) return st;
-        if ((st = ensure_tiles(c))) return st;
+        ensure_tiles(c, c->gbuf_cap + c->vbuf_cap);
         if ((st = build_round_graph(c, rs))) return st;
         c->cb = 0;
         // the delta index starts clear: inside the graph each round clears what the previous
@@ -4936,9 +4970,9 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
             cb.row = nullptr;
             cb.vcap = 0;
             const uint64_t vc = (uint64_t)c->V + 1 + c->V / 4;
-            GRG_CUDA(c, cudaMalloc(&cb.ptr, vc * 4));
-            GRG_CUDA(c, cudaMalloc(&cb.row, vc * 8));
-            GRG_CUDA(c, cudaMalloc(&cb.sums, ((vc + 1023) / 1024 + 1) * 4));
+            GRG_CUDA(c, must_alloc(c, &cb.ptr, vc * 4));
+            GRG_CUDA(c, must_alloc(c, &cb.row, vc * 8));
+            GRG_CUDA(c, must_alloc(c, &cb.sums, ((vc + 1023) / 1024 + 1) * 4));
             cb.vcap = vc;
         }
         uint32_t *ptr = cb.ptr, *sums = cb.sums;
@@ -4959,7 +4993,7 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
             cb.col = nullptr;
             cb.colcap = 0;
             const uint64_t cc = std::max<uint64_t>(total, 1) + total / 4;
-            GRG_CUDA(c, cudaMalloc(&cb.col, cc * 4));
+            GRG_CUDA(c, must_alloc(c, &cb.col, cc * 4));
             cb.colcap = cc;
         }
         k_csr_fill<<<grid_for(c, c->V, 256), 256, 0, s>>>(d, (uint32_t)l, ptr, row, cb.col);
@@ -5122,7 +5156,7 @@ int grg_get_degree(grg_ctx *c, uint32_t first_var, uint32_t last_var, uint32_t *
     if (int rs = rows_by_source(c)) return rs;
     const uint64_t n = (uint64_t)last_var - first_var + 1;
     uint32_t *dd = nullptr;
-    GRG_CUDA(c, cudaMalloc(&dd, n * 8));
+    GRG_CUDA(c, must_alloc(c, &dd, n * 8));
     GRG_CUDA(c, cudaMemsetAsync(dd, 0, n * 8, c->stream));
     int st = count_pass(c, dd, dd + n, first_var, last_var, 0);
     if (st) { cudaFree(dd); return st; }
@@ -5143,8 +5177,8 @@ int grg_export_edges(grg_ctx *c, uint64_t cap, uint32_t *src, uint32_t *dst, uin
     uint32_t *d32 = nullptr;
     uint8_t *d8 = nullptr;
     if (cap) {
-        GRG_CUDA(c, cudaMalloc(&d32, cap * 8));
-        GRG_CUDA(c, cudaMalloc(&d8, cap));
+        GRG_CUDA(c, must_alloc(c, &d32, cap * 8));
+        GRG_CUDA(c, must_alloc(c, &d8, cap));
     }
     GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_EXPORT, 0, 8, s));
     Dev d = make_dev(c);
@@ -5213,8 +5247,8 @@ static int stage_elements(grg_ctx *c, uint32_t v_begin, uint32_t v_end, uint64_t
         c->xbuf = nullptr; c->xst = nullptr;
         c->xcap = 0;
         const uint64_t xc = n + n / 4;
-        GRG_CUDA(c, cudaMalloc(&c->xbuf, xc * 32));
-        GRG_CUDA(c, cudaMalloc(&c->xst, xc * 4));
+        GRG_CUDA(c, must_alloc(c, &c->xbuf, xc * 32));
+        GRG_CUDA(c, must_alloc(c, &c->xst, xc * 4));
         c->xcap = xc;
     }
     GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_EXPORT, 0, 8, s));
@@ -5524,15 +5558,15 @@ int grg_batch_begin(grg_ctx *c, uint32_t max_vars, uint32_t max_jobs, int num_ru
     c->V = max_vars;
     c->ntables = (uint64_t)c->L * max_vars;
     const uint64_t nt_all = (uint64_t)c->L * max_vars;
-    GRG_CUDA(c, cudaMalloc(&c->desc, nt_all * 8));
-    GRG_CUDA(c, cudaMalloc(&c->cnt, nt_all * 4));
-    GRG_CUDA(c, cudaMalloc(&c->want, nt_all * 4));
-    GRG_CUDA(c, cudaMalloc(&c->grow, nt_all * 4));
+    GRG_CUDA(c, must_alloc(c, &c->desc, nt_all * 8));
+    GRG_CUDA(c, must_alloc(c, &c->cnt, nt_all * 4));
+    GRG_CUDA(c, must_alloc(c, &c->want, nt_all * 4));
+    GRG_CUDA(c, must_alloc(c, &c->grow, nt_all * 4));
     c->ntables_alloc = nt_all;
     st = alloc_dindex(c);
     if (st) return st;
-    GRG_CUDA(c, cudaMalloc(&c->row_job, (uint64_t)max_vars * 4));
-    GRG_CUDA(c, cudaMalloc(&c->job_cnt, (uint64_t)max_jobs * 4));
+    GRG_CUDA(c, must_alloc(c, &c->row_job, (uint64_t)max_vars * 4));
+    GRG_CUDA(c, must_alloc(c, &c->job_cnt, (uint64_t)max_jobs * 4));
     c->max_jobs = max_jobs;
     c->jobs.assign(max_jobs, grg_ctx::JobRange());
     GRG_CUDA(c, cudaMemsetAsync(c->desc, 0, nt_all * 8, s));

@@ -178,3 +178,25 @@ def test_partitions_keep_the_row_join(grg_mod, oracle_mod):
         p.close()
         assert (counts.tolist(), h) == (r.label_counts().tolist(), r.set_hash)
         assert ctx.last_joins()["rows"] == 1
+
+
+@pytest.mark.parametrize("device_rounds", [True, False])
+def test_closure_without_room_for_tile_lists(grg_mod, oracle_mod, monkeypatch, device_rounds):
+    """The tile lists are memory a closure can do without: where they cannot be had, at all or past a size,
+    the rounds run without tiles and the closure is the same."""
+    w = G.alias(seed=9_000, num_vars=9_000, num_base_edges=36_000, block=1000)
+    r = oracle_mod.closure(w.num_vars, w.rule_ids(), w.num_labels, 0, w.src, w.dst, w.lab)
+    want = (r.label_counts().tolist(), r.set_hash)
+    tiles = []
+    for room in (None, "0", "40000"):
+        if room is not None:
+            monkeypatch.setenv("GRG_TILE_ROOM", room)
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(device_rounds)
+            ctx.transfer_rules(w.rule_ids(), w.num_labels)
+            for _ in range(2):
+                ctx.load_edges(w.num_vars, w.src, w.dst, w.lab)
+                ctx.closure(0)
+                assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
+            tiles.append(ctx.last_joins()["tiles"])
+    assert tiles[0] > 0 and tiles[1] == 0 and tiles[2] < tiles[0]
