@@ -80,7 +80,9 @@ enum : int {
     C_TSUM = C_LABEL0 + MAX_SLOTS + 27,   // tiles joined over the closure
     C_LSUM = C_LABEL0 + MAX_SLOTS + 28,   // records they left to k_join over the closure
     C_JCNT = C_LABEL0 + MAX_SLOTS + 29,   // join launches of the device-driven rounds (grg_stats.join_launches)
-    NCTR = C_LABEL0 + MAX_SLOTS + 30
+    C_RNEAR = C_LABEL0 + MAX_SLOTS + 30,  // row joins, records in windows of their own: destinations these held,
+    C_RWIDE = C_LABEL0 + MAX_SLOTS + 31,  // and that one window over the run would have held (k_rows)
+    NCTR = C_LABEL0 + MAX_SLOTS + 32
 };
 // error bits of C_ERR; ERR_IN_* (in C_BADIN) flag input edges that were refused
 // (label outside 1..L, vertex id outside the graph) and never touched a table

@@ -2240,8 +2240,10 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
 // is its distance from the window's first id. The warp's ROWS_ELEMS window elements are split over
 // the batch's runs of a row's records: 8 windows of 12 elements (4 of 24 when they are few) for rows
 // within a procedure, and all 96 for a row whose records spread wider (an unconfined graph's row of
-// 52 elements, or one that reaches several blocks, sent most of its items to k_join's hash). What
-// even that leaves out becomes a candidate of one bit. Bound by integer issue (2.3 of 2-4 warp
+// 52 elements, or one that reaches several blocks, sent most of its items to k_join's hash). Records of
+// rows that reach across more than 96 get windows of their own where their destinations are local, the
+// row's one window where they are not (see `near`). What the windows leave out becomes a candidate of
+// one bit. Bound by integer issue (2.3 of 2-4 warp
 // instructions a clock, 13 a pair). Closures: 10k vertices unconfined 11.1 -> 7.8 ms, 97k in blocks
 // 6.2 -> 5.8 ms, 2M in blocks 53.5 -> 48.7 ms (at 8 blocks a SM 48.8, at 6 51.3, at 10 56.4).
 constexpr int ROWS_WARPS = 4;
@@ -2260,6 +2262,8 @@ struct __align__(16) RowsSmem {
     uint2 beyond[ROWS_QUEUE];                  // destinations outside the windows: id, record
     uint16_t list[ROWS_LIST];                  // record << 8 | position of its bit
     uint8_t first[8];                          // the first record of each window's run
+    unsigned long long near, wide;             // C_RNEAR and C_RWIDE of this warp's batches
+    uint32_t seen;                             // destinations of the batch
 };
 
 __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
@@ -2288,6 +2292,14 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
         }
         inserts = n_left = n_right = n_out = 0;
     };
+    // Runs that reach across more than the whole window: near their own intermediates the destinations of
+    // each record are dense where calls are local (50,000 vertices, 80% of the edges within 256 ids), and
+    // nowhere in a graph without locality. Windows a record are kept while they hold more of the
+    // destinations than a window over ROWS_ELEMS of the run's `reach` elements would. Closures with one
+    // window a run, with this rule, and k_join's: 30,000 local vertices 69.7, 56.4, 86.9 ms; 50,000
+    // 260, 147, 240; 100,000 1254, 647, 1048; 60,000 vertices without locality 126, 125, 168 ms.
+    bool near = d.ctr[C_RNEAR] >= d.ctr[C_RWIDE];
+    if (lane == 0) w.near = w.wide = 0;
     const uint32_t batch = batch_records(n, (uint64_t)gridDim.x * ROWS_WARPS);
     const uint64_t nbatch = (n + batch - 1) / batch;
     uint64_t bt = 0;
@@ -2304,9 +2316,9 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
         const uint32_t B = real ? lab : 0;
         // runs of records of one row and label (a table's records are contiguous)
         const uint32_t prow = __shfl_up_sync(0xffffffffu, row, 1), pB = __shfl_up_sync(0xffffffffu, B, 1);
-        const bool start = lane == 0 || !have || B == 0 || prow != row || pB != B;
+        bool start = lane == 0 || !have || B == 0 || prow != row || pB != B;
         const unsigned sm = __ballot_sync(0xffffffffu, start);
-        const uint32_t lead = 31 - __clz(sm & (0xFFFFFFFFu >> (31 - lane)));
+        uint32_t lead = 31 - __clz(sm & (0xFFFFFFFFu >> (31 - lane)));
         // the lowest and highest block of intermediates of each run
         const uint32_t nlead = sm & (0xFFFFFFFEu << lane) ? __ffs(sm & (0xFFFFFFFEu << lane)) - 1 : 32u;  // next run
         uint32_t lo = base, hi = base;
@@ -2322,7 +2334,19 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
         hi = __shfl_sync(0xffffffffu, hi, lead);
         // windows: a run's destinations are taken to lie as far around its intermediates as a group of
         // ROWS_NEAR elements that holds them all reaches; runs in more than that get the warp's
-        // whole window to themselves, in a pass of their own
+        // whole window to themselves, in a pass of their own, and records of a run that even the whole
+        // window does not reach across are runs of their own (near)
+        const bool far = real && hi - lo >= (uint32_t)ROWS_ELEMS;
+        const uint32_t reach = __reduce_max_sync(0xffffffffu, far ? hi - lo + 1 : 0u);
+        if (reach && near) {
+            if (lane == 0) w.seen = 0;
+            flush_counters();
+            if (far) {
+                start = true;
+                lead = lane;
+                lo = hi = base;
+            }
+        }
         const bool wide = hi - lo >= (uint32_t)ROWS_NEAR;
         const uint32_t narrow = __popc(__ballot_sync(0xffffffffu, start && real && !wide));
         bool ok = true;
@@ -2436,6 +2460,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
                                 if (lane >= (uint32_t)o) inc += y;
                             }
                             const uint32_t items = __shfl_sync(0xffffffffu, inc, 31), s1 = inc - deg;
+                            if (lane == 0) w.seen += items;
                             const unsigned some = __ballot_sync(0xffffffffu, deg != 0);
                             __syncwarp();
                             if (deg) w.rows[__popc(some & lt)] = make_uint4(rw.x - s1, tid0, tat0, r);
@@ -2492,6 +2517,15 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
                 __syncwarp();
             }
         }
+        if (reach && near) {
+            const uint32_t out = __reduce_add_sync(0xffffffffu, n_out);
+            if (lane == 0) {
+                w.near += (uint64_t)(w.seen - out) * reach;
+                w.wide += (uint64_t)w.seen * ROWS_ELEMS;
+            }
+            __syncwarp();
+            near = w.near >= w.wide;
+        }
         // a failed insert re-runs the records of its run (of the record, for a unary rule or a
         // destination outside the window)
         fail = __reduce_or_sync(0xffffffffu, fail);
@@ -2508,6 +2542,10 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
         __syncwarp();
     }
     flush_counters();
+    if (lane == 0 && w.wide) {
+        atomicAdd(&d.ctr[C_RNEAR], w.near);
+        atomicAdd(&d.ctr[C_RWIDE], w.wide);
+    }
 }
 
 // Tables of labels 1..L by log2 of their occupied elements (buckets 0..7, the

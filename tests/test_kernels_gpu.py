@@ -200,3 +200,31 @@ def test_closure_without_room_for_tile_lists(grg_mod, oracle_mod, monkeypatch, d
                 assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
             tiles.append(ctx.last_joins()["tiles"])
     assert tiles[0] > 0 and tiles[1] == 0 and tiles[2] < tiles[0]
+
+
+@pytest.mark.parametrize("local,device_rounds", [(True, True), (True, False), (False, True), (False, False)])
+def test_row_joins_of_rows_wider_than_the_window(grg_mod, local, device_rounds):
+    """Rows of more elements than the row join's whole window (96): records of local graphs keep their
+    destinations in windows of their own, others in one a row. Compared with the plain join: the same
+    closure, fewer destinations outside the windows."""
+    if local:
+        w = G.dataflow_small(seed=30, num_vars=30_000, num_edges=90_000)
+        V, src, dst, lab = w.num_vars, w.src, w.dst, w.lab
+    else:
+        w = G.dataflow_small(seed=30, num_vars=100, num_edges=300)
+        rng = np.random.default_rng(30)
+        V = 40_000
+        src, dst = rng.integers(0, V, (2, 60_000)).astype(np.uint32)
+        lab = np.full(len(src), w.labels.index("e") + 1, np.uint8)
+    got = []
+    for window, items in ((2, 2), (1, 0)):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(device_rounds)
+            ctx.set_join_window(window)
+            ctx.set_join_items(items)
+            ctx.transfer_rules(w.rule_ids(), w.num_labels)
+            ctx.load_edges(V, src, dst, lab)
+            st = ctx.closure(0)
+            got.append((ctx.label_counts().tolist(), ctx.set_hash(), st["window_out_elems"], ctx.last_joins()["rows"]))
+    assert got[0][:2] == got[1][:2] and (got[0][3], got[1][3]) == (1, 0)
+    assert 0 < got[0][2] < (0.3 if local else 0.7) * got[1][2]
