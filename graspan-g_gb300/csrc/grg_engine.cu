@@ -1262,7 +1262,13 @@ constexpr int TILE_Q = TILE_W * EW / 4;
 constexpr int TILE_G = EIDS / 4;               // groups of 4 intermediates
 constexpr int TILE_RECS = 2048;                // records a tile holds at once (more are taken in turns)
 constexpr int TILE_KB = 32;                    // distinct blocks of intermediates at once
-constexpr int TILE_WINDOWS = 8;
+// Windows of a tile: this many, and on while the last one held TILE_RICH quads of 16 bytes a panel (half an
+// element a row). A panel costs some 7,000 clocks an SM in every window; what the windows leave out sends the
+// tile's records to k_join whole, which takes about 14 clocks an SM for a pair and element: 96 elements
+// that 1,024 pairs over 192 rows join cost it the same. Unconfined alias rows of 105 elements
+// (20,000 vertices, dense): see the test of many windows.
+constexpr uint32_t TILE_WINDOWS = 8;
+constexpr uint32_t TILE_RICH = 144;
 // Pairs (record, k) of a tile that pay for reading a panel; records of blocks with fewer go to k_join,
 // whose warps share them out over the chip. A panel holds an SM for some 7,000 clocks whatever it joins,
 // k_join takes a pair at a time: 4 pairs a row of the tile. Closures (ms) with 128 pairs at every size,
@@ -1290,8 +1296,11 @@ struct TileSmem {
     uint32_t rowoff[TILE_ROWS];                // first pool slot of A[i]
     uint32_t rowhas[TILE_ROWS / 32], rowfail[TILE_ROWS / 32];
     uint32_t rowchg[TILE_ROWS];                // accumulator quads that changed
-    uint32_t wins[TILE_WINDOWS];
     uint32_t next_w, end, tile, kmin;
+    uint32_t took, need;                       // quads of right-hand rows in the window (counted from the
+                                               // 7th on), and as many as another window asks for
+    uint32_t last;                             // the window is the last
+    uint32_t n_left, inserts;                  // counted by the block (a register each spills: 1M alias +4%)
     uint32_t heavy;                            // entries of kb with enough pairs
     uint16_t ord[TILE_RECS];
     __align__(8) uint16_t look[TILE_WARPS][TILE_G + 8];   // a record's lookups: subset entries of tab
@@ -1352,6 +1361,7 @@ __device__ __forceinline__ uint4 tab_at(const unsigned char *tb, uint32_t i)
 {
     return *reinterpret_cast<const uint4 *>(tb + i * (TILE_Q * 16));
 }
+__device__ __forceinline__ bool any4(const uint4 a) { return (a.x | a.y | a.z | a.w) != 0; }
 // b has no bit that a lacks
 __device__ __forceinline__ bool covers4(const uint4 a, const uint4 b)
 {
@@ -1367,13 +1377,13 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
     if (d.ctr[C_HALT]) return;
     if (!sh) sh = (uint32_t)d.ctr[C_TS];
     if (!sh) return;
-    const uint64_t ntiles = min((uint64_t)d.ctr[C_TN], list_cap);
+    const uint32_t ntiles = (uint32_t)min((uint64_t)d.ctr[C_TN], list_cap);
     if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr[C_TSUM] += ntiles;
-    const uint64_t nd = d.ctr[C_DIRTY_N], nv = d.ctr[C_VN];
     const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, rows = 1u << sh;
     // in the joins, lanes 0-11 and 16-27 hold a row's 12 quads of 16 bytes (12-15 and 28-31 repeat the last)
     const uint32_t half = lane >> 4, q = min(lane & 15, (uint32_t)TILE_Q - 1);
-    uint32_t n_left = 0, n_right = 0, inserts = 0;
+    uint32_t n_right = 0;
+    if (tid == 0) w.n_left = w.inserts = 0;
     for (uint32_t i = tid; i < TILE_G * TILE_Q; i += TILE_THREADS)      // the empty subsets
         w.tab[i / TILE_Q][0][i % TILE_Q] = make_uint4(0, 0, 0, 0);
 
@@ -1385,9 +1395,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
         const uint32_t at = list[w.tile];
         const bool virt = at >> 31;
         const uint4 *recs = virt ? vrecs : grecs;
-        const uint64_t nrec = virt ? nv : nd;
-        uint64_t pos = at & 0x7FFFFFFFu;
-        const uint2 head = reinterpret_cast<const uint2 *>(recs)[4 * pos + 3];
+        const uint32_t nrec = (uint32_t)d.ctr[virt ? C_VN : C_DIRTY_N];
+        uint32_t pos = at & 0x7FFFFFFFu;
+        const uint2 head = reinterpret_cast<const uint2 *>(recs)[4 * (size_t)pos + 3];
         const uint32_t lab = head.x >> KEY_SHIFT, row0 = (head.y >> sh) << sh;
         const bool real = !virt && lab >= 1 && lab <= (uint32_t)d.rt.L;
         const uint32_t qv = lab - OL_SLOT0;
@@ -1413,7 +1423,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                 nbits[u] = 0;
                 if (pos + i < nrec) {
                     uint4 a, b;
-                    ld32(recs + 2 * (pos + i), a, b);
+                    ld32(recs + 2 * (size_t)(pos + i), a, b);
                     if ((b.z >> KEY_SHIFT) == lab && (b.w >> sh) == (row0 >> sh)) {
                         mine = true;
                         nbits[u] = popc6(Bits{{a.x, a.y, a.z, a.w, b.x, b.y}});
@@ -1490,14 +1500,14 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                 // unary rules A ::= B (records left to k_join take theirs there)
                 if (real && (take || !nrules) && d.rt.un_start[lab + 1] > d.rt.un_start[lab]) {
                     uint4 r0, r1;
-                    ld32(recs + 2 * (pos + i), r0, r1);
+                    ld32(recs + 2 * (size_t)(pos + i), r0, r1);
                     const uint32_t kb = r1.z & BASE_MASK;
                     bool ok = true;
                     const Bits b = {{r0.x, r0.y, r0.z, r0.w, r1.x, r1.y}};
                     for (int u = d.rt.un_start[lab]; u < d.rt.un_start[lab + 1]; u++) {
                         const uint32_t A = d.rt.un_A[u];
                         ok &= g_insert(d, A, row0 + row, kb, b, d.rt.track[A]);
-                        inserts++;
+                        atomicAdd(&w.inserts, 1u);
                     }
                     if (!ok) atomicOr(&w.rowfail[row >> 5], 1u << (row & 31));
                 }
@@ -1509,12 +1519,12 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                 const uint32_t A = virt ? d.rt.ol_A[rq] : d.rt.bin_A[rq], C = virt ? d.rt.ol_C[rq] : d.rt.bin_C[rq];
                 const bool prefA = (d.prefix_mask >> (A - 1)) & 1ull, prefC = (d.prefix_mask >> (C - 1)) & 1ull;
                 uint32_t win = w.kmin, todo = w.heavy;       // the window, the blocks to join in it
-                for (int nw = 0; nw < TILE_WINDOWS; nw++) {
-                    const bool last = nw == TILE_WINDOWS - 1;
+                for (uint32_t nw = 0;; nw++) {
                     if (tid == 0) {
-                        w.wins[nw] = win;
+                        w.last = nw >= TILE_WINDOWS - 1 && w.took < w.need;
+                        w.need = TILE_RICH * __popc(todo);
                         w.next_w = EMPTY;
-                        w.kmore = 0;
+                        w.kmore = w.took = 0;
                     }
                     // ---- the rows A[i]: 8 lanes a row, the loads of a thread's rows in flight together
                     {
@@ -1571,7 +1581,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                         auto fetch = [&](uint32_t m) {
                             const uint32_t j = wid + TILE_WARPS * (m + (lane >> 3));
                             return j < cnt ? __ldg(reinterpret_cast<const uint32_t *>(recs) +
-                                                   8 * (pos + w.ord[first + j]) + (lane & 7))
+                                                   8 * (size_t)(pos + w.ord[first + j]) + (lane & 7))
                                            : 0u;
                         };
                         uint32_t v = fetch(0);
@@ -1579,6 +1589,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                         const uint64_t k0 = (uint64_t)w.kb[e] * EIDS;
                         if (tid < TILE_W * EW) w.U[tid] = 0;
                         if (tid < EW) w.outk[tid] = 0;
+                        if (tid == 0 && nw == 0) w.n_left += cnt;
                         __syncthreads();
                         {
                             constexpr int NR = (EIDS + TILE_THREADS / 8 - 1) / (TILE_THREADS / 8);
@@ -1629,12 +1640,12 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                                         p[2] = make_uint2(e1[u].x, e1[u].y);
                                         continue;
                                     }
-                                    bool done = false;                 // an earlier window held it
-                                    for (int x = 0; x < nw; x++) done |= b - w.wins[x] < (uint32_t)TILE_W;
-                                    if (done) continue;
+                                    // an earlier window held it: the first, or one of those after it, which
+                                    // go up from the lowest base that the first left out
+                                    if (nw && (b < win || b - w.kmin < (uint32_t)TILE_W)) continue;
                                     atomicOr(&w.kmore, 1u << e);
                                     atomicMin(&w.next_w, b);
-                                    if (last) atomicOr(&w.outk[r >> 5], 1u << (r & 31));
+                                    if (w.last) atomicOr(&w.outk[r >> 5], 1u << (r & 31));
                                 }
                             }
                         }
@@ -1645,6 +1656,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                             const uint32_t c = tid % TILE_Q;
                             const uint4 r0 = g[1][c], r1 = g[2][c], r2 = g[4][c], r3 = g[8][c];
                             const uint4 a = or4(r0, r1), b = or4(r2, r3), all = or4(a, b);
+                            if (nw >= TILE_WINDOWS - 2)
+                                atomicAdd(&w.took, (uint32_t)any4(r0) + any4(r1) + any4(r2) + any4(r3));
                             g[3][c] = a;
                             g[5][c] = or4(r0, r2);
                             g[6][c] = or4(r1, r2);
@@ -1674,8 +1687,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                             for (uint32_t m = 0; m < 4 && wid + TILE_WARPS * (m0 + m) < cnt; m++) {
                                 const uint32_t row = __shfl_sync(0xffffffffu, v, m * 8 + 7) - row0;
                                 const uint4 a0 = w.acc[row][q];
-                                n_left += lane == 0 && nw == 0;
-                                if (last) {
+                                if (w.last) {
                                     const unsigned o = __ballot_sync(0xffffffffu, lane >> 3 == m && (lane & 7) < EW &&
                                                                                       (v & w.outk[min(lane & 7, EW - 1u)]));
                                     if (o && lane == 0) w.rmeta[w.ord[first + wid + TILE_WARPS * (m0 + m)]] |= TM_LEFT;
@@ -1738,7 +1750,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                             } else {
                                 // an element seen when the row was read is ORed where it is
                                 const uint32_t s = w.slot[row][e];
-                                inserts++;
+                                atomicAdd(&w.inserts, 1u);
                                 if (s != 0xFFu)
                                     g_or_into(d, w.rowoff[row] + s, b, d.rt.track[A]);
                                 else if (!g_insert(d, A, row0 + row, win + e, b, d.rt.track[A]))
@@ -1749,6 +1761,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                     __syncthreads();
                     win = w.next_w;
                     todo = w.kmore;
+                    if (w.last) win = EMPTY;
                     __syncthreads();
                     if (win == EMPTY) break;
                 }
@@ -1759,7 +1772,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                 const bool left = m & TM_LEFT, failed = (w.rowfail[row >> 5] >> (row & 31)) & 1u;
                 if (!left && !failed) continue;
                 uint4 r0, r1;
-                ld32(recs + 2 * (pos + i), r0, r1);
+                ld32(recs + 2 * (size_t)(pos + i), r0, r1);
                 if (left) list_push(&d.ctr[C_LN], left_cap, left_out, r0, r1);
                 else list_push(&d.ctr[C_RETRY_N], d.retry_cap, retry_out, r0, r1);
             }
@@ -1767,15 +1780,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
             __syncthreads();
         }
     }
-    for (int o = 16; o; o >>= 1) {
-        n_left += __shfl_xor_sync(0xffffffffu, n_left, o);
-        n_right += __shfl_xor_sync(0xffffffffu, n_right, o);
-        inserts += __shfl_xor_sync(0xffffffffu, inserts, o);
-    }
-    if (lane == 0) {
-        if (n_left) atomicAdd(&d.ctr[C_LEFT], (unsigned long long)n_left);
-        if (n_right) atomicAdd(&d.ctr[C_RIGHT], (unsigned long long)n_right);
-        if (inserts) atomicAdd(&d.ctr[C_INSERTS], (unsigned long long)inserts);
+    for (int o = 16; o; o >>= 1) n_right += __shfl_xor_sync(0xffffffffu, n_right, o);
+    if (lane == 0 && n_right) atomicAdd(&d.ctr[C_RIGHT], (unsigned long long)n_right);
+    if (tid == 0) {
+        if (w.n_left) atomicAdd(&d.ctr[C_LEFT], (unsigned long long)w.n_left);
+        if (w.inserts) atomicAdd(&d.ctr[C_INSERTS], (unsigned long long)w.inserts);
     }
 }
 

@@ -228,3 +228,66 @@ def test_row_joins_of_rows_wider_than_the_window(grg_mod, local, device_rounds):
             got.append((ctx.label_counts().tolist(), ctx.set_hash(), st["window_out_elems"], ctx.last_joins()["rows"]))
     assert got[0][:2] == got[1][:2] and (got[0][3], got[1][3]) == (1, 0)
     assert 0 < got[0][2] < (0.3 if local else 0.7) * got[1][2]
+
+
+def _wide(nv, rows, kblocks, bits, deg, seed=0):
+    """A ::= B C over rows 0..rows-1 of B with `bits` intermediates in each of the first `kblocks` blocks of
+    192 ids, and `deg` destinations of C for each of these (-deg: in the first 8 blocks); B and C are derived,
+    so C is joined old-left too."""
+    span, deg = (nv if deg > 0 else 8 * 192), abs(deg)
+    rng = np.random.default_rng(seed + nv + kblocks + deg)
+    k = np.concatenate([b * 192 + np.argsort(rng.random((rows, 192)), axis=1)[:, :bits] for b in range(kblocks)], axis=1)
+    bsrc, bdst = np.repeat(np.arange(rows), kblocks * bits), k.ravel()
+    esrc, edst = np.repeat(np.arange(kblocks * 192), deg), rng.integers(0, span, kblocks * 192 * deg)
+    src, dst = np.concatenate([bsrc, esrc]).astype(np.uint32), np.concatenate([bdst, edst]).astype(np.uint32)
+    lab = np.repeat(np.array([4, 5], np.uint8), [len(bsrc), len(esrc)])
+    return nv, np.array([[2, 4, 0], [3, 5, 0], [1, 2, 3]], np.int32), 5, 0, src, dst, lab
+
+
+@pytest.mark.parametrize("nv,rows,kblocks,bits,deg,left", [
+    (20_000, 4000, 4, 50, 2000, "none"),     # right rows of 105 elements, dense: 14 windows
+    (20_000, 4000, 4, 50, 150, "none"),      # the same, 79 of 105 elements in a row
+    (200_000, 4000, 4, 50, 3, "all"),        # 3 elements a right row, anywhere in 1,042: given up after 8 windows
+    (20_000, 3000, 40, 30, 5, "some"),       # more blocks of intermediates than a tile's table holds (32)
+    (20_000, 3000, 50, 30, 4, "whole"),      # more leftovers than are cut: joined as they are
+    (20_000, 4000, 100, 60, 4, "whole"),
+    (20_000, 3000, 50, 30, -4, "whole"),     # (destinations in 8 blocks)
+    (20_000, 1200, 36, 30, -4, "split"),     # leftovers cut by bitmap word (32,768 to 131,072 of them)
+    (20_000, 300, 36, 30, -4, "parts"),      # fewer: cut into parts of 8 bits
+])
+def test_tiles_of_wide_rows(grg_mod, oracle_mod, nv, rows, kblocks, bits, deg, left):
+    """Tiles at their limits: windows, blocks of intermediates, and the sizes of the list they leave (rows of
+    more than 12 elements outgrow their tables, which then lie in any order: their own records make no tiles)."""
+    w = _wide(nv, rows, kblocks, bits, deg)
+    r = oracle_mod.closure(*w)
+    want = (r.label_counts().tolist(), r.set_hash)
+    for dev in (True, False):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(dev)
+            ctx.transfer_rules(w[1], w[2])
+            ctx.load_edges(w[0], *w[4:])
+            ctx.closure(0)
+            assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
+            j = ctx.last_joins()
+        assert j["tiles"] > 0
+        lo, hi = {"none": (0, 0), "all": (8 * rows, None), "some": (1, None), "parts": (1, 32_767),
+                  "split": (32_768, 131_071), "whole": (131_072, None)}[left]
+        assert lo <= j["tile_left"] and (hi is None or j["tile_left"] <= hi)
+
+
+@pytest.mark.parametrize("room", [None, "16"])
+def test_tile_rows_that_outgrow_their_tables(grg_mod, oracle_mod, monkeypatch, room):
+    """Rows of tiles whose inserts fail are joined again after their tables grow, or (more failures than the
+    retry list holds) the whole round is."""
+    if room:
+        monkeypatch.setenv("GRG_RETRY_ROOM", room)
+    w = _wide(20_000, 4000, 4, 50, 150)
+    r = oracle_mod.closure(*w)
+    for dev in (True, False):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(dev)
+            ctx.transfer_rules(w[1], w[2])
+            ctx.load_edges(w[0], *w[4:])
+            st = ctx.closure(0)
+            assert (ctx.label_counts().tolist(), ctx.set_hash()) == (r.label_counts().tolist(), r.set_hash)
+            assert ctx.last_joins()["tiles"] > 0 and st["retry_records"] > 0 and st["grow_rows"] >= 4000
