@@ -76,7 +76,7 @@ enum : int {
     C_TN = C_LABEL0 + MAX_SLOTS + 23,     // tiles of the round (k_tile_starts); zeroed with the next two
     C_TQ = C_LABEL0 + MAX_SLOTS + 24,     // work queue of k_tile: next tile
     C_LN = C_LABEL0 + MAX_SLOTS + 25,     // records k_tile left to k_join
-    C_TS = C_LABEL0 + MAX_SLOTS + 26,     // log2 of the rows of a tile in a device-driven round (0 = not tiled)
+    C_TS = C_LABEL0 + MAX_SLOTS + 26,     // log2 of the rows of a tile this round (0 = cut into parts, TILE_NONE = no tiles)
     C_TSUM = C_LABEL0 + MAX_SLOTS + 27,   // tiles joined over the closure
     C_LSUM = C_LABEL0 + MAX_SLOTS + 28,   // records they left to k_join over the closure
     C_JCNT = C_LABEL0 + MAX_SLOTS + 29,   // join launches of the device-driven rounds (grg_stats.join_launches)

@@ -1285,6 +1285,16 @@ __host__ __device__ inline uint32_t tile_rows_lg(uint64_t n)
     return lg;
 }
 
+// A round whose joined records hold fewer than TILE_MEAN intermediates in the mean goes without tiles (C_TS =
+// TILE_NONE): its panels would have few pairs each, and short right-hand rows besides. Closures (ms) without
+// this line, with it at 16, 24, 32 and 40, and with k_join alone: chains of 20 ids 2.6, 1.8, 1.8, 1.8, 1.8, 1.9;
+// of 100 3.7, 3.1, 2.5, 2.3, 2.3, 2.6; of 250 3.8, 3.1, 2.8, 2.7, 2.5, 3.2; 100k alias of 1 edge a vertex 3.5,
+// 2.2, 2.2, 2.2, 2.2, 3.3; alias in blocks of 100 4.0, 3.1, 2.8, 1.9, 1.9, 3.2; of 200 11.9, 11.4, 10.9, 10.4,
+// 9.7, 11.1; of 1,000, 120k vertices 11.8, 11.2, 11.4, 11.5, 12.4; 1M 69.4, 68.8, 68.6, 68.6, 68.8, 189.
+constexpr uint32_t TILE_MEAN = 32;
+constexpr uint32_t TILE_NONE = 0xFF;
+constexpr uint32_t TILE_SAMPLE = 256;          // records that the mean is taken of: a thread each
+
 struct TileSmem {
     uint4 tab[TILE_G][16][TILE_Q];             // per 4 rows C[k]: the unions of their 16 subsets
     uint4 acc[TILE_ROWS][TILE_Q];              // rows A[i]
@@ -1311,14 +1321,12 @@ constexpr uint32_t TM_LEFT = 1u << 16;         // the record goes to k_join
 
 // Tiles of the round's records: a tile starts where the label or the row block (row >> C_TS)
 // differs from the record before it. Starts are listed in any order (bit 31: virtual records).
-// sh: log2 of the rows of a tile; 0 = take it from the counters (device-driven rounds), where 0
-// means a round that is joined as sub-records.
 __global__ void k_tile_starts(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint32_t *list,
-                              uint64_t list_cap, uint32_t sh)
+                              uint64_t list_cap)
 {
     if (d.ctr[C_HALT]) return;
-    if (!sh) sh = (uint32_t)d.ctr[C_TS];
-    if (!sh) return;
+    const uint32_t sh = (uint32_t)d.ctr[C_TS];
+    if (!sh || sh == TILE_NONE) return;
     const uint64_t nd = d.ctr[C_DIRTY_N], n = nd + d.ctr[C_VN];
     for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); i0 < n;
          i0 += (uint64_t)gridDim.x * blockDim.x) {
@@ -1370,13 +1378,13 @@ __device__ __forceinline__ bool covers4(const uint4 a, const uint4 b)
 
 __global__ void __launch_bounds__(TILE_THREADS, 1)
     k_tile(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, const uint32_t *__restrict__ list,
-           uint64_t list_cap, uint4 *left_out, uint64_t left_cap, uint4 *retry_out, uint32_t sh)
+           uint64_t list_cap, uint4 *left_out, uint64_t left_cap, uint4 *retry_out)
 {
     extern __shared__ __align__(16) unsigned char tile_smem_raw[];
     TileSmem &w = *reinterpret_cast<TileSmem *>(tile_smem_raw);
     if (d.ctr[C_HALT]) return;
-    if (!sh) sh = (uint32_t)d.ctr[C_TS];
-    if (!sh) return;
+    const uint32_t sh = (uint32_t)d.ctr[C_TS];
+    if (!sh || sh == TILE_NONE) return;
     const uint32_t ntiles = (uint32_t)min((uint64_t)d.ctr[C_TN], list_cap);
     if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr[C_TSUM] += ntiles;
     const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, rows = 1u << sh;
@@ -1395,7 +1403,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
         const uint32_t at = list[w.tile];
         const bool virt = at >> 31;
         const uint4 *recs = virt ? vrecs : grecs;
-        const uint32_t nrec = (uint32_t)d.ctr[virt ? C_VN : C_DIRTY_N];
+        const uint32_t nrec = (uint32_t)d.ctr[virt ? C_VN : C_DIRTY_N];   // (below 2^31 in a round with tiles)
         uint32_t pos = at & 0x7FFFFFFFu;
         const uint2 head = reinterpret_cast<const uint2 *>(recs)[4 * (size_t)pos + 3];
         const uint32_t lab = head.x >> KEY_SHIFT, row0 = (head.y >> sh) << sh;
@@ -1821,26 +1829,60 @@ __host__ __device__ inline uint32_t join_launches(bool split, bool tiles, uint64
 }
 constexpr uint64_t SPLIT_LEFT_MAX = (uint64_t)SPLIT_MAX * SPLIT_PARTS / EW;
 
-// tile: 1: the rounds that are not split go through k_tile (C_TS: its rows), not k_join; SPLIT_LEFT: the
-// records are those that k_tile left (C_LN of grecs), and those not split are joined as they are (C_JN1).
+// tile: 1: the rounds that are not split go through k_tile (C_TS: its rows), not k_join; SPLIT_LEFT: after
+// k_tile, the records are those that it left (C_LN of left), and those not split are joined as they are
+// (C_JN1); of a round without tiles (TILE_NONE) they are the round's own, cut below none_max records and
+// copied to left above. In the static scratch such rounds are never cut (none_max = 0; 3,000-vertex alias
+// closure 3.7 ms, cut 4.3), and half the mean is enough for tiles.
 // A thread cuts one bitmap word of a record (up to 4 parts), and a warp reserves its parts' room
 // at once, in record order: a thread a record took 14 us for the 192 bits of a dense one.
-// passes (round graphs, else 0): join kernels of a pass, for the count of their launches (C_JCNT).
-__global__ void k_split(Dev d, const uint4 *__restrict__ grecs, const uint4 *__restrict__ vrecs, uint4 *out, int tile,
-                        uint64_t split_max, uint32_t passes)
+// passes: join kernels of a pass, for the count of their launches (C_JCNT); 0: the host counts.
+__global__ void __launch_bounds__(TILE_SAMPLE) k_split(Dev d, const uint4 *__restrict__ grecs,
+                                                       const uint4 *__restrict__ vrecs, uint4 *__restrict__ left_recs,
+                                                       uint4 *out, int tile, uint64_t split_max, uint64_t none_max,
+                                                       uint32_t passes)
 {
     if (d.ctr[C_HALT]) return;
-    const bool left = tile == SPLIT_LEFT;
-    const uint64_t nd = d.ctr[left ? C_LN : C_DIRTY_N], nv = left ? 0 : d.ctr[C_VN];
-    const bool split = nd + nv < split_max;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        d.ctr[C_JN1] = split || tile == 1 ? 0 : nd;
-        d.ctr[C_JN2] = split || tile ? 0 : nv;
-        if (!left) d.ctr[C_TS] = split || !tile ? 0 : tile_rows_lg(nd + nv);
-        if (left) d.ctr[C_LSUM] += nd;
-        if (passes) d.ctr[C_JCNT] += join_launches(split, tile != 0, nv, passes);
+    const bool left = tile == SPLIT_LEFT, none = left && d.ctr[C_TS] == TILE_NONE;
+    const uint64_t nd = d.ctr[left && !none ? C_LN : C_DIRTY_N], nv = left && !none ? 0 : d.ctr[C_VN];
+    const bool split = nd + nv < (none ? none_max : split_max);
+    if (blockIdx.x == 0) {
+        __shared__ uint32_t recs_s, bits_s;
+        if (threadIdx.x == 0) recs_s = bits_s = 0;
+        __syncthreads();
+        if (tile == 1 && !split) {               // uniform: the mean of the round's records that join
+            const uint64_t i = threadIdx.x * (nd + nv) / TILE_SAMPLE;
+            uint4 a = make_uint4(0, 0, 0, 0), b = make_uint4(0, 0, EMPTY, 0);
+            if (i < nd + nv) ld32(i < nd ? grecs + 2 * i : vrecs + 2 * (i - nd), a, b);
+            const uint32_t lab = b.z >> KEY_SHIFT;
+            const bool joins = i < nd + nv && (i >= nd || (lab >= 1 && lab <= (uint32_t)d.rt.L &&
+                                                           d.rt.bin_start[lab + 1] > d.rt.bin_start[lab]));
+            const uint32_t n = __popc(__ballot_sync(0xffffffffu, joins));
+            const uint32_t p = __reduce_add_sync(0xffffffffu, joins ? popc6(Bits{{a.x, a.y, a.z, a.w, b.x, b.y}}) : 0u);
+            if (lane_id() == 0) {
+                atomicAdd(&recs_s, n);
+                atomicAdd(&bits_s, p);
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            // (31 bits in the tile list)
+            const uint32_t mean = nd + nv < none_max ? TILE_MEAN : TILE_MEAN / 2;
+            const bool sparse = !bits_s || bits_s < mean * recs_s || (nd | nv) >> 31;
+            const uint32_t ts = split || tile != 1 ? 0 : sparse ? TILE_NONE : tile_rows_lg(nd + nv);
+            d.ctr[C_JN1] = split || tile == 1 ? 0 : none ? nd + nv : nd;
+            d.ctr[C_JN2] = split || tile ? 0 : nv;
+            if (!left) d.ctr[C_TS] = ts;
+            if (left && !none) d.ctr[C_LSUM] += nd;
+            if (passes) d.ctr[C_JCNT] += ts == TILE_NONE ? 1u : join_launches(split, ts != 0, nv, passes);
+        }
     }
+    if (none && !split)
+        for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 2 * (nd + nv);
+             i += (uint64_t)gridDim.x * blockDim.x)
+            left_recs[i] = i < 2 * nd ? grecs[i] : vrecs[i - 2 * nd];
     if (!split) return;
+    if (left && !none) grecs = left_recs;
     // bits of a part: 8, or a word's when more records are left than the buffer holds 24 parts of
     const uint32_t part_bits = left && nd >= SPLIT_MAX ? 32u : SPLIT_BITS;
     const uint64_t total = (nd + nv) * EW, stride = (uint64_t)gridDim.x * blockDim.x;
@@ -4111,15 +4153,14 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
 static bool tiles_wanted(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
 static bool use_tiles(const grg_ctx *c) { return tiles_wanted(c) && c->lbuf_cap > 0; }
 
-// The tiles of a round's gathered and virtual records (counts on the device): list, then join.
-// sh: log2 of a tile's rows, 0 = from the device.
+// The tiles of a round's gathered and virtual records, list, then join: counts and rows (C_TS) from the device.
 static void launch_tiles(int sms, cudaStream_t s, const Dev &d, const uint4 *grecs, const uint4 *vrecs, uint32_t *list,
-                         uint4 *left, uint64_t cap, uint4 *retry_out, uint32_t sh)
+                         uint4 *left, uint64_t cap, uint4 *retry_out)
 {
     cudaMemsetAsync(d.ctr + C_TN, 0, 24, s);                    // tiles, tile queue, records left to k_join
     cudaFuncSetAttribute(k_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
-    k_tile_starts<<<sms * 8, 256, 0, s>>>(d, grecs, vrecs, list, cap, sh);
-    k_tile<<<sms, TILE_THREADS, sizeof(TileSmem), s>>>(d, grecs, vrecs, list, cap, left, cap, retry_out, sh);
+    k_tile_starts<<<sms * 8, 256, 0, s>>>(d, grecs, vrecs, list, cap);
+    k_tile<<<sms, TILE_THREADS, sizeof(TileSmem), s>>>(d, grecs, vrecs, list, cap, left, cap, retry_out);
 }
 
 static bool any_csr(const grg_ctx *c)
@@ -4512,13 +4553,14 @@ static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv,
         return;
     }
     if (use_tiles(c)) {
-        launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], tile_rows_lg(nd + nv));
+        k_split<<<1, TILE_SAMPLE, 0, s>>>(d, c->gbuf, c->vbuf, nullptr, nullptr, 1, 0, ~0ull, pass_kernels(c));
+        launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]);
         cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s);
-        k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX, 0);
+        k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->lbuf, c->sbuf, SPLIT_LEFT,
+                                                                SPLIT_LEFT_MAX, SPLIT_MAX, 0);
         launch_join(c, grid_for(c, (nd + nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
         launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0]);
-        c->launches += 5;
-        joins += join_launches(false, true, nv, pass_kernels(c));
+        c->launches += 6;
         return;
     }
     launch_pass(c, grid_for(c, (nd + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
@@ -4631,7 +4673,7 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
     if (split) {
         // few records: their parts spread the join over more warps
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_SPLIT_N, 0, 8, s));
-        k_split<<<grid_for(c, (nd + nv) * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, 0, split_max(c), 0);
+        k_split<<<grid_for(c, (nd + nv) * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, nullptr, c->sbuf, 0, split_max(c), 0, 0);
         c->launches++;
     }
     if (c->tune_pending && c->need_join && !split && nd >= TUNE_MIN_RECORDS) {
@@ -4818,15 +4860,16 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
     }
     const int jgrid = grid_for(c, ~0u, JOIN_WARPS, 16);
     const bool tiles = use_tiles(c);
-    k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->sbuf, tiles, split_max(c),
+    k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, nullptr, c->sbuf, tiles, split_max(c), ~0ull,
                                                             pass_kernels(c));
     nk++;
     {
         const uint64_t launches0 = c->launches;
         uint64_t unused = 0;
         if (tiles) {
-            launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0], 0);
-            k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->lbuf, nullptr, c->sbuf, SPLIT_LEFT, SPLIT_LEFT_MAX, 0);
+            launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]);
+            k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->lbuf, c->sbuf, SPLIT_LEFT,
+                                                                    SPLIT_LEFT_MAX, SPLIT_MAX, 0);
             launch_join(c, jgrid, s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
             nk += 4;
         } else {
@@ -4925,8 +4968,6 @@ static int run_rounds(grg_ctx *c, uint64_t max_rounds, grg_stats &S, double &joi
         const unsigned long long halt = c->h_ctr[C_HALT], rounds = c->h_ctr[C_GROUNDS];
         S.rounds += rounds;
         S.delta_elems += c->h_ctr[C_GDSUM];
-        joins += c->h_ctr[C_JCNT];
-        GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_JCNT, 0, 8, s));
         c->launches += c->h_ctr[C_ITERS] * c->rg_kernels;
         join_ms += c->h_ctr[C_JNS] * 1e-6;
         done_rounds += rounds;
@@ -5077,7 +5118,7 @@ int grg_closure_ex(grg_ctx *c, uint32_t filter, uint32_t run_stamp, grg_stats *s
     cudaEventElapsedTime(&ms, c->ev_a, c->ev_b);
     S.closure_ms = ms;
     S.join_ms = join_ms;
-    S.join_launches = joins;
+    S.join_launches = joins + c->h_ctr[C_JCNT];
     S.left_elems = c->h_ctr[C_LEFT];
     S.window_out_elems = c->h_ctr[C_WOUT];
     S.window_noslot_items = c->h_ctr[C_NOSLOT];
@@ -6043,14 +6084,16 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
             if (pass == 0 && nd + nv < (rt.nol ? tile_min(rt.nol) : (uint64_t)SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
                 // few records: their parts (in rbuf[1], free in this pass)
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
-                k_split<<<grid((nd + nv) * EW, 256, 8), 256, 0, s>>>(d, gbuf, vbuf, rbuf[1], 0, ~0ull, 0);
+                k_split<<<grid((nd + nv) * EW, 256, 8), 256, 0, s>>>(d, gbuf, vbuf, nullptr, rbuf[1], 0, ~0ull, 0, 0);
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
                 k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_SPLIT_N, rbuf[0]);
             } else if (pass == 0 && rt.nol) {
                 // gslot and rbuf[1] are free in this pass: the tile list and the records left to k_join
-                launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0], tile_rows_lg(nd + nv));
+                k_split<<<1, TILE_SAMPLE, 0, s>>>(d, gbuf, vbuf, nullptr, nullptr, 1, 0, 0, 0);
+                launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0]);
+                k_split<<<sms, TILE_SAMPLE, 0, s>>>(d, gbuf, vbuf, rbuf[1], nullptr, SPLIT_LEFT, 0, 0, 0);
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
-                k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_LN, rbuf[0]);
+                k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_JN1, rbuf[0]);
             } else {
                 // the round's records (pass 0, no virtual ones), or those that failed in the last pass
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));

@@ -248,12 +248,12 @@ def _wide(nv, rows, kblocks, bits, deg, seed=0):
     (20_000, 4000, 4, 50, 2000, "none"),     # right rows of 105 elements, dense: 14 windows
     (20_000, 4000, 4, 50, 150, "none"),      # the same, 79 of 105 elements in a row
     (200_000, 4000, 4, 50, 3, "all"),        # 3 elements a right row, anywhere in 1,042: given up after 8 windows
-    (20_000, 3000, 40, 30, 5, "some"),       # more blocks of intermediates than a tile's table holds (32)
-    (20_000, 3000, 50, 30, 4, "whole"),      # more leftovers than are cut: joined as they are
+    (20_000, 3000, 40, 40, 5, "some"),       # more blocks of intermediates than a tile's table holds (32)
+    (20_000, 3000, 50, 40, 4, "whole"),      # more leftovers than are cut: joined as they are
     (20_000, 4000, 100, 60, 4, "whole"),
-    (20_000, 3000, 50, 30, -4, "whole"),     # (destinations in 8 blocks)
-    (20_000, 1200, 36, 30, -4, "split"),     # leftovers cut by bitmap word (32,768 to 131,072 of them)
-    (20_000, 300, 36, 30, -4, "parts"),      # fewer: cut into parts of 8 bits
+    (20_000, 3000, 50, 40, -4, "whole"),     # (destinations in 8 blocks)
+    (20_000, 1200, 36, 40, -4, "split"),     # leftovers cut by bitmap word (32,768 to 131,072 of them)
+    (20_000, 300, 36, 40, -4, "parts"),      # fewer: cut into parts of 8 bits
 ])
 def test_tiles_of_wide_rows(grg_mod, oracle_mod, nv, rows, kblocks, bits, deg, left):
     """Tiles at their limits: windows, blocks of intermediates, and the sizes of the list they leave (rows of
@@ -291,3 +291,50 @@ def test_tile_rows_that_outgrow_their_tables(grg_mod, oracle_mod, monkeypatch, r
             st = ctx.closure(0)
             assert (ctx.label_counts().tolist(), ctx.set_hash()) == (r.label_counts().tolist(), r.set_hash)
             assert ctx.last_joins()["tiles"] > 0 and st["retry_records"] > 0 and st["grow_rows"] >= 4000
+
+
+def _chains(nv, length):
+    """A ::= e, A ::= A A over chains of `length` vertices."""
+    src = np.arange(nv - 1, dtype=np.uint32)
+    src = src[(src + 1) % length != 0]
+    return nv, np.array([[1, 2, 0], [1, 1, 1]], np.int32), 2, 0, src, src + 1, np.full(len(src), 2, np.uint8)
+
+
+@pytest.mark.parametrize("nv,length,tiled", [(60_000, 20, False), (6_000, 24, False), (150_000, 30, False),
+                                             (60_000, 400, True)])
+def test_sparse_rounds_join_without_tiles(grg_mod, oracle_mod, nv, length, tiled):
+    """Rounds whose records hold few intermediates run without tiles, however many they are."""
+    w = _chains(nv, length)
+    r = oracle_mod.closure(*w)
+    for dev in (True, False):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(dev)
+            ctx.transfer_rules(w[1], w[2])
+            ctx.load_edges(w[0], *w[4:])
+            ctx.closure(0)
+            assert (ctx.label_counts().tolist(), ctx.set_hash()) == (r.label_counts().tolist(), r.set_hash)
+            assert (ctx.last_joins()["tiles"] > 0) == tiled
+
+
+@pytest.mark.parametrize("w", [_chains(6_000, 24), _chains(6_000, 3_000), "alias"], ids=["sparse", "dense", "alias"])
+def test_static_scratch_above_the_split_line(grg_mod, oracle_mod, w):
+    """The allocation-free closure with rounds of more records than it cuts: with tiles and without."""
+    import torch
+
+    if w == "alias":
+        a = G.alias(seed=9, num_vars=3_000, num_base_edges=12_000, block=1000)
+        w = a.num_vars, a.rule_ids(), a.num_labels, 0, a.src, a.dst, a.lab
+    nv, rules, nl, f, src, dst, lab = w
+    r = oracle_mod.closure(*w)
+    d = [torch.from_numpy(x).cuda() for x in (src.view(np.int32), dst.astype(np.uint32).view(np.int32), lab)]
+    counts = torch.full((nl,), -1, dtype=torch.int64, device="cuda")
+    h = torch.zeros(1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    ptr = [ctypes.c_void_p(x.data_ptr()) for x in (*d, counts, h)]
+    rules = np.ascontiguousarray(rules, np.int32).reshape(-1)
+    rounds = ctypes.c_uint64()
+    st = grg_mod.load_library().grg_closure_noalloc(0, None, len(rules) // 3, ctypes.c_void_p(rules.ctypes.data), nl, f,
+                                                    nv, len(src), *ptr, ctypes.byref(rounds))
+    assert st == grg_mod.OK
+    got = counts.cpu().numpy().view(np.uint64).tolist(), int(h.cpu().numpy().view(np.uint64)[0])
+    assert got == (r.label_counts().tolist(), r.set_hash)
