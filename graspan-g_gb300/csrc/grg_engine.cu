@@ -1804,16 +1804,12 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
 // as they are. The choice is made here, on the device: the joins read their
 // counts from C_JN1 / C_JN2 / C_SPLIT_N.
 constexpr uint32_t SPLIT_MAX = 32768;
-// The same line for rounds that otherwise go through k_tile: it depends on how many old-left rules
-// the round's records are spread over. 3,000-vertex alias graph (2 rules), in the static scratch:
-// 6.1 ms with the line at 8,192 records, 8.2 ms at 32,768; 600-vertex points-to graph (6 rules):
-// 3.8 ms at 8,192 and 3.2 ms at 32,768.
-constexpr uint32_t TILE_MIN_RULE = 5461;
-__host__ __device__ inline uint64_t tile_min(int nol)
-{
-    const uint64_t n = (uint64_t)TILE_MIN_RULE * (uint64_t)nol;
-    return n < SPLIT_MAX ? n : SPLIT_MAX;
-}
+// The same line for rounds that otherwise go through k_tile. Closures (ms) with it at 5,461, 10,922, 21,844 and
+// 32,768 records: alias (2 old-left rules) of 1,500 vertices 1.75, 1.59, 1.54, 1.66; 5,000 2.61, 2.74, 2.55,
+// 2.60; 10,000 3.02, 3.01, 2.99, 3.00; 3,000 in the static scratch 4.28, 3.59, 4.47, 4.17; points-to (6 rules)
+// of 300 vertices 1.54, 1.47, 1.47, 1.47; 600 2.22, 2.21, 2.29, 2.32; 1,500 3.31, 3.28, 3.27, 3.39; chains
+// (1 rule) of 2,000 vertices 1.10, 1.22, 1.32, 1.35; of 4,000 1.12, 1.10, 1.07, 1.08.
+constexpr uint32_t TILE_MIN = SPLIT_MAX / 3;
 constexpr uint32_t SPLIT_BITS = 8;
 constexpr uint32_t SPLIT_PARTS = (EIDS + SPLIT_BITS - 1) / SPLIT_BITS;
 // Records that tiles leave to k_join are cut too: a warp that takes 32 of them whole is done long after
@@ -4539,7 +4535,7 @@ static int round_oldleft(grg_ctx *c, uint64_t *nv_out)
 // pass are re-run until nothing fails.
 // Retry list size for a round of n records: retries come only from tables at
 // their load limit, a small share; a round with more is re-run whole.
-static uint64_t split_max(const grg_ctx *c) { return use_tiles(c) ? tile_min(c->rt.nol) : SPLIT_MAX; }
+static uint64_t split_max(const grg_ctx *c) { return use_tiles(c) ? TILE_MIN : SPLIT_MAX; }
 static uint64_t retry_room(const grg_ctx *c, uint64_t n) { return std::max<uint64_t>(c->retry_min, n / 8); }
 
 // The first join pass of a round over its records: the parts of a small round
@@ -4665,7 +4661,7 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
     cudaStream_t s = c->stream;
     int st = ensure_rbuf(c, retry_room(c, nd + nv));
     if (st) return st;
-    if (nd + nv >= tile_min(c->rt.nol)) ensure_tiles(c, nd + nv + (nd + nv) / 2);
+    if (nd + nv >= TILE_MIN) ensure_tiles(c, nd + nv + (nd + nv) / 2);
     const bool split = nd + nv < split_max(c);
     if ((split || use_tiles(c)) && (st = ensure_sbuf(c))) return st;
     Dev d = make_dev(c);
@@ -6081,7 +6077,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
         for (int pass = 0;; pass++) {
             const int g = grid((n + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16);
             // each join launch pulls 32-record batches from a queue that starts at 0
-            if (pass == 0 && nd + nv < (rt.nol ? tile_min(rt.nol) : (uint64_t)SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
+            if (pass == 0 && nd + nv < (rt.nol ? TILE_MIN : SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
                 // few records: their parts (in rbuf[1], free in this pass)
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
                 k_split<<<grid((nd + nv) * EW, 256, 8), 256, 0, s>>>(d, gbuf, vbuf, nullptr, rbuf[1], 0, ~0ull, 0, 0);
