@@ -2289,7 +2289,7 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
 // within a procedure, and all 96 for a row whose records spread wider (an unconfined graph's row of
 // 52 elements, or one that reaches several blocks, sent most of its items to k_join's hash). Records of
 // rows that reach across more than 96 get windows of their own where their destinations are local, the
-// row's one window where they are not (see `near`). What the windows leave out becomes a candidate of
+// row's one window where they are not (see `apart`). What the windows leave out becomes a candidate of
 // one bit. Bound by integer issue (2.3 of 2-4 warp
 // instructions a clock, 13 a pair). Closures: 10k vertices unconfined 11.1 -> 7.8 ms, 97k in blocks
 // 6.2 -> 5.8 ms, 2M in blocks 53.5 -> 48.7 ms (at 8 blocks a SM 48.8, at 6 51.3, at 10 56.4).
@@ -2310,7 +2310,9 @@ struct __align__(16) RowsSmem {
     uint16_t list[ROWS_LIST];                  // record << 8 | position of its bit
     uint8_t first[8];                          // the first record of each window's run
     unsigned long long near, wide;             // C_RNEAR and C_RWIDE of this warp's batches
-    uint32_t seen;                             // destinations of the batch
+    uint32_t apart;                            // records of runs wider than the window get windows of their own,
+    uint32_t on, seen, reach;                  // some of this batch do: its destinations, its widest run's elements
+                                               // (here and not in registers: 2M blocks 42.6 ms, 43.3)
 };
 
 __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
@@ -2345,8 +2347,11 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
     // destinations than a window over ROWS_ELEMS of the run's `reach` elements would. Closures with one
     // window a run, with this rule, and k_join's: 30,000 local vertices 69.7, 56.4, 86.9 ms; 50,000
     // 260, 147, 240; 100,000 1254, 647, 1048; 60,000 vertices without locality 126, 125, 168 ms.
-    bool near = d.ctr[C_RNEAR] >= d.ctr[C_RWIDE];
-    if (lane == 0) w.near = w.wide = 0;
+    if (lane == 0) {
+        w.near = w.wide = 0;
+        w.apart = d.ctr[C_RNEAR] >= d.ctr[C_RWIDE];
+    }
+    __syncwarp();
     const uint32_t batch = batch_records(n, (uint64_t)gridDim.x * ROWS_WARPS);
     const uint64_t nbatch = (n + batch - 1) / batch;
     uint64_t bt = 0;
@@ -2382,11 +2387,17 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
         // windows: a run's destinations are taken to lie as far around its intermediates as a group of
         // ROWS_NEAR elements that holds them all reaches; runs in more than that get the warp's
         // whole window to themselves, in a pass of their own, and records of a run that even the whole
-        // window does not reach across are runs of their own (near)
+        // window does not reach across are runs of their own
         const bool far = real && hi - lo >= (uint32_t)ROWS_ELEMS;
-        const uint32_t reach = __reduce_max_sync(0xffffffffu, far ? hi - lo + 1 : 0u);
-        if (reach && near) {
-            if (lane == 0) w.seen = 0;
+        __syncwarp();
+        if (lane == 0) w.on = 0;
+        if (w.apart && __any_sync(0xffffffffu, far)) {
+            const uint32_t reach = __reduce_max_sync(0xffffffffu, far ? hi - lo + 1 : 0u);
+            if (lane == 0) {
+                w.seen = 0;
+                w.on = 1;
+                w.reach = reach;
+            }
             flush_counters();
             if (far) {
                 start = true;
@@ -2507,7 +2518,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
                                 if (lane >= (uint32_t)o) inc += y;
                             }
                             const uint32_t items = __shfl_sync(0xffffffffu, inc, 31), s1 = inc - deg;
-                            if (lane == 0) w.seen += items;
+                            if (w.on && lane == 0) w.seen += items;
                             const unsigned some = __ballot_sync(0xffffffffu, deg != 0);
                             __syncwarp();
                             if (deg) w.rows[__popc(some & lt)] = make_uint4(rw.x - s1, tid0, tat0, r);
@@ -2564,14 +2575,15 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, GRG_ROWS_MINB)
                 __syncwarp();
             }
         }
-        if (reach && near) {
+        __syncwarp();
+        if (w.on) {
             const uint32_t out = __reduce_add_sync(0xffffffffu, n_out);
             if (lane == 0) {
-                w.near += (uint64_t)(w.seen - out) * reach;
+                w.near += (uint64_t)(w.seen - out) * w.reach;
                 w.wide += (uint64_t)w.seen * ROWS_ELEMS;
+                w.apart = w.near >= w.wide;
             }
             __syncwarp();
-            near = w.near >= w.wide;
         }
         // a failed insert re-runs the records of its run (of the record, for a unary rule or a
         // destination outside the window)
