@@ -4129,8 +4129,8 @@ static void choose_window(grg_ctx *c)
 
 // The join kernel in the window chosen for this closure (join_wide), reading the
 // right-hand rows of CSR-copied labels as ids or (join_elems) as table elements.
-static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d, const uint4 *recs, uint64_t n,
-                        int n_ctr, uint4 *retry_out)
+static cudaError_t launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d, const uint4 *recs, uint64_t n,
+                               int n_ctr, uint4 *retry_out)
 {
     const Dev *dp = &d;
     Dev de;
@@ -4140,11 +4140,11 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
         dp = &de;
     }
     // the launch's work queue starts at batch 0; the grid is what the SMs hold at once
-    cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s);
+    if (cudaError_t e = cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s)) return e;
     if (c->join_rows) {
         const int g = std::min(grid, c->sms * GRG_ROWS_MINB);
         k_rows<<<g, ROWS_WARPS * 32, 0, s>>>(d, recs, n, n_ctr, retry_out);
-        return;
+        return cudaGetLastError();
     }
     const int resident = c->sms * (c->join_wide ? GRG_JOIN_MINB_WIDE : GRG_JOIN_MINB);
     if (grid > resident) grid = resident;
@@ -4152,6 +4152,7 @@ static void launch_join(const grg_ctx *c, int grid, cudaStream_t s, const Dev &d
         k_join<WIN2, WIN2_LO><<<grid, JOIN_WARPS * 32, 0, s>>>(*dp, recs, n, n_ctr, retry_out);
     else
         k_join<WIN, WIN_LO><<<grid, JOIN_WARPS * 32, 0, s>>>(*dp, recs, n, n_ctr, retry_out);
+    return cudaGetLastError();
 }
 
 // Rounds go through k_tile where a rule's second symbol is derivable (old-left joins): their right
@@ -4162,13 +4163,15 @@ static bool tiles_wanted(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_pu
 static bool use_tiles(const grg_ctx *c) { return tiles_wanted(c) && c->lbuf_cap > 0; }
 
 // The tiles of a round's gathered and virtual records, list, then join: counts and rows (C_TS) from the device.
-static void launch_tiles(int sms, cudaStream_t s, const Dev &d, const uint4 *grecs, const uint4 *vrecs, uint32_t *list,
-                         uint4 *left, uint64_t cap, uint4 *retry_out)
+static cudaError_t launch_tiles(int sms, cudaStream_t s, const Dev &d, const uint4 *grecs, const uint4 *vrecs,
+                                uint32_t *list, uint4 *left, uint64_t cap, uint4 *retry_out)
 {
-    cudaMemsetAsync(d.ctr + C_TN, 0, 24, s);                    // tiles, tile queue, records left to k_join
-    cudaFuncSetAttribute(k_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
+    cudaError_t e = cudaMemsetAsync(d.ctr + C_TN, 0, 24, s);    // tiles, tile queue, records left to k_join
+    if (!e) e = cudaFuncSetAttribute(k_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
+    if (e) return e;
     k_tile_starts<<<sms * 8, 256, 0, s>>>(d, grecs, vrecs, list, cap);
     k_tile<<<sms, TILE_THREADS, sizeof(TileSmem), s>>>(d, grecs, vrecs, list, cap, left, cap, retry_out);
+    return cudaGetLastError();
 }
 
 static bool any_csr(const grg_ctx *c)
@@ -4205,23 +4208,24 @@ static uint32_t pass_kernels(const grg_ctx *c) { return (c->need_join ? 1u : 0u)
 
 // One join pass over n records (or the device count n_ctr): the kernels the rule
 // table needs, each taking its own records and skipping the others'.
-static void launch_pass(grg_ctx *c, int grid, cudaStream_t s, const Dev &d, const uint4 *recs, uint64_t n, int n_ctr,
-                        uint4 *retry_out, uint64_t &joins)
+static cudaError_t launch_pass(grg_ctx *c, int grid, cudaStream_t s, const Dev &d, const uint4 *recs, uint64_t n,
+                               int n_ctr, uint4 *retry_out, uint64_t &joins)
 {
     if (c->need_join) {
-        launch_join(c, grid, s, d, recs, n, n_ctr, retry_out);
+        if (cudaError_t e = launch_join(c, grid, s, d, recs, n, n_ctr, retry_out)) return e;
         c->launches++;
         joins++;
     }
     if (c->need_push) {
         if (c->push_flat) {
-            cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s);
+            if (cudaError_t e = cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s)) return e;
             k_push_flat<<<c->sms * 4, PUSH_WARPS * 32, 0, s>>>(d, recs, n, n_ctr, retry_out);
         } else
             k_push<<<c->sms * 8, 256, 0, s>>>(d, recs, n, n_ctr, retry_out);
         c->launches++;
         joins++;
     }
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- join-window tuning
@@ -4328,7 +4332,7 @@ static int tune_begin(grg_ctx *c, uint32_t filter)
     return GRG_OK;
 }
 
-static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, bool split, uint64_t &joins);
+static int first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, bool split, uint64_t &joins);
 
 // The first pass of a round with its window measured (see above): both windows
 // are timed twice, interleaved, on a slice of the round's records (an eighth, at
@@ -4356,7 +4360,7 @@ static int tune_first_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, u
     float best[2][2] = {{1e30f, 1e30f}, {1e30f, 1e30f}}, best_rows = 1e30f;        // [wide][elems], k_rows
     auto trial = [&](bool timed, float &ms_best) -> int {
         if (timed) GRG_CUDA(c, cudaEventRecord(c->ev_t0, s));
-        launch_join(c, grid, s, d, c->gbuf, nt, -1, c->rbuf[0]);
+        GRG_CUDA(c, launch_join(c, grid, s, d, c->gbuf, nt, -1, c->rbuf[0]));
         c->launches++;
         joins++;
         if (!timed) return GRG_OK;
@@ -4418,8 +4422,7 @@ static int tune_first_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, u
         g_tune_cache[c->tune_key] = JoinChoice{wide, elems, c->tuned_rows};
         if (rows) g_rows_measured.insert(c->tune_input);
     }
-    first_pass_joins(c, d, nd, nv, false, joins);
-    return GRG_OK;
+    return first_pass_joins(c, d, nd, nv, false, joins);
 }
 
 // The first pass of a round whose join pass is pushes only, with the push kernel
@@ -4443,7 +4446,7 @@ static int tune_push_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, ui
         const int k = it < 0 ? 1 : it & 1;     // 0 one lane per record, 1 flattened
         c->push_flat = k == 1;
         if (it >= 0) GRG_CUDA(c, cudaEventRecord(c->ev_t0, s));
-        launch_pass(c, 0, s, d, c->gbuf, nt, -1, c->rbuf[0], joins);
+        GRG_CUDA(c, launch_pass(c, 0, s, d, c->gbuf, nt, -1, c->rbuf[0], joins));
         if (it < 0) continue;
         float ms = 0;
         GRG_CUDA(c, cudaEventRecord(c->ev_t1, s));
@@ -4465,8 +4468,7 @@ static int tune_push_pass(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, ui
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_push_cache[c->tune_key] = flat;
     }
-    first_pass_joins(c, d, nd, nv, false, joins);
-    return GRG_OK;
+    return first_pass_joins(c, d, nd, nv, false, joins);
 }
 
 // Round head: count and gather the dirty slots (rs: stamp for elements that
@@ -4552,32 +4554,36 @@ static uint64_t retry_room(const grg_ctx *c, uint64_t n) { return std::max<uint6
 
 // The first join pass of a round over its records: the parts of a small round
 // (sub-records in sbuf, count on the device) or the gathered and virtual records.
-static void first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, bool split, uint64_t &joins)
+static int first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, bool split, uint64_t &joins)
 {
     cudaStream_t s = c->stream;
     if (split) {
-        launch_pass(c, grid_for(c, ((nd + nv) * SPLIT_PARTS + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0,
-                    C_SPLIT_N, c->rbuf[0], joins);
-        return;
+        GRG_CUDA(c, launch_pass(c, grid_for(c, ((nd + nv) * SPLIT_PARTS + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d,
+                                c->sbuf, 0, C_SPLIT_N, c->rbuf[0], joins));
+        return GRG_OK;
     }
     if (use_tiles(c)) {
         k_split<<<1, TILE_SAMPLE, 0, s>>>(d, c->gbuf, c->vbuf, nullptr, nullptr, 1, 0, ~0ull, pass_kernels(c));
-        launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]);
-        cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s);
+        GRG_CUDA(c, launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]));
+        GRG_CUDA(c, cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
         k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->lbuf, c->sbuf, SPLIT_LEFT,
                                                                 SPLIT_LEFT_MAX, SPLIT_MAX, 0);
-        launch_join(c, grid_for(c, (nd + nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
-        launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0]);
+        GRG_CUDA(c, launch_join(c, grid_for(c, (nd + nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->lbuf, 0, C_JN1,
+                                c->rbuf[0]));
+        GRG_CUDA(c, launch_join(c, grid_for(c, SPLIT_MAX * SPLIT_PARTS / RB_MIN, JOIN_WARPS, 16), s, d, c->sbuf, 0,
+                                C_SPLIT_N, c->rbuf[0]));
         c->launches += 6;
-        return;
+        return GRG_OK;
     }
-    launch_pass(c, grid_for(c, (nd + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0], joins);
+    GRG_CUDA(c, launch_pass(c, grid_for(c, (nd + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->gbuf, nd, -1, c->rbuf[0],
+                            joins));
     if (nv) {
         // virtual old-left records: joined by source rows only
-        launch_join(c, grid_for(c, (nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->vbuf, nv, -1, c->rbuf[0]);
+        GRG_CUDA(c, launch_join(c, grid_for(c, (nv + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->vbuf, nv, -1, c->rbuf[0]));
         c->launches++;
         joins++;
     }
+    return GRG_OK;
 }
 
 // Tables that overflowed grow (the pool too, when it is full); then the failed
@@ -4619,11 +4625,11 @@ static int round_retries(grg_ctx *c, uint64_t nr, uint64_t nf, grg_stats &S, dou
         GRG_CUDA(c, cudaMemsetAsync(c->ctr + C_RETRY_N, 0, 16, s));
         if (c->timing) GRG_CUDA(c, cudaEventRecord(c->ev_c, s));
         if (rerun_all) {
-            first_pass_joins(c, d, nd, nv, split, joins);
+            if (int st1 = first_pass_joins(c, d, nd, nv, split, joins)) return st1;
             rb = 0;
         } else if (nr) {
-            launch_pass(c, grid_for(c, (nr + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->rbuf[rb], nr, -1, c->rbuf[rb ^ 1],
-                        joins);
+            GRG_CUDA(c, launch_pass(c, grid_for(c, (nr + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16), s, d, c->rbuf[rb], nr, -1,
+                                    c->rbuf[rb ^ 1], joins));
             rb ^= 1;
         }
         if (c->cand_cap) {
@@ -4688,8 +4694,8 @@ static int round_joins(grg_ctx *c, uint64_t nd, uint64_t nv, grg_stats &S, doubl
         if ((st = tune_first_pass(c, d, nd, nv, joins))) return st;
     } else if (c->push_pending && c->need_push && !c->need_join && !split && nd >= TUNE_MIN_RECORDS) {
         if ((st = tune_push_pass(c, d, nd, nv, joins))) return st;
-    } else {
-        first_pass_joins(c, d, nd, nv, split, joins);
+    } else if ((st = first_pass_joins(c, d, nd, nv, split, joins))) {
+        return st;
     }
     // insert the candidates the joins wrote (count read on the device)
     if (c->cand_cap) {
@@ -4841,7 +4847,10 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
         k_dindex_clear<<<grid_for(c, c->gbuf_cap, 256), 256, 0, s>>>(d, c->gbuf, C_DIRTY_N);
         nk++;
     }
-    if (c->job_cnt) cudaMemsetAsync(c->job_cnt, 0, (size_t)c->max_jobs * 4, s);
+    // the first call that fails; the capture is ended before it is reported
+    cudaError_t le = cudaSuccess;
+    auto call = [&](cudaError_t e) { if (le == cudaSuccess) le = e; };
+    if (c->job_cnt) call(cudaMemsetAsync(c->job_cnt, 0, (size_t)c->max_jobs * 4, s));
     if (c->timing) {
         k_tmark<<<1, 32, 0, s>>>(ctr, C_GT0, C_GNS, 0);
         nk++;
@@ -4875,20 +4884,20 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
         const uint64_t launches0 = c->launches;
         uint64_t unused = 0;
         if (tiles) {
-            launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]);
+            call(launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]));
             k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->lbuf, c->sbuf, SPLIT_LEFT,
                                                                     SPLIT_LEFT_MAX, SPLIT_MAX, 0);
-            launch_join(c, jgrid, s, d, c->lbuf, 0, C_JN1, c->rbuf[0]);
+            call(launch_join(c, jgrid, s, d, c->lbuf, 0, C_JN1, c->rbuf[0]));
             nk += 4;
         } else {
-            launch_pass(c, jgrid, s, d, c->gbuf, 0, C_JN1, c->rbuf[0], unused);
+            call(launch_pass(c, jgrid, s, d, c->gbuf, 0, C_JN1, c->rbuf[0], unused));
         }
-        launch_pass(c, jgrid, s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0], unused);
+        call(launch_pass(c, jgrid, s, d, c->sbuf, 0, C_SPLIT_N, c->rbuf[0], unused));
         nk += (int)(c->launches - launches0);
         c->launches = launches0;
     }
     if (c->rt.nol && !tiles) {
-        launch_join(c, jgrid, s, d, c->vbuf, 0, C_JN2, c->rbuf[0]);
+        call(launch_join(c, jgrid, s, d, c->vbuf, 0, C_JN2, c->rbuf[0]));
         nk++;
     }
     if (c->cand_cap) {
@@ -4902,8 +4911,11 @@ static int build_round_graph(grg_ctx *c, uint32_t rs)
     k_gate_end<<<1, 32, 0, s>>>(ctr, h);
     nk++;
     cudaGraph_t captured = body;
-    const cudaError_t ce = cudaStreamEndCapture(s, &captured);
+    call(cudaGetLastError());
+    cudaError_t ce = cudaStreamEndCapture(s, &captured);
+    if (le != cudaSuccess) ce = le;
     if (ce != cudaSuccess) {
+        cudaGetLastError();
         free_round_graph(c);
         return fail(c, GRG_E_CUDA, std::string("round graph capture: ") + cudaGetErrorString(ce));
     }
@@ -6098,7 +6110,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
             } else if (pass == 0 && rt.nol) {
                 // gslot and rbuf[1] are free in this pass: the tile list and the records left to k_join
                 k_split<<<1, TILE_SAMPLE, 0, s>>>(d, gbuf, vbuf, nullptr, nullptr, 1, 0, 0, 0);
-                launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0]);
+                NA_CUDA(launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0]));
                 k_split<<<sms, TILE_SAMPLE, 0, s>>>(d, gbuf, vbuf, rbuf[1], nullptr, SPLIT_LEFT, 0, 0, 0);
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
                 k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_JN1, rbuf[0]);
