@@ -280,7 +280,7 @@ constexpr int ALLOC_ROWS = 1024;
 __global__ void __launch_bounds__(ALLOC_ROWS) k_load_alloc(Dev d, uint32_t first, uint32_t nv, uint32_t L, MinCap mc,
                                                            const uint32_t *__restrict__ rowmark)
 {
-    __shared__ uint32_t warp_sum[ALLOC_ROWS / 32];
+    __shared__ uint64_t warp_sum[ALLOC_ROWS / 32];
     __shared__ unsigned long long base_s;
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     const uint64_t groups = ((uint64_t)nv + ALLOC_ROWS - 1) / ALLOC_ROWS;
@@ -300,18 +300,20 @@ __global__ void __launch_bounds__(ALLOC_ROWS) k_load_alloc(Dev d, uint32_t first
             if (cap < 4) cap = 4;
             while (cap < need) cap <<= 1;
         }
-        uint32_t incl = cap;
+        // 64-bit sums: tables are sized by edges, and 1,024 rows of 2M edges ask for 2^32 slots, which
+        // has to be refused below
+        uint64_t incl = cap;
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= (uint32_t)o) incl += y;
         }
         if (lane == 31) warp_sum[wid] = incl;
         __syncthreads();
         if (wid == 0) {
-            const uint32_t s = warp_sum[lane];
-            uint32_t si = s;
+            const uint64_t s = warp_sum[lane];
+            uint64_t si = s;
             for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, si, o);
+                const uint64_t y = __shfl_up_sync(0xffffffffu, si, o);
                 if (lane >= (uint32_t)o) si += y;
             }
             warp_sum[lane] = si - s;
