@@ -61,7 +61,7 @@ enum : int {
     C_LABEL0 = 24,    // per-label edge counts: C_LABEL0 + slot
     C_JT0 = C_LABEL0 + MAX_SLOTS + 2,   // start time of the current join pass (device-driven rounds)
     C_MAXR = C_LABEL0 + MAX_SLOTS + 3,  // rounds a device-driven launch may run (0 = until the fixpoint)
-    C_WOUT = C_LABEL0 + MAX_SLOTS + 4,  // right-hand items the join's dense window could not hold
+    C_WOUT = C_LABEL0 + MAX_SLOTS + 4,  // right-hand items outside the joins' dense windows
     C_SPLIT_N = C_LABEL0 + MAX_SLOTS + 5,  // sub-records of a small round (k_split)
     C_JN1 = C_LABEL0 + MAX_SLOTS + 6,   // records the join reads from the gathered buffer (or, after k_tile, as it left them) this round
     C_JN2 = C_LABEL0 + MAX_SLOTS + 7,   // records the join reads from the virtual-record buffer this round
@@ -70,7 +70,7 @@ enum : int {
     C_BADIN = C_LABEL0 + MAX_SLOTS + 10, // input edges refused: ERR_IN_LABEL / ERR_IN_RANGE bits
     C_DH0 = C_LABEL0 + MAX_SLOTS + 11,   // 8 counters: tables by log2 of their elements (tuning key)
     C_CHECK = C_LABEL0 + MAX_SLOTS + 19, // first failed bounds check of the push kernels: id << 56 | value
-    C_JQ = C_LABEL0 + MAX_SLOTS + 20,    // work queue of a join or push launch: next 32-record batch (zeroed before each launch)
+    C_JQ = C_LABEL0 + MAX_SLOTS + 20,    // work queue of a join or push launch: next batch of 8 to 32 records (zeroed before each launch)
     C_NOSLOT = C_LABEL0 + MAX_SLOTS + 21, // of C_WOUT: items of a run of records left without a window slot
     C_CANDS = C_LABEL0 + MAX_SLOTS + 22,  // candidates k_apply inserted over the closure
     C_TN = C_LABEL0 + MAX_SLOTS + 23,     // tiles of the round (k_tile_starts); zeroed with the next two

@@ -1994,14 +1994,14 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
     // a persistent grid: each warp pulls its next batch of records from the launch's
     // device queue (C_JQ, zeroed before the launch), so warps that drew light batches take
     // more of them instead of idling behind the ones that drew heavy records
-    const uint32_t rb = batch_records(n, (uint64_t)gridDim.x * JOIN_WARPS);
-    const uint64_t nbatch = (n + rb - 1) / rb;
+    const uint32_t batch = batch_records(n, (uint64_t)gridDim.x * JOIN_WARPS);
+    const uint64_t nbatch = (n + batch - 1) / batch;
     uint64_t bt = 0;
     if (lane == 0) bt = atomicAdd(&d.ctr[C_JQ], 1ull);
     bt = __shfl_sync(0xffffffffu, bt, 0);
     for (; bt < nbatch; bt = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(&d.ctr[C_JQ], 1ull) : 0ull, 0)) {
-        const uint64_t ri = bt * rb + lane;
-        const bool have = lane < rb && ri < n;
+        const uint64_t ri = bt * batch + lane;
+        const bool have = lane < batch && ri < n;
         Bits rb;
         uint32_t key = EMPTY, row = 0;
         if (have) {
@@ -6102,7 +6102,7 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
         int rb = 0;
         for (int pass = 0;; pass++) {
             const int g = grid((n + RB_MIN - 1) / RB_MIN, JOIN_WARPS, 16);
-            // each join launch pulls 32-record batches from a queue that starts at 0
+            // each join launch pulls batches of 8 to 32 records from a queue that starts at 0
             if (pass == 0 && nd + nv < (rt.nol ? TILE_MIN : SPLIT_MAX) && (nd + nv) * SPLIT_PARTS <= pool) {
                 // few records: their parts (in rbuf[1], free in this pass)
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
