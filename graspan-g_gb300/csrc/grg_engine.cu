@@ -1248,13 +1248,17 @@ __global__ void __launch_bounds__(PUSH_WARPS * 32, 4) k_push_flat(Dev d, const u
 //  - a record whose panel's union adds nothing to A[i] is done at once: late rounds (0.9M (i, k)
 //    pairs a block and round in the old-left joins, against a few thousand new edges) cost a
 //    compare a record instead of a pass over C's rows.
-// 1M-vertex alias closure: right-hand elements read 2.3e10 -> 5.4e8, closure 189 -> 70.9 ms;
-// 37k vertices 13.4 -> 6.0 ms. A block holds one tile a SM (214 KB), bound by the lookups' shared
-// memory reads (21 of 16 bytes a lane and record in the mean) and by the waits between its phases.
+// 1M-vertex alias closure: right-hand elements read 2.3e10 -> 6.0e8, closure 189 -> 68.6 ms;
+// 37k vertices 13.4 -> 5.4 ms. A block holds one tile a SM (217,424 bytes), bound by waits: 1.5 to 1.7
+// warp instructions a clock of 4 on a 100k-vertex graph, a warp waiting on shared memory (the lookups),
+// on dependent loads (descriptors, then elements) and on the barriers between phases in like parts, L1
+// and shared memory at 49 to 60% of peak. 1,024 threads leave 64 registers, with 156 and 300 bytes of
+// spill stores and loads.
 // Only accumulator words that changed are inserted. Right-hand elements outside the window of
-// TILE_W elements are joined in further windows (up to TILE_WINDOWS, each from the lowest base
-// not yet covered); blocks of intermediates with few records, and records that even the last
-// window leaves something of, go to a list that k_join takes.
+// TILE_W elements are joined in further windows (see TILE_WINDOWS; the first from the lowest block of
+// intermediates, each further one from the lowest base not yet covered); blocks of intermediates with few
+// records, or past the tile's TILE_KB, and records that even the last window leaves something of, go to
+// a list that k_join takes.
 constexpr int TILE_THREADS = 1024;
 constexpr int TILE_WARPS = TILE_THREADS / 32;
 constexpr int TILE_ROWS_LG = 8, TILE_ROWS = 1 << TILE_ROWS_LG;
@@ -1265,15 +1269,14 @@ constexpr int TILE_G = EIDS / 4;               // groups of 4 intermediates
 constexpr int TILE_RECS = 2048;                // records a tile holds at once (more are taken in turns)
 constexpr int TILE_KB = 32;                    // distinct blocks of intermediates at once
 // Windows of a tile: this many, and on while the last one held TILE_RICH quads of 16 bytes a panel (half an
-// element a row). A panel costs some 7,000 clocks an SM in every window; what the windows leave out sends the
-// tile's records to k_join whole, which takes about 14 clocks an SM for a pair and element: 96 elements
-// that 1,024 pairs over 192 rows join cost it the same. Unconfined alias rows of 105 elements
-// (20,000 vertices, dense): see the test of many windows.
+// element a row); what they leave out sends the tile's records to k_join whole. Unconfined alias rows of 73
+// elements (14,000 vertices): 32.8 s with 8 windows, 24.7 s so, 35.7 s with k_join alone. Rows of a few
+// elements anywhere in 1,000 blocks would take a window each: they stop at the eighth.
 constexpr uint32_t TILE_WINDOWS = 8;
 constexpr uint32_t TILE_RICH = 144;
 // Pairs (record, k) of a tile that pay for reading a panel; records of blocks with fewer go to k_join,
-// whose warps share them out over the chip. A panel holds an SM for some 7,000 clocks whatever it joins,
-// k_join takes a pair at a time: 4 pairs a row of the tile. Closures (ms) with 128 pairs at every size,
+// whose warps share them out over the chip. A panel costs its reads, subset unions and barriers whatever it
+// joins, k_join takes a pair at a time: 4 pairs a row of the tile. Closures (ms) with 128 pairs at every size,
 // 1,024 at 256 rows, and 4,096: 1M-vertex alias 82.6, 70.8, 69.3; 300k 28.3, 25.0, 25.2; 37k vertices
 // 6.8, 6.0, 8.9; tiles of 64 rows and fewer (3,000 vertices) 5.5 with 128, 6.3 with 512.
 __device__ __forceinline__ uint32_t tile_min_bits(uint32_t sh) { return 4u << sh; }
@@ -1704,7 +1707,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
                                 }
                                 const bool need = !covers4(a0, un);
                                 if (!__any_sync(0xffffffffu, need)) continue;
-                                // the groups of 4 bits that are not empty (21 of 48 in the mean)
+                                // the groups of 4 bits that are not empty
                                 const uint32_t g0 = (__shfl_sync(0xffffffffu, v, m * 8 + (lane >> 3)) >> (4 * (lane & 7))) & 15u;
                                 uint32_t g1 = (__shfl_sync(0xffffffffu, v, m * 8 + 4 + (lane >> 3 & 1)) >>
                                                (4 * (lane & 7))) & 15u;
@@ -1798,7 +1801,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
     }
 }
 
-// Small rounds: a warp joins 32 records, so a round of few, dense records (alias
+// Small rounds: a warp joins 8 to 32 records, so a round of few, dense records (alias
 // rows reach a whole block) leaves most SMs idle. Below SPLIT_MAX records the
 // round's gathered and virtual records are cut into sub-records of at most
 // SPLIT_BITS bits each (the union over a record's bits is the union over its
@@ -2292,9 +2295,10 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
 // 52 elements, or one that reaches several blocks, sent most of its items to k_join's hash). Records of
 // rows that reach across more than 96 get windows of their own where their destinations are local, the
 // row's one window where they are not (see `apart`). What the windows leave out becomes a candidate of
-// one bit. Bound by integer issue (2.3 of 2-4 warp
-// instructions a clock, 13 a pair). Closures: 10k vertices unconfined 11.1 -> 7.8 ms, 97k in blocks
-// 6.2 -> 5.8 ms, 2M in blocks 53.5 -> 48.7 ms (at 8 blocks a SM 48.8, at 6 51.3, at 10 56.4).
+// one bit. Bound by issue and short waits: 2.4 of 4 warp instructions a clock over the 2M-vertex closure in
+// blocks, 14.7 a pair, DRAM at 4% of its peak; 72 registers, with 128 and 220 bytes of spill stores and loads.
+// Closures: 10k vertices unconfined 11.1 -> 7.8 ms, 97k in blocks 6.2 -> 5.8 ms, 2M in blocks 53.5 -> 48.7 ms
+// (at 8 blocks a SM 48.8, at 6 51.3, at 10 56.4).
 constexpr int ROWS_WARPS = 4;
 constexpr int ROWS_ELEMS = 96;
 constexpr int ROWS_LIST = 512;                 // tasks listed at once
@@ -4112,9 +4116,10 @@ static bool rows_possible(const grg_ctx *c)
     return any;
 }
 
-// Window of this closure's joins. Measured on dataflow, alias, points-to and
-// small alias jobs, the wide window was fastest or within 1.5% on every one, so
-// it is the default; the narrow window stays selectable. Wide is 12 elements
+// Window of this closure's k_join launches (none where k_rows joins). With k_join
+// taking every join of dataflow, alias, points-to and small alias jobs the wide
+// window was fastest or within 1.5% on every one, so it is the default; the narrow
+// window stays selectable. Wide is 12 elements
 // (5 below the run's base). A warp has 8 window slots, one per run of a row's
 // records, and joins a batch of more runs in passes; a block takes 22 KB of
 // shared memory, and at 64 registers a thread (some bytes spilled) 8 blocks fit
@@ -4158,9 +4163,10 @@ static cudaError_t launch_join(const grg_ctx *c, int grid, cudaStream_t s, const
 }
 
 // Rounds go through k_tile where a rule's second symbol is derivable (old-left joins): their right
-// rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 70.9 ms).
+// rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 68.6 ms).
 // With static second symbols a right row is 1-2 elements, too few to pay for a panel: k_rows or k_join.
-// They do while there was room for the tile lists (ensure_tiles); k_join needs none.
+// They do while there is room for the tile lists (ensure_tiles), which k_join does not need, and for records
+// that are dense enough (TILE_MEAN).
 static bool tiles_wanted(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
 static bool use_tiles(const grg_ctx *c) { return tiles_wanted(c) && c->lbuf_cap > 0; }
 

@@ -79,7 +79,8 @@ typedef struct grg_stats {
                                       joined by rows, see grg_last_joins) */
     double gather_ms;              /* time of the rounds' gathers (when kernel timing is on) */
     uint64_t window_tuned;         /* how the join window was chosen: 0 fixed by grg_set_join_window
-                                      or nothing to choose (joins by rows), 1 measured in this closure, 2 taken from the tuning cache */
+                                      or nothing to choose (joins by rows), 1 measured in this closure,
+                                      2 taken from the tuning cache */
     double window_trial_ms[2];     /* the measured trial passes (narrow, wide) when window_tuned = 1 */
     uint64_t column_labels;        /* labels stored by destination in this closure (bit l-1 = label l;
                                       grg_set_layout); their joins are pushes, so right_elems then
@@ -147,9 +148,12 @@ int grg_set_device_rounds(grg_ctx *ctx, int on);
  * when the key is cached, and updates the cache. Environment
  * GRG_JOIN_WINDOW=narrow / wide / tuned selects the default. Grammars with a
  * derivable right-hand label join tiles of rows instead and use the window for
- * small rounds and for what the tiles leave; with static right-hand rows, mode
- * 2 or 3 here and for the items below joins by rows, whose window follows the
- * width of each row. Results are identical in every mode. */
+ * small and sparse rounds and for what the tiles leave. With static right-hand
+ * rows, mode 2 here and for the items below joins by rows, whose window follows
+ * the width of each row, and times nothing; mode 3 also times the row join, and
+ * it and later closures of the key in mode 2 keep the window's join where that
+ * is faster by 10%. grg_last_joins tells which join ran. Results are identical
+ * in every mode. */
 int grg_set_join_window(grg_ctx *ctx, int mode);
 /* Right-hand items of labels that have a CSR copy (never derived, read as a
  * binary rule's second symbol): mode 0 reads destination ids (4 bytes each,

@@ -338,3 +338,31 @@ def test_static_scratch_above_the_split_line(grg_mod, oracle_mod, w):
     assert st == grg_mod.OK
     got = counts.cpu().numpy().view(np.uint64).tolist(), int(h.cpu().numpy().view(np.uint64)[0])
     assert got == (r.label_counts().tolist(), r.set_hash)
+
+
+@pytest.mark.parametrize("direct", ["0", "1"])
+@pytest.mark.parametrize("room", [None, "16"])
+@pytest.mark.parametrize("nv,ne", [(400, 900), (4_000, 5_200), (40_000, 30_000)])
+def test_row_joins_of_several_rules(grg_mod, oracle_mod, monkeypatch, nv, ne, room, direct):
+    """Two right-hand labels and unary rules through the row join, in a pool that leaves no room to presize
+    rows: inserts of the join and of k_apply fail, tables grow, and the failed records (or, past the retry
+    list, the whole pass) run again."""
+    if room:
+        monkeypatch.setenv("GRG_RETRY_ROOM", room)
+    monkeypatch.setenv("GRG_DIRECT_INSERTS", direct)
+    rng = np.random.default_rng(nv)
+    src, dst = rng.integers(0, nv, (2, ne)).astype(np.uint32)
+    lab = rng.integers(2, 4, ne).astype(np.uint8)
+    rules = np.array([[1, 2, 0], [1, 1, 2], [1, 1, 3], [4, 1, 2], [4, 4, 3], [5, 4, 0]], np.int32)
+    r = oracle_mod.closure(nv, rules, 5, 0, src, dst, lab)
+    want = (r.label_counts().tolist(), r.set_hash)
+    for dev in (True, False):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_device_rounds(dev)
+            ctx.transfer_rules(rules, 5)
+            ctx.set_pool_limit(95 * nv * 65)              # slots of 65 bytes; presized rows take half of 96 nv
+            ctx.load_edges(nv, src, dst, lab)
+            st = ctx.closure(0)
+            assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
+            assert ctx.last_joins()["rows"] == 1 and st["direct_inserts"] == int(direct)
+            assert st["retry_records"] > 0 and st["grow_rows"] > 0
