@@ -49,8 +49,8 @@ sys.path[:0] = [ROOT, os.path.join(ROOT, "graspan-g_gb300")]
 import numpy as np  # noqa: E402
 
 # DRAM bytes (read + write) per join pass measured by ncu on the named workload, with the file
-# that records the capture: none of the row and tile joins yet
-TRAFFIC = {}
+# that records the capture
+TRAFFIC = {("dataflow", 2000): (432.8e6, "profiles/row_joins_dataflow_blocks.md")}
 METRIC = "closure_edges_per_sec"
 UNIT = "edges/s"
 WORKLOAD = ("dataflow_blocks: 2000 blocks x 1000 vertices, 6M 'e' edges + 6M 'N' seeds, "
@@ -519,7 +519,7 @@ def main():
         launches = s["rounds"]
         achieved = alg_bytes / (join_ms * 1e-3) / 1e9 if (join_ms > 0 and alg_bytes) else None
         # DRAM bytes per join pass, from a one-pass ncu capture of every launch of one closure
-        traffic = TRAFFIC.get((args.workload, args.blocks)) if not s["column_labels"] else None
+        traffic = TRAFFIC.get((args.workload, args.blocks)) if joins["rows"] else None
         cb = None if args.no_cpu_baseline else cpu_baseline(w)
         # the other configurations run once, on a single GPU (replica runs hold every GPU meanwhile)
         single = world == 1 and not args.quick

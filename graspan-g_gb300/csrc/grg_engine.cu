@@ -2296,7 +2296,7 @@ __global__ void __launch_bounds__(JOIN_WARPS * 32, (W <= 8 ? GRG_JOIN_MINB : GRG
 // rows that reach across more than 96 get windows of their own where their destinations are local, the
 // row's one window where they are not (see `apart`). What the windows leave out becomes a candidate of
 // one bit. Bound by issue and short waits: 2.4 of 4 warp instructions a clock over the 2M-vertex closure in
-// blocks, 14.7 a pair, DRAM at 4% of its peak; 72 registers, with 128 and 220 bytes of spill stores and loads.
+// blocks, 14.6 a pair, DRAM at 4% of its peak; 72 registers, with 128 and 220 bytes of spill stores and loads.
 // Closures: 10k vertices unconfined 11.1 -> 7.8 ms, 97k in blocks 6.2 -> 5.8 ms, 2M in blocks 53.5 -> 48.7 ms
 // (at 8 blocks a SM 48.8, at 6 51.3, at 10 56.4).
 constexpr int ROWS_WARPS = 4;
