@@ -1290,15 +1290,17 @@ __host__ __device__ inline uint32_t tile_rows_lg(uint64_t n)
     return lg;
 }
 
-// A round whose joined records hold fewer than TILE_MEAN intermediates in the mean goes without tiles (C_TS =
-// TILE_NONE): its panels would have few pairs each, and short right-hand rows besides. Closures (ms) without
-// this line, with it at 16, 24, 32 and 40, and with k_join alone: chains of 20 ids 2.6, 1.8, 1.8, 1.8, 1.8, 1.9;
-// of 100 3.7, 3.1, 2.5, 2.3, 2.3, 2.6; of 250 3.8, 3.1, 2.8, 2.7, 2.5, 3.2; 100k alias of 1 edge a vertex 3.5,
-// 2.2, 2.2, 2.2, 2.2, 3.3; alias in blocks of 100 4.0, 3.1, 2.8, 1.9, 1.9, 3.2; of 200 11.9, 11.4, 10.9, 10.4,
-// 9.7, 11.1; of 1,000, 120k vertices 11.8, 11.2, 11.4, 11.5, 12.4; 1M 69.4, 68.8, 68.6, 68.6, 68.8, 189.
-constexpr uint32_t TILE_MEAN = 32;
+// A round whose records have less than TILE_WORK elements to join a rule in the mean -- intermediates times the
+// elements of a right-hand row -- goes without tiles (C_TS = TILE_NONE): a panel costs the same whatever it joins.
+// Closures (ms) with tiles in every round, with the line at 40, 70, 100 and 150, and with k_join alone: chains of
+// 20 ids 2.6, 1.9, 1.8, 1.8, 1.8, 1.9; of 100 3.7, 2.4, 2.4, 2.4, 2.4, 2.6; of 250 3.8, 2.7, 2.6, 2.6, 2.6, 3.2;
+// 100k alias of 1 edge a vertex 3.5, 2.3, 2.3, 2.3, 2.3, 3.3; alias in blocks of 100 4.0, 2.0, 2.0, 2.0, 2.0, 3.2;
+// of 200 11.9, 10.3, 8.8, 8.9, 8.9, 11.1; 24 dataflow jobs in a batch 37, 20, 20, 20, 20, 22; 1M alias in blocks of
+// 1,000 69.4, 68.7, 68.6, 69 to 73, 79, 189. The intermediates alone do not tell a chain's rows of one element from
+// alias rows of six: a line at 32 of them moved the 1M alias closure between 69 and 75 ms from run to run.
+constexpr uint32_t TILE_WORK = 70;
 constexpr uint32_t TILE_NONE = 0xFF;
-constexpr uint32_t TILE_SAMPLE = 256;          // records that the mean is taken of: a thread each
+constexpr uint32_t SPLIT_THREADS = 256, TILE_SAMPLE = 4 * SPLIT_THREADS;   // records that the mean is taken of
 
 struct TileSmem {
     uint4 tab[TILE_G][16][TILE_Q];             // per 4 rows C[k]: the unions of their 16 subsets
@@ -1834,42 +1836,61 @@ constexpr uint64_t SPLIT_LEFT_MAX = (uint64_t)SPLIT_MAX * SPLIT_PARTS / EW;
 // k_tile, the records are those that it left (C_LN of left), and those not split are joined as they are
 // (C_JN1); of a round without tiles (TILE_NONE) they are the round's own, cut below none_max records and
 // copied to left above. In the static scratch such rounds are never cut (none_max = 0; 3,000-vertex alias
-// closure 3.7 ms, cut 4.3), and half the mean is enough for tiles.
+// closure 3.7 ms, cut 4.3), and half the line is enough for tiles.
 // A thread cuts one bitmap word of a record (up to 4 parts), and a warp reserves its parts' room
 // at once, in record order: a thread a record took 14 us for the 192 bits of a dense one.
 // passes: join kernels of a pass, for the count of their launches (C_JCNT); 0: the host counts.
-__global__ void __launch_bounds__(TILE_SAMPLE) k_split(Dev d, const uint4 *__restrict__ grecs,
-                                                       const uint4 *__restrict__ vrecs, uint4 *__restrict__ left_recs,
-                                                       uint4 *out, int tile, uint64_t split_max, uint64_t none_max,
-                                                       uint32_t passes)
+__global__ void __launch_bounds__(SPLIT_THREADS) k_split(Dev d, const uint4 *__restrict__ grecs,
+                                                         const uint4 *__restrict__ vrecs, uint4 *__restrict__ left_recs,
+                                                         uint4 *out, int tile, uint64_t split_max, uint64_t none_max,
+                                                         uint32_t passes)
 {
     if (d.ctr[C_HALT]) return;
     const bool left = tile == SPLIT_LEFT, none = left && d.ctr[C_TS] == TILE_NONE;
     const uint64_t nd = d.ctr[left && !none ? C_LN : C_DIRTY_N], nv = left && !none ? 0 : d.ctr[C_VN];
     const bool split = nd + nv < (none ? none_max : split_max);
     if (blockIdx.x == 0) {
-        __shared__ uint32_t recs_s, bits_s;
-        if (threadIdx.x == 0) recs_s = bits_s = 0;
+        __shared__ uint32_t joins_s, work_s;
+        if (threadIdx.x == 0) joins_s = work_s = 0;
         __syncthreads();
-        if (tile == 1 && !split) {               // uniform: the mean of the round's records that join
-            const uint64_t i = threadIdx.x * (nd + nv) / TILE_SAMPLE;
-            uint4 a = make_uint4(0, 0, 0, 0), b = make_uint4(0, 0, EMPTY, 0);
-            if (i < nd + nv) ld32(i < nd ? grecs + 2 * i : vrecs + 2 * (i - nd), a, b);
-            const uint32_t lab = b.z >> KEY_SHIFT;
-            const bool joins = i < nd + nv && (i >= nd || (lab >= 1 && lab <= (uint32_t)d.rt.L &&
-                                                           d.rt.bin_start[lab + 1] > d.rt.bin_start[lab]));
-            const uint32_t n = __popc(__ballot_sync(0xffffffffu, joins));
-            const uint32_t p = __reduce_add_sync(0xffffffffu, joins ? popc6(Bits{{a.x, a.y, a.z, a.w, b.x, b.y}}) : 0u);
+        if (tile == 1 && !split) {               // uniform: a sample of the round's records
+            uint32_t joins = 0, work = 0;
+#pragma unroll
+            for (uint32_t u = 0; u < TILE_SAMPLE / SPLIT_THREADS; u++) {
+                const uint64_t i = (u * SPLIT_THREADS + threadIdx.x) * (nd + nv) / TILE_SAMPLE;
+                if (i >= nd + nv) continue;
+                const bool virt = i >= nd;
+                uint4 a, b;
+                ld32(virt ? vrecs + 2 * (i - nd) : grecs + 2 * i, a, b);
+                const uint32_t lab = b.z >> KEY_SHIFT, w[EW] = {a.x, a.y, a.z, a.w, b.x, b.y};
+                uint32_t bits = 0, k = 0;        // intermediates, the last of them
+#pragma unroll
+                for (uint32_t x = 0; x < EW; x++) {
+                    bits += __popc(w[x]);
+                    if (w[x]) k = x * 32 + 31 - __clz(w[x]);
+                }
+                k += (b.z & BASE_MASK) * EIDS;
+                if (!bits || k >= d.V || (!virt && (lab < 1 || lab > (uint32_t)d.rt.L))) continue;
+                const uint32_t q0 = virt ? lab - OL_SLOT0 : d.rt.bin_start[lab];
+                const uint32_t q1 = virt ? min(q0 + 1, (uint32_t)d.rt.nol) : d.rt.bin_start[lab + 1];
+                for (uint32_t q = q0; q < q1; q++) {
+                    const size_t ti = (size_t)((virt ? d.rt.ol_C[q] : d.rt.bin_C[q]) - 1) * d.V + k;
+                    const uint32_t width = !virt ? d.cnt[ti] : d.drs[ti] == EMPTY ? 0u : d.drc[ti];
+                    joins++;
+                    work += bits * min(width, 255u);
+                }
+            }
+            joins = __reduce_add_sync(0xffffffffu, joins);
+            work = __reduce_add_sync(0xffffffffu, work);
             if (lane_id() == 0) {
-                atomicAdd(&recs_s, n);
-                atomicAdd(&bits_s, p);
+                atomicAdd(&joins_s, joins);
+                atomicAdd(&work_s, work);
             }
             __syncthreads();
         }
         if (threadIdx.x == 0) {
-            // (31 bits in the tile list)
-            const uint32_t mean = nd + nv < none_max ? TILE_MEAN : TILE_MEAN / 2;
-            const bool sparse = !bits_s || bits_s < mean * recs_s || (nd | nv) >> 31;
+            const bool sparse = !work_s || work_s < (nd + nv < none_max ? TILE_WORK : TILE_WORK / 2) * joins_s ||
+                                (nd | nv) >> 31;                                  // (31 bits in the tile list)
             const uint32_t ts = split || tile != 1 ? 0 : sparse ? TILE_NONE : tile_rows_lg(nd + nv);
             d.ctr[C_JN1] = split || tile == 1 ? 0 : none ? nd + nv : nd;
             d.ctr[C_JN2] = split || tile ? 0 : nv;
@@ -4166,7 +4187,7 @@ static cudaError_t launch_join(const grg_ctx *c, int grid, cudaStream_t s, const
 // rows are derived rows, dense and alike (1M-vertex alias closure 189 ms with k_join alone, 68.6 ms).
 // With static second symbols a right row is 1-2 elements, too few to pay for a panel: k_rows or k_join.
 // They do while there is room for the tile lists (ensure_tiles), which k_join does not need, and for records
-// that are dense enough (TILE_MEAN).
+// and right-hand rows that are dense enough (TILE_WORK).
 static bool tiles_wanted(const grg_ctx *c) { return c->rt.nol > 0 && !c->need_push; }
 static bool use_tiles(const grg_ctx *c) { return tiles_wanted(c) && c->lbuf_cap > 0; }
 
@@ -4571,7 +4592,7 @@ static int first_pass_joins(grg_ctx *c, const Dev &d, uint64_t nd, uint64_t nv, 
         return GRG_OK;
     }
     if (use_tiles(c)) {
-        k_split<<<1, TILE_SAMPLE, 0, s>>>(d, c->gbuf, c->vbuf, nullptr, nullptr, 1, 0, ~0ull, pass_kernels(c));
+        k_split<<<1, SPLIT_THREADS, 0, s>>>(d, c->gbuf, c->vbuf, nullptr, nullptr, 1, 0, ~0ull, pass_kernels(c));
         GRG_CUDA(c, launch_tiles(c->sms, s, d, c->gbuf, c->vbuf, c->tlist, c->lbuf, c->lbuf_cap, c->rbuf[0]));
         GRG_CUDA(c, cudaMemsetAsync(d.ctr + C_SPLIT_N, 0, 8, s));
         k_split<<<grid_for(c, SPLIT_MAX * EW, 256), 256, 0, s>>>(d, c->gbuf, c->vbuf, c->lbuf, c->sbuf, SPLIT_LEFT,
@@ -6117,9 +6138,9 @@ static int noalloc_closure(int device, void *stream, int num_rules, const int *r
                 k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_SPLIT_N, rbuf[0]);
             } else if (pass == 0 && rt.nol) {
                 // gslot and rbuf[1] are free in this pass: the tile list and the records left to k_join
-                k_split<<<1, TILE_SAMPLE, 0, s>>>(d, gbuf, vbuf, nullptr, nullptr, 1, 0, 0, 0);
+                k_split<<<1, SPLIT_THREADS, 0, s>>>(d, gbuf, vbuf, nullptr, nullptr, 1, 0, 0, 0);
                 NA_CUDA(launch_tiles(sms, s, d, gbuf, vbuf, gslot, rbuf[1], pool, rbuf[0]));
-                k_split<<<sms, TILE_SAMPLE, 0, s>>>(d, gbuf, vbuf, rbuf[1], nullptr, SPLIT_LEFT, 0, 0, 0);
+                k_split<<<sms, SPLIT_THREADS, 0, s>>>(d, gbuf, vbuf, rbuf[1], nullptr, SPLIT_LEFT, 0, 0, 0);
                 NA_CUDA(cudaMemsetAsync(d.ctr + C_JQ, 0, 8, s));
                 k_join<WIN2, WIN2_LO><<<sms * GRG_JOIN_MINB_WIDE, JOIN_WARPS * 32, 0, s>>>(d, rbuf[1], 0, C_JN1, rbuf[0]);
             } else {
