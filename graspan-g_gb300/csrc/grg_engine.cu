@@ -1851,9 +1851,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split(Dev d, const uint4 *__r
     const bool split = nd + nv < (none ? none_max : split_max);
     if (blockIdx.x == 0) {
         __shared__ uint32_t joins_s, work_s;
-        if (threadIdx.x == 0) joins_s = work_s = 0;
-        __syncthreads();
         if (tile == 1 && !split) {               // uniform: a sample of the round's records
+            if (threadIdx.x == 0) joins_s = work_s = 0;
+            __syncthreads();
             uint32_t joins = 0, work = 0;
 #pragma unroll
             for (uint32_t u = 0; u < TILE_SAMPLE / SPLIT_THREADS; u++) {
@@ -1889,9 +1889,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split(Dev d, const uint4 *__r
             __syncthreads();
         }
         if (threadIdx.x == 0) {
-            const bool sparse = !work_s || work_s < (nd + nv < none_max ? TILE_WORK : TILE_WORK / 2) * joins_s ||
-                                (nd | nv) >> 31;                                  // (31 bits in the tile list)
-            const uint32_t ts = split || tile != 1 ? 0 : sparse ? TILE_NONE : tile_rows_lg(nd + nv);
+            uint32_t ts = 0;
+            if (tile == 1 && !split) {
+                const uint32_t line = nd + nv < none_max ? TILE_WORK : TILE_WORK / 2;
+                const bool sparse = !work_s || work_s < line * joins_s || (nd | nv) >> 31;   // (31 bits in the tile list)
+                ts = sparse ? TILE_NONE : tile_rows_lg(nd + nv);
+            }
             d.ctr[C_JN1] = split || tile == 1 ? 0 : none ? nd + nv : nd;
             d.ctr[C_JN2] = split || tile ? 0 : nv;
             if (!left) d.ctr[C_TS] = ts;
