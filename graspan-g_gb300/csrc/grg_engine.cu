@@ -1252,7 +1252,7 @@ __global__ void __launch_bounds__(PUSH_WARPS * 32, 4) k_push_flat(Dev d, const u
 // 37k vertices 13.4 -> 5.4 ms. A block holds one tile a SM (217,424 bytes), bound by waits: 1.5 to 1.7
 // warp instructions a clock of 4 on a 100k-vertex graph, a warp waiting on shared memory (the lookups),
 // on dependent loads (descriptors, then elements) and on the barriers between phases in like parts, L1
-// and shared memory at 49 to 60% of peak. 1,024 threads leave 64 registers, with 156 and 300 bytes of
+// and shared memory at 49 to 59% of peak. 1,024 threads leave 64 registers, with 156 and 300 bytes of
 // spill stores and loads.
 // Only accumulator words that changed are inserted. Right-hand elements outside the window of
 // TILE_W elements are joined in further windows (see TILE_WINDOWS; the first from the lowest block of
