@@ -366,3 +366,22 @@ def test_row_joins_of_several_rules(grg_mod, oracle_mod, monkeypatch, nv, ne, ro
             assert (ctx.label_counts().tolist(), ctx.set_hash()) == want
             assert ctx.last_joins()["rows"] == 1 and st["direct_inserts"] == int(direct)
             assert st["retry_records"] > 0 and st["grow_rows"] > 0
+
+
+def test_window_tuned_for_the_plain_join(grg_mod, oracle_mod):
+    """With the item form fixed the plain join runs, and the window that was measured for it is the one that
+    later closures of the input report and use."""
+    w = G.dataflow_blocks(seed=77, num_blocks=140, block=1000, num_edges=420_000)
+    r = oracle_mod.closure(w.num_vars, w.rule_ids(), w.num_labels, w.filter_flag, w.src, w.dst, w.lab)
+    seen = []
+    for mode in (3, 2):
+        with grg_mod.Context(0) as ctx:
+            ctx.set_join_window(mode)
+            ctx.set_join_items(1)
+            ctx.transfer_rules(w.rule_ids(), w.num_labels)
+            ctx.load_edges(w.num_vars, w.src, w.dst, w.lab)
+            st = ctx.closure(w.filter_flag)
+            assert (ctx.label_counts().tolist(), ctx.set_hash()) == (r.label_counts().tolist(), r.set_hash)
+            assert ctx.last_joins()["rows"] == 0 and st["join_elements"] == 1
+            seen.append((st["window_tuned"], st["wide_window"], min(st["window_trial_ms"]) > 0))
+    assert seen == [(1, seen[0][1], True), (2, seen[0][1], False)]
