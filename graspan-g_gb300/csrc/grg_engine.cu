@@ -1393,7 +1393,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
     const uint32_t sh = (uint32_t)d.ctr[C_TS];
     if (!sh || sh == TILE_NONE) return;
     const uint32_t ntiles = (uint32_t)min((uint64_t)d.ctr[C_TN], list_cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr[C_TSUM] += ntiles;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&d.ctr[C_TSUM], (unsigned long long)ntiles);
     const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5, rows = 1u << sh;
     // in the joins, lanes 0-11 and 16-27 hold a row's 12 quads of 16 bytes (12-15 and 28-31 repeat the last)
     const uint32_t half = lane >> 4, q = min(lane & 15, (uint32_t)TILE_Q - 1);
@@ -1898,8 +1898,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split(Dev d, const uint4 *__r
             d.ctr[C_JN1] = split || tile == 1 ? 0 : none ? nd + nv : nd;
             d.ctr[C_JN2] = split || tile ? 0 : nv;
             if (!left) d.ctr[C_TS] = ts;
-            if (left && !none) d.ctr[C_LSUM] += nd;
-            if (passes) d.ctr[C_JCNT] += ts == TILE_NONE ? 1u : join_launches(split, ts != 0, nv, passes);
+            // (additions that nothing waits for)
+            if (left && !none && nd) atomicAdd(&d.ctr[C_LSUM], (unsigned long long)nd);
+            if (passes) atomicAdd(&d.ctr[C_JCNT], ts == TILE_NONE ? 1ull : join_launches(split, ts != 0, nv, passes));
         }
     }
     if (none && !split)
